@@ -43,7 +43,7 @@ KUFDTD_KAPPA_INC = "kuFDTD/before_CUDA/v0.3.0/boundary/core"
 
 
 def available():
-    return os.path.isdir(REF) and platform.machine() in ("x86_64", "AMD64")
+    return os.path.isfile(os.path.join(REF, KEMP_SRC)) and platform.machine() in ("x86_64", "AMD64")
 
 
 def _kemp_source(coeff_use, pad):
