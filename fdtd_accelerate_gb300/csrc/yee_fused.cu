@@ -28,22 +28,6 @@ __global__ void __launch_bounds__(128) k_zband_h(const __grid_constant__ Params 
     for (int kb = threadIdx.x & 31; kb < nk; kb += 32) zband_h_at(p, i, j, kb);
 }
 
-// Batched band kernels: the band cells of all grids numbered consecutively
-// (off[s] = first cell of grid s); one launch each for E and H per step.
-__global__ void __launch_bounds__(128) k_zband_e_batch(const __grid_constant__ BandBatch d) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= d.off[d.nsims]) return;
-    const int s = band_sim(d, t);
-    zband_e_cell(d.params[2 * s + d.cur], d.t, t - d.off[s]);
-}
-
-__global__ void __launch_bounds__(128) k_zband_h_batch(const __grid_constant__ BandBatch d) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= d.off[d.nsims]) return;
-    const int s = band_sim(d, t);
-    zband_h_cell(d.params[2 * s + d.cur], t - d.off[s]);
-}
-
 }  // namespace fused
 }  // namespace fdtd
 
@@ -72,16 +56,16 @@ static EncodeTiledFn get_encode_fn() {
 }
 
 struct KernelEntry {
-    int ty, ns, threads, stage, enew, psiring;
-    FusedKernel fn[3];        // single grid, EXT = 0, 1, 2
-    FusedKernel fn_batch[2];  // batched, EXT = 0, 1 (batched plans take no plane wave)
+    int ty, ns, threads, smem;  // smem: without the CPML tables
+    FusedKernel fn[2][4];       // single grid: without / with the z-slab terms; bit 0: Drude, bit 1: TFSF
+    FusedKernel fn_batch[2];    // batched, without / with Drude (batched plans take no plane wave)
 };
 
 template <int TY, int NS>
 static KernelEntry entry() {
-    KernelEntry e{TY, NS, Layout<TY, NS>::THREADS, Layout<TY, NS>::STAGE, Layout<TY, NS>::ENEW,
-                  Layout<TY, NS>::PSIRING, {}, {}};
-    single_kernels(TY, NS, e.fn);
+    KernelEntry e{TY, NS, Layout<TY, NS>::THREADS, Layout<TY, NS>::SMEM, {}, {}};
+    single_kernels(TY, NS, e.fn[0]);
+    single_kernels_z(TY, NS, e.fn[1]);
     batch_kernels(TY, NS, e.fn_batch);
     return e;
 }
@@ -133,16 +117,70 @@ static int encode_map(EncodeTiledFn enc, CUtensorMap *m, const float *ptr, const
     return encode_map3(enc, m, ptr, g.nz, g.ny, g.nx, g.sy, g.sx, box_z, box_y, promo);
 }
 
+// Default launch shape: tile rows and pipeline stages.
+constexpr int kTileY = 8, kStages = 3;
+
+// Whether a single grid's z slab is left to the band kernels.  In the fused
+// kernel a z-edge tile takes twice the time of a plain one a plane (its row
+// warps run the z code for a quarter of their lanes); the band kernels cost two
+// launches and a second pass over the row ends.  Measured, fused / bands, us a
+// step with CPML on all faces: 64^3 16.6 / 24.9, 80^3 33 / 38, 128^3 65 / 66,
+// 256x256x128 186 / 167, 256^3 315 / 260, 400x300x200 633 / 429, 512^3 1739 /
+// 1655, 1024x1024x512 6083 / 6596.  Grids of few (i, j) rows keep the bands'
+// three launches, which plan_info reports and the tests of it expect.
+static bool use_bands(const Grid &g) {
+    const int64_t rows = g.nx * g.ny, cells = rows * g.nz;
+    return rows < 2048 || (cells >= ((int64_t)1 << 21) && cells < ((int64_t)1 << 28));
+}
+
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 extern "C" {
 
-// refine: let the default chunk follow the launch-length model below (a plan
-// of its own); the batched plan pools every grid's items over one launch and
-// keeps the provisional chunk
+// Shared memory, resident CTAs and SM count of a kernel variant.
+static int fused_residency(FusedKernel fn, int threads, int smem, int *nsm, int *occ) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void *)fn);
+    if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
+    const int max_dyn = optin - (int)fa.sharedSizeBytes;
+    if (smem > max_dyn) return FDTD_ERR_UNSUPPORTED;
+    // the attribute is an upper bound; every plan of this kernel fits under it
+    e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, (const void *)fn, threads, smem);
+    if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
+    return *occ < 1 ? FDTD_ERR_UNSUPPORTED : FDTD_OK;
+}
+
+// Default x chunk of a single grid: of the splits of nx into 1 .. nx chunks,
+// the one whose launch is shortest when `slots` resident CTAs work through
+// tiles * chunks items of chunk + kItemPlanes plane steps (an item's pipeline
+// fill and its recomputed halo plane); the longer chunk on a tie.
+constexpr int kItemPlanes = 4;
+static int single_chunk(int64_t nx, int64_t tiles, int64_t slots) {
+    int64_t best = nx, best_t = -1;
+    for (int64_t n = 1; n <= nx; n++) {
+        const int64_t c = (nx + n - 1) / n, items = tiles * ((nx + c - 1) / c);
+        const int64_t t = (items + slots - 1) / slots * (c + kItemPlanes);
+        if (c > 128 && n < nx) continue;
+        if (c < 2) break;  // one-plane items would compute every E plane twice
+        if (best_t < 0 || t < best_t) {
+            best_t = t;
+            best = c;
+        }
+    }
+    return (int)best;
+}
+
+// batch: a grid of a batched plan, which pools every grid's items over one
+// launch (x_chunk comes from the batched plan) and whose kernel applies the
+// z-slab terms itself
 static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_yee_state *s, const fdtd_cpml *c,
                            const fdtd_sources *src, const fdtd_tile *tile, int32_t *status_dev, int32_t cur,
-                           void *stream, bool refine) {
+                           void *stream, bool batch) {
     if (!out || !s || !status_dev) return FDTD_ERR_ARG;
     *out = nullptr;
     Grid g;
@@ -160,37 +198,22 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         if (!s->ce[q]) return FDTD_ERR_ARG;
         if (!aligned16(s->ce[q])) return FDTD_ERR_ALIGN;
     }
-    const int ty = tile && tile->tile_y ? tile->tile_y : 8;
-    const int ns = tile && tile->stages ? tile->stages : 3;
+    const int ty = tile && tile->tile_y ? tile->tile_y : kTileY;
+    const int ns = tile && tile->stages ? tile->stages : kStages;
     const KernelEntry *ke = find_kernel(ty, ns);
     if (!ke) return FDTD_ERR_UNSUPPORTED;
-    int xch = tile && tile->x_chunk ? tile->x_chunk : 128;
-    if (xch < 1) return FDTD_ERR_ARG;
-    if (!(tile && tile->x_chunk)) {
-        // provisional default chunk: at least ~3 work items per SM so small
-        // grids fill the GPU (shorter chunks add pipeline fill and halo planes
-        // per item); refined below once the resident CTAs are known
-        int dev = 0, nsm = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && nsm > 0) {
-            const int64_t tiles = ((g.nz + TZ - 1) / TZ) * ((g.ny + ty - 1) / ty);
-            while (xch > 8 && tiles * ((g.nx + xch - 1) / xch) < 3 * (int64_t)nsm) xch /= 2;
-        }
-    }
+    int xch = tile && tile->x_chunk ? tile->x_chunk : 0;  // 0: chosen below
+    if (xch < 0) return FDTD_ERR_ARG;
 
     fdtd_yee_plan *pl = new fdtd_yee_plan();
     pl->g = g;
     pl->k = ke;
-    pl->x_chunk = (int)std::min<int64_t>(xch, g.nx);
     pl->cur = cur;
     Params &p = pl->base;
     p = Params{};
     p.nx = g.nx; p.ny = g.ny; p.nz = g.nz; p.sx = g.sx; p.sy = g.sy;
     p.ntz = (int)((g.nz + TZ - 1) / TZ);
     p.nty = (int)((g.ny + ty - 1) / ty);
-    p.nxc = (int)((g.nx + pl->x_chunk - 1) / pl->x_chunk);
-    p.x_chunk = pl->x_chunk;
-    pl->nitems = (int64_t)p.ntz * p.nty * p.nxc;
     p.status = status_dev;
     p.wait_ns = 0;         // the 1 s limit
     p.test_withhold = -1;  // every copy issued
@@ -255,8 +278,34 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         p.te1d = t.e1d;
         p.th1d = t.h1d;
     }
-    // the z slab (when a z face has CPML) is finished by the band kernels
-    p.zfix = (p.P[2] > 0 && ((p.faces >> 4) & 3)) ? 1 : 0;
+    // the z slab (when a z face has CPML): inside the fused kernel or by the band kernels
+    p.zfix = (!batch && p.P[2] > 0 && ((p.faces >> 4) & 3) && use_bands(g)) ? 1 : 0;
+    // tile rows with y slab cells (rows j0-1 .. j0+ty-1), counted from either end
+    if (p.P[1] > 0)
+        for (int t = 0; t < p.nty; t++) {
+            if (((p.faces >> 2) & 1) && t * ty - 1 <= p.P[1]) p.yf = t + 1;
+            if (((p.faces >> 3) & 1) && (int64_t)(t + 1) * ty - 1 >= g.ny - p.P[1] - 1) {
+                p.yb = p.nty - std::max(t, p.yf);
+                break;
+            }
+        }
+    // launch configuration: shared memory, resident CTAs, x chunk
+    pl->smem = ke->smem + 6 * 2 * (p.P[0] + p.P[1] + p.P[2]) * 4;
+    pl->fn = ke->fn[p.P[2] > 0 && ((p.faces >> 4) & 3) && !p.zfix][(p.drude ? 1 : 0) | (p.tfsf ? 2 : 0)];
+    int nsm = 0, occ = 0;
+    {
+        const int st = fused_residency(pl->fn, ke->threads, pl->smem, &nsm, &occ);
+        if (st != FDTD_OK) { delete pl; return st; }
+    }
+    const int max_ctas = tile ? (int)tile->ctas_per_sm : 0;
+    if (max_ctas > 0) occ = std::min(occ, max_ctas);
+    if (!xch) xch = single_chunk(g.nx, (int64_t)p.ntz * p.nty, (int64_t)nsm * occ);
+    pl->x_chunk = p.x_chunk = (int)std::min<int64_t>(xch, g.nx);
+    p.nxc = (int)((g.nx + pl->x_chunk - 1) / pl->x_chunk);
+    pl->nitems = (int64_t)p.ntz * p.nty * p.nxc;
+    if (pl->nitems >= ((int64_t)1 << 31)) { delete pl; return FDTD_ERR_UNSUPPORTED; }
+    // one CTA an item, or a persistent grid where the caller limits the CTAs per SM
+    pl->nblocks = (int)(max_ctas > 0 ? std::min<int64_t>(pl->nitems, (int64_t)nsm * occ) : pl->nitems);
     if (src && src->nsrc > 0) {
         if (!all_nonnull(src->ijk, src->comp, src->amp) || src->namp < 0) { delete pl; return FDTD_ERR_ARG; }
         p.nsrc = src->nsrc; p.src_ijk = src->ijk; p.src_comp = src->comp; p.src_amp = src->amp; p.namp = src->namp;
@@ -336,90 +385,17 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         }
         if (st != FDTD_OK) { delete pl; return st; }
     }
-    p.stage_bytes = ke->stage;
-    // x/y psi slabs through TMA: rows of nz floats must be 16-byte multiples
-    {
-        const int P0 = p.P[0], P1 = p.P[1];
-        bool ok = (P0 > 0 || P1 > 0) && g.nz % 4 == 0;
-        for (int q = 0; q < 2 && ok; q++) {
-            if (P0 > 0) ok = aligned16(s->psi_e[0][q]) && aligned16(s->psi_e[1][q]) && aligned16(s->psi_h[q]);
-            if (ok && P1 > 0)
-                ok = aligned16(s->psi_e[0][2 + q]) && aligned16(s->psi_e[1][2 + q]) && aligned16(s->psi_h[2 + q]);
-        }
-        int st = FDTD_OK;
-        const int ec = EC, by = ty + 1;
-        for (int b = 0; b < 2 && ok && st == FDTD_OK; b++)
-            for (int q = 0; q < 2 && st == FDTD_OK; q++) {
-                if (P0 > 0) {
-                    st = encode_map3(enc, &pl->maps[b].xpe[q], s->psi_e[b][q], g.nz, g.ny, 2 * P0, g.nz,
-                                     g.ny * g.nz, ec, by, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-                    if (st == FDTD_OK)
-                        st = encode_map3(enc, &pl->maps[b].xph[q], s->psi_h[q], g.nz, g.ny, 2 * P0, g.nz,
-                                         g.ny * g.nz, ec, by, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-                }
-                if (P1 > 0 && st == FDTD_OK) {
-                    st = encode_map3(enc, &pl->maps[b].ype[q], s->psi_e[b][2 + q], g.nz, 2 * P1, g.nx, g.nz,
-                                     2 * P1 * g.nz, ec, by, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-                    if (st == FDTD_OK)
-                        st = encode_map3(enc, &pl->maps[b].yph[q], s->psi_h[2 + q], g.nz, 2 * P1, g.nx, g.nz,
-                                         2 * P1 * g.nz, ec, by, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
-                }
-            }
-        if (st != FDTD_OK) { delete pl; return st; }
-        p.xypsi = ok ? 1 : 0;
-    }
-    const int tab_bytes = 6 * 2 * (p.P[0] + p.P[1] + p.P[2]) * 4;
-    pl->smem = ns * p.stage_bytes + ke->enew + 128 /*barriers*/ + ke->psiring + tab_bytes + 128 /*align slack*/;
-    pl->fn = ke->fn[p.tfsf ? 2 : (p.drude ? 1 : 0)];
-    int dev = 0, nsm = 0, occ = 0, optin = 0;
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void *)pl->fn);
-    if (e != cudaSuccess) { set_cuda_error(e); delete pl; return FDTD_ERR_CUDA; }
-    const int max_dyn = optin - (int)fa.sharedSizeBytes;
-    if (pl->smem > max_dyn) { delete pl; return FDTD_ERR_UNSUPPORTED; }
-    // the attribute is an upper bound; every plan of this kernel fits under it
-    e = cudaFuncSetAttribute((const void *)pl->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)pl->fn, ke->threads, pl->smem);
-    if (e != cudaSuccess) { set_cuda_error(e); delete pl; return FDTD_ERR_CUDA; }
-    if (occ < 1) { delete pl; return FDTD_ERR_UNSUPPORTED; }
-    if (tile && tile->ctas_per_sm > 0) occ = std::min(occ, (int)tile->ctas_per_sm);
-    pl->nblocks = (int)std::min<int64_t>(pl->nitems, (int64_t)nsm * occ);
-    if (refine && !pml && !(tile && tile->x_chunk)) {
-        // the default chunk of a grid without CPML (items of equal cost), now
-        // that the resident CTAs are known: CTA b takes items b, b + CTAs, ...,
-        // so a launch lasts ceil(items / CTAs) items of (chunk + 3) plane steps
-        // (the pipeline fill and the halo plane of an item); of 128, 96, 64,
-        // 48, 32, 24, 16, 12 and 8 planes the chunk with the shortest such
-        // launch, the longer one on a tie.  A chunk other than the provisional
-        // one re-creates the plan with it (the source capacity per item is
-        // checked again).  With CPML the x-slab items cost more and the
-        // provisional chunk stays (at 256x256x128 with a 12-cell CPML the
-        // model's 64 planes ran the step 7 % slower than 32).
-        const int64_t tiles = (int64_t)p.ntz * p.nty, ctas = (int64_t)nsm * occ;
-        int best = pl->x_chunk;
-        int64_t best_t = -1;
-        for (int cand : {128, 96, 64, 48, 32, 24, 16, 12, 8}) {
-            const int64_t cc = std::min<int64_t>(cand, g.nx), items = tiles * ((g.nx + cc - 1) / cc);
-            const int64_t rounds = (items + std::min(items, ctas) - 1) / std::min(items, ctas);
-            const int64_t t = rounds * (cc + 3);
-            if (best_t < 0 || t < best_t) {
-                best_t = t;
-                best = (int)cc;
-            }
-        }
-        if (best != pl->x_chunk) {
-            fdtd_tile t2 = tile ? *tile : fdtd_tile{0, 0, 0, 0, 0};
-            t2.x_chunk = best;
-            fdtd_yee_plan *alt = nullptr;
-            if (yee_plan_create(&alt, gp, s, c, src, &t2, status_dev, cur, stream, false) == FDTD_OK) {
-                delete pl;
-                *out = alt;
-                return FDTD_OK;
-            }
-        }
+    // 16-byte accesses of the x/y psi slabs: rows of nz floats must be 16-byte
+    // multiples
+    p.vpsi = g.nz % 4 == 0;
+    for (int q = 0; q < 4 && pml; q++)
+        if (p.P[q / 2] > 0)
+            p.vpsi = p.vpsi && aligned16(s->psi_e[0][q]) && aligned16(s->psi_e[1][q]) && aligned16(s->psi_h[q]);
+    if (p.drude) {
+        p.dvec = p.dbox[2] % 4 == 0 && p.dbox[5] % 4 == 0;
+        for (int q = 0; q < 3; q++)
+            p.dvec = p.dvec && aligned16(pl->dj[0][q]) && aligned16(pl->dj[1][q]) && aligned16(p.dcja[q]) &&
+                     aligned16(p.dcjb[q]);
     }
     *out = pl;
     return FDTD_OK;
@@ -428,7 +404,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
 int fdtd_yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_yee_state *s, const fdtd_cpml *c,
                          const fdtd_sources *src, const fdtd_tile *tile, int32_t *status_dev, int32_t cur,
                          void *stream) {
-    return yee_plan_create(out, gp, s, c, src, tile, status_dev, cur, stream, true);
+    return yee_plan_create(out, gp, s, c, src, tile, status_dev, cur, stream, false);
 }
 
 int fdtd_yee_plan_run(fdtd_yee_plan *pl, int64_t t0, int64_t nsteps, void *stream) {
@@ -532,13 +508,9 @@ struct fdtd_batch_plan {
     int nblocks;
     int cur;
     int64_t nitems;
-    int stage_bytes;
     TMaps *d_maps;
     Params *d_params;
     int64_t *d_off;        // work-item offsets of the fused kernel
-    int64_t *d_band_e;     // band cell offsets (E, H) of the band kernels
-    int64_t *d_band_h;
-    int64_t band_e, band_h;  // band cells in all grids
     int32_t *d_queue;        // work queue of the fused kernel (2 counters)
 };
 
@@ -549,8 +521,8 @@ static size_t batch_ws_layout(int32_t nsims, size_t *off_params, size_t *off_ite
     *off_params = o;
     o += (size_t)2 * nsims * sizeof(Params);
     o = (o + 63) / 64 * 64;
-    *off_items = o;  // work-item offsets, then E and H band cell offsets, then the queue
-    o += (size_t)3 * (nsims + 1) * sizeof(int64_t);
+    *off_items = o;  // work-item offsets, then the queue
+    o += (size_t)(nsims + 1) * sizeof(int64_t);
     o += 64;
     return o;
 }
@@ -574,17 +546,41 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     if (workspace_bytes < need) return FDTD_ERR_CAPACITY;
     std::vector<TMaps> maps((size_t)2 * nsims);
     std::vector<Params> params((size_t)2 * nsims);
-    std::vector<int64_t> off((size_t)3 * (nsims + 1), 0);
-    int64_t *boff_e = off.data() + (nsims + 1), *boff_h = off.data() + 2 * (nsims + 1);
+    std::vector<int64_t> off((size_t)nsims + 1, 0);
     const KernelEntry *ke = nullptr;
-    int stage_bytes = 0, tab_bytes = 0;
+    int tab_bytes = 0;
     bool any_drude = false;
+    const int ty = tile && tile->tile_y ? tile->tile_y : kTileY;
+    fdtd_tile bt = tile ? *tile : fdtd_tile{0, 0, 0, 0, 0};
+    if (ty > 0 && !bt.x_chunk) {
+        // default chunk for all grids: of 8 .. 128 planes, the one for which the
+        // items (planes + kItemPlanes each) of all grids, spread evenly over
+        // the CTAs, plus one last item end first
+        int dev = 0, nsm = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1)
+            nsm = 1;
+        double best_t = -1;
+        for (int c : {128, 96, 64, 48, 32, 24, 16, 12, 8}) {
+            double work = 0;
+            int64_t longest = 0;
+            for (int32_t s = 0; s < nsims; s++) {
+                const int64_t tiles = ((grids[s].nz + TZ - 1) / TZ) * ((grids[s].ny + ty - 1) / ty);
+                work += (double)tiles * (double)(grids[s].nx + kItemPlanes * ((grids[s].nx + c - 1) / c));
+                longest = std::max(longest, std::min<int64_t>(c, grids[s].nx) + kItemPlanes);
+            }
+            const double t = work / (2.0 * nsm) + (double)longest;
+            if (best_t < 0 || t < best_t) {
+                best_t = t;
+                bt.x_chunk = c;
+            }
+        }
+    }
     // grids with the longest items (x planes per chunk, then tile rows) come first
     std::vector<int32_t> order((size_t)nsims);
     for (int32_t s = 0; s < nsims; s++) order[s] = s;
     auto item_len = [&](int32_t s) {
-        const int64_t xc = tile && tile->x_chunk ? tile->x_chunk : 128;
-        return std::min<int64_t>(xc, grids[s].nx) * 65536 + std::min<int64_t>(grids[s].ny, 65535);
+        return std::min<int64_t>(bt.x_chunk, grids[s].nx) * 65536 + std::min<int64_t>(grids[s].ny, 65535);
     };
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return item_len(a) > item_len(b); });
     for (int32_t s = 0; s < nsims; s++)
@@ -593,10 +589,9 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
         const int32_t u = order[s];
         fdtd_yee_plan *pl = nullptr;
         const int st = yee_plan_create(&pl, &grids[u], &states[u], cpmls ? &cpmls[u] : nullptr,
-                                       srcs ? &srcs[u] : nullptr, tile, status_dev, cur, stream, false);
+                                       srcs ? &srcs[u] : nullptr, &bt, status_dev, cur, stream, true);
         if (st != FDTD_OK) return st;
         ke = pl->k;
-        stage_bytes = std::max(stage_bytes, pl->base.stage_bytes);
         any_drude = any_drude || pl->base.drude;
         tab_bytes = std::max(tab_bytes, 6 * 2 * (pl->base.P[0] + pl->base.P[1] + pl->base.P[2]) * 4);
         for (int b = 0; b < 2; b++) {
@@ -615,8 +610,6 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
             maps[2 * s + b] = pl->maps[b];
         }
         off[s + 1] = off[s] + pl->nitems;
-        boff_e[s + 1] = boff_e[s] + zband_e_cells(pl->base);
-        boff_h[s + 1] = boff_h[s] + zband_h_cells(pl->base);
         fdtd_yee_plan_destroy(pl);
     }
     // fill the workspace on the caller's stream (ordered after that stream's
@@ -636,33 +629,17 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     fdtd_batch_plan *bp = new fdtd_batch_plan();
     bp->nsims = nsims;
     bp->k = ke;
-    bp->stage_bytes = stage_bytes;
-    bp->smem = ke->ns * stage_bytes + ke->enew + 128 + ke->psiring + tab_bytes + 128;
+    bp->smem = ke->smem + tab_bytes;
     bp->cur = cur;
     bp->nitems = off[nsims];
     bp->d_maps = reinterpret_cast<TMaps *>(ws);
     bp->d_params = reinterpret_cast<Params *>(ws + off_p);
     bp->d_off = reinterpret_cast<int64_t *>(ws + off_i);
-    bp->d_band_e = bp->d_off + (nsims + 1);
-    bp->d_band_h = bp->d_off + 2 * (nsims + 1);
-    bp->band_e = boff_e[nsims];
-    bp->band_h = boff_h[nsims];
     bp->d_queue = reinterpret_cast<int32_t *>(ws + off_i + off.size() * sizeof(int64_t));
-    int dev = 0, nsm = 0, occ = 0, optin = 0;
-    cudaFuncAttributes fa;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     bp->fn = ke->fn_batch[any_drude ? 1 : 0];
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void *)bp->fn);
-    if (e != cudaSuccess) { set_cuda_error(e); delete bp; return FDTD_ERR_CUDA; }
-    const int max_dyn = optin - (int)fa.sharedSizeBytes;
-    if (bp->smem > max_dyn) { delete bp; return FDTD_ERR_UNSUPPORTED; }
-    e = cudaFuncSetAttribute((const void *)bp->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)bp->fn, ke->threads, bp->smem);
-    if (e != cudaSuccess) { set_cuda_error(e); delete bp; return FDTD_ERR_CUDA; }
-    if (occ < 1) { delete bp; return FDTD_ERR_UNSUPPORTED; }
+    int nsm = 0, occ = 0;
+    const int rs = fused_residency(bp->fn, ke->threads, bp->smem, &nsm, &occ);
+    if (rs != FDTD_OK) { delete bp; return rs; }
     if (tile && tile->ctas_per_sm > 0) occ = std::min(occ, (int)tile->ctas_per_sm);
     bp->nblocks = (int)std::min<int64_t>(bp->nitems, (int64_t)nsm * occ);
     *out = bp;
@@ -684,15 +661,8 @@ int fdtd_batch_plan_run(fdtd_batch_plan *bp, int64_t t0, int64_t nsteps, void *s
         bd.params = bp->d_params;
         bd.maps = bp->d_maps;
         bd.item_off = bp->d_off;
-        bd.stage_bytes = bp->stage_bytes;
         bd.queue = bp->d_queue;
         bp->fn<<<bp->nblocks, bp->k->threads, bp->smem, st>>>(dummy_maps, dummy, bd);
-        if (bp->band_e > 0 || bp->band_h > 0) {
-            BandBatch d{bp->nsims, bp->cur, t0 + n, bp->d_params, bp->d_band_e};
-            if (bp->band_e > 0) k_zband_e_batch<<<(unsigned)((bp->band_e + 127) / 128), 128, 0, st>>>(d);
-            d.off = bp->d_band_h;
-            if (bp->band_h > 0) k_zband_h_batch<<<(unsigned)((bp->band_h + 127) / 128), 128, 0, st>>>(d);
-        }
         FDTD_TRY(check_launch());
         bp->cur = 1 - bp->cur;
     }

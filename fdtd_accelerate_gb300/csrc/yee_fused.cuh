@@ -13,30 +13,48 @@
 //    and writes buffer `1-cur`.  E-psi slabs are ping-ponged too; H-psi is
 //    updated in place (only its owner touches it).
 //  * A CTA owns a tile of TZ=64 (z) x TY (y) cells for a chunk of x planes
-//    and marches along x.  For plane i it needs H(i), H(i+1), E(i), CE(i)
-//    with a one-cell halo at j0-1 / k0-1 (and j0+TY / k0+TZ for H).  These
-//    arrive by 3-D TMA box loads (cp.async.bulk.tensor) into a ring of NS
-//    shared-memory stages, completion tracked by mbarriers.
+//    and marches along x.  A thread owns a group of 4 z cells of one row, so
+//    every shared and global access of the plain path is 16 bytes wide: about
+//    50 instructions a cell and step, where a thread with two cells and
+//    64-bit plane indices took 300 and kept the schedulers 58 % busy.
+//  * For plane i the tile needs H(i), H(i+1), E(i), CE(i) with a one-cell
+//    halo at j0-1 / k0-1 (and j0+TY / k0+TZ for H).  3-D TMA box loads
+//    (cp.async.bulk.tensor) bring stage q = {E(q), CE(q), H(q+1)} into rings
+//    of NS (E, CE) and NS+1 (H) shared-memory slots; one mbarrier a stage.
 //  * E_new is computed on the tile plus the j0-1 row and k0-1 column
 //    (halo cells are recomputed from the untouched input buffer, never read
 //    from a neighbour), then H_new(i) for the tile uses E_new(i) from shared
-//    memory and E_new(i-1) kept in registers.
+//    memory (two buffers) and E_new(i-1) kept in registers.  One CTA barrier
+//    a plane: after it E_new is visible and the plane's slots are free, and
+//    the spare lane of the halo warp refills them.
 //  * A chunk starting at x0 > 0 recomputes E_new(x0-1) without storing it.
+//  * What bounds it: DRAM on plain grids (512^3 1.25 ms a step, 6.4 TB/s on 60
+//    bytes a cell, 0.95 of the measured copy; the kernel before this one 1.8 ms),
+//    on absorbing grids the instruction stream of the slab planes (a plane of
+//    a z-edge tile executes twice a plain one's) and halos read twice where
+//    tiles of different speed drift apart.  Measured and dropped: 2 cells a
+//    thread (1024x1024x512 with CPML 7.2 against 6.1 ms), the E and the H phase
+//    on warps of their own (8.4 ms: 96 registers a thread, spills), the z-slab
+//    terms on two extra warps (7.1 ms: warps on different code miss the
+//    instruction cache), psi prefetched into registers a plane ahead (no gain
+//    over the L2 prefetch), two stages with 3 CTAs per SM (6.6 ms).
 //  * Every mbarrier wait is bounded; on expiry the kernel records
 //    FDTD_ERR_TIMEOUT in a device status word and the CTA leaves its loop.
 #pragma once
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
 namespace fdtd {
 namespace fused {
 
-// Tile: TZ cells along z (two per lane: lanes work on float2 pairs) x TY rows.
+// Tile: TZ cells along z (4 per thread) x TY rows.
 constexpr int TZ = 64;
+constexpr int GZ = TZ / 4;   // groups of 4 z cells in a tile row
 constexpr int HC = TZ + 8;   // H box:    k0-4 .. k0+TZ+3 (needs k0-1 .. k0+TZ)
-constexpr int EC = TZ + 4;   // E/CE box: k0-4 .. k0+TZ-1 (needs k0-1 .. k0+TZ-1)
-constexpr int NCW = TZ + 4;  // E_new row stride; column c holds k = k0-2+c
+constexpr int EC = TZ + 4;   // E/CE box: k0-4 .. k0+TZ-1 (needs k0-1 .. k0+TZ-1); E_new rows too
 constexpr int MAX_LOCAL_SRC = 128;
 constexpr int MAX_BAND_SRC = 32;
 constexpr uint64_t WAIT_NS = 1000000000ull;  // a wait gives up after 1 s
@@ -44,47 +62,41 @@ constexpr uint64_t WAIT_NS = 1000000000ull;  // a wait gives up after 1 s
 constexpr int al128(int b) { return (b + 127) / 128 * 128; }
 
 // Shared-memory layout of one CTA for tile height TY and NS pipeline stages.
-// Warps 0..TY-1 own rows j0..j0+TY-1 (E and H); warp TY recomputes E_new on
-// the halo row j0-1; warp TY+1 recomputes E_new on the halo column k0-1;
-// lane 0 of warp TY+2 is the producer (mbarrier waits, TMA issue).
+// Threads 0 .. OWN-1 own the tile's groups (E and H); the next HALO threads
+// recompute E_new on the halo row j0-1 (GZ groups) and on the halo column
+// k0-1 (one group a row, of which the last cell counts); the last thread
+// issues the TMA copies.
 template <int TY, int NS>
 struct Layout {
-    static constexpr int HR = TY + 2, ER = TY + 1;
+    static constexpr int HR = TY + 2, ER = TY + 1, NH = NS + 1;
     static constexpr int HBOX = HR * HC, EBOX = ER * EC;  // floats per component box
     static constexpr int HBOXB = al128(HBOX * 4), EBOXB = al128(EBOX * 4);
-    static constexpr int STAGE = 3 * HBOXB + 6 * EBOXB;  // H(3), E(3), CE(3)
-    static constexpr uint32_t TX = 3 * HBOX * 4 + 6 * EBOX * 4;
-    // a stage completes on two barriers: H (needed one plane early, as H(i+1))
-    // and E + CE (needed on its own plane only)
+    static constexpr int HSLOT = 3 * HBOXB, ESLOT = 6 * EBOXB;  // H(3); E(3), CE(3)
     static constexpr uint32_t TX_H = 3 * HBOX * 4, TX_E = 6 * EBOX * 4;
-    static constexpr int NR = TY + 1;
-    static constexpr int ENEWC = NR * NCW;  // floats per component
-    // TY row warps, the halo-row warp, the halo-column warp, the producer warp
-    static constexpr int THREADS = (TY + 3) * 32;
-    static constexpr int ENEW = al128(3 * ENEWC * 4);
-    // psi ring: 2 slots x 4 boxes (E psi 1, 2 and H psi 1, 2 of one axis)
-    static constexpr int PSIRING = 2 * 4 * EBOXB;
-    static constexpr uint32_t PSI_TX = EBOX * 4;
-    static constexpr int SMEM = NS * STAGE + ENEW + 128 /*barriers*/ + PSIRING + 128 /*align slack*/;
-    // CTAs per SM the register budget is sized for (shared memory may allow fewer)
-    static constexpr int MINB = TY == 4 ? 3 : (TY == 8 ? 2 : 1);
+    static constexpr int OWN = TY * GZ, HALO = GZ + TY;
+    static constexpr int THREADS = (OWN + HALO + 1 + 31) / 32 * 32;
+    static constexpr int PRODUCER = THREADS - 1;
+    static constexpr int OFF_E = NH * HSLOT;
+    static constexpr int OFF_N = OFF_E + NS * ESLOT;  // E_new: two buffers of three boxes
+    static constexpr int OFF_BAR = OFF_N + 2 * 3 * EBOXB;
+    static constexpr int OFF_TAB = OFF_BAR + 128 + 16;  // z groups read up to 4 floats before a table
+    static constexpr int SMEM = OFF_TAB + 16 + 128 /*align slack*/;  // plus the CPML tables
+    // CTAs per SM that shared memory allows: what the register budget is sized for
+    static constexpr int FIT = 232448 / (SMEM + 2048);
+    static constexpr int MINB = FIT < 1 ? 1 : (FIT > 4 ? 4 : FIT);
 };
 
 struct TMaps {
     CUtensorMap h[3];   // hx, hy, hz of the input buffer, box (HC, TY+2, 1)
     CUtensorMap e[3];   // ex, ey, ez of the input buffer, box (EC, TY+1, 1)
     CUtensorMap ce[3];  // cex, cey, cez,                  box (EC, TY+1, 1)
-    // x/y CPML psi slabs, box (EC, TY+1, 1): x arrays (2P, ny, nz) at (k0-4, j0-1, s),
-    // y arrays (nx, 2P, nz) at (k0-4, first slab index of the tile, i)
-    CUtensorMap xpe[2];  // eyx, ezx of the input buffer
-    CUtensorMap xph[2];  // hyx, hzx
-    CUtensorMap ype[2];  // ezy, exy of the input buffer
-    CUtensorMap yph[2];  // hzy, hxy
 };
 
 struct Params {
     int64_t nx, ny, nz, sx, sy;
     int32_t ntz, nty, nxc, x_chunk;
+    // tile rows at either end that hold y slab cells (item order)
+    int32_t yf, yb;
     float *out[6];  // ex, ey, ez, hx, hy, hz of the output buffer
     const float *psi_e_in[6];
     float *psi_e_out[6];
@@ -100,12 +112,11 @@ struct Params {
     int64_t namp;
     int64_t t;
     int32_t *status;
-    int32_t stage_bytes;  // bytes per pipeline stage
-    int32_t xypsi;        // 1: x/y psi slabs arrive by TMA in the psi ring
-    // z band (1 when a z face has CPML): the z-slab CPML is finished by the
-    // band kernels.  The fused kernel leaves them the E z-psi correction, the
-    // sources on E z-slab nodes and every H cell of the band (k in [1, P+1]
-    // and [n-P-1, n-1]).
+    int32_t vpsi;         // 1: rows of the x/y psi slabs are 16-byte multiples (float4 accesses)
+    // 1: the z-slab CPML is finished by the band kernels.  The fused kernel
+    // leaves them the E z-psi correction, the sources on E z-slab nodes and
+    // every H cell of the band (k in [1, P+1] and [n-P-1, n-1]).  0: the fused
+    // kernel applies the z terms itself, like the x and y ones.
     int32_t zfix;
     const float *in[6];   // input buffer fields (read by the band kernels)
     const float *in_ce[3];
@@ -115,7 +126,7 @@ struct Params {
     int32_t bsrc[MAX_BAND_SRC];
     // Drude box (drude = 1): cells [i0, i0+ni) x [j0, j0+nj) x [k0, k0+nk); dense J, CJA, CJB;
     // J is read from dj_in and written to dj_out (ping-pong like E-psi)
-    int32_t drude;
+    int32_t drude, dvec;  // dvec: the box's rows are 16-byte multiples on the grid's groups of 4 cells
     int64_t dbox[6];  // i0, j0, k0, ni, nj, nk
     const float *dj_in[3];
     float *dj_out[3];
@@ -145,6 +156,7 @@ __host__ __device__ __forceinline__ int64_t pext_y(const Params &p, int q) {
     return ax == 0 ? P2 * p.ny * p.nz : (ax == 1 ? p.nx * P2 * p.nz : p.nx * p.ny * P2);
 }
 
+
 // Many independent grids advanced by one launch: work items of all grids are
 // numbered consecutively; item_off[s] is the first item of grid s.
 struct BatchDesc {
@@ -154,7 +166,6 @@ struct BatchDesc {
     const Params *params;    // [2*nsims]: grid s reading buffer b at params[2*s + b]
     const TMaps *maps;       // [2*nsims]: tensor maps of grid s, input buffer b
     const int64_t *item_off; // [nsims + 1]
-    int32_t stage_bytes;     // pipeline stage size (max over grids)
     // work queue: [0] next item, [1] CTAs finished; zero between launches (the
     // last CTA to finish clears both)
     int32_t *queue;
@@ -221,52 +232,24 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map) {
 }
 
 // CPML slab index of an E node / H node along one axis, or -1.
-__device__ __forceinline__ int slab_e(int64_t idx, int P, int64_t n, int front, int back) {
+__device__ __forceinline__ int slab_e(int idx, int P, int n, int front, int back) {
     if (P <= 0) return -1;
-    if (front && idx >= 1 && idx <= P) return (int)(idx - 1);
-    if (back && idx >= n - P - 1 && idx <= n - 2) return (int)(P + idx - (n - P - 1));
+    if (front && idx >= 1 && idx <= P) return idx - 1;
+    if (back && idx >= n - P - 1 && idx <= n - 2) return P + idx - (n - P - 1);
     return -1;
 }
-__device__ __forceinline__ int slab_h(int64_t idx, int P, int64_t n, int front, int back) {
+__device__ __forceinline__ int slab_h(int idx, int P, int n, int front, int back) {
     if (P <= 0) return -1;
-    if (front && idx >= 1 && idx <= P) return (int)(idx - 1);
-    if (back && idx >= n - P && idx <= n - 1) return (int)(P + idx - (n - P));
+    if (front && idx >= 1 && idx <= P) return idx - 1;
+    if (back && idx >= n - P && idx <= n - 1) return P + idx - (n - P);
     return -1;
 }
 
 // H cells whose update reads an E z-slab node or that carry a z psi:
 // k in [1, P+1] (front) or [n-P-1, n-1] (back)
-__device__ __forceinline__ bool in_zband_h(int64_t k, int P, int64_t n, int front, int back) {
+__device__ __forceinline__ bool in_zband_h(int k, int P, int n, int front, int back) {
     if (P <= 0) return false;
     return (front && k >= 1 && k <= P + 1) || (back && k >= n - P - 1 && k <= n - 1);
-}
-
-__device__ __forceinline__ float cpml_corr(float &psi, float b, float a, float km1, float d) {
-    psi = fadd(fmul(b, psi), fmul(a, d));
-    return fadd(fmul(km1, d), psi);
-}
-
-__device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
-__device__ __forceinline__ void st2(float *p, float2 v) { *reinterpret_cast<float2 *>(p) = v; }
-#ifndef FDTD_PACKED_F32X2
-#define FDTD_PACKED_F32X2 0
-#endif
-#if FDTD_PACKED_F32X2
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-// a - b rounds exactly like a + (-b)
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-#else
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(fadd(a.x, b.x), fadd(a.y, b.y)); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return make_float2(fsub(a.x, b.x), fsub(a.y, b.y)); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(fmul(a.x, b.x), fmul(a.y, b.y)); }
-#endif
-__device__ __forceinline__ float2 curl4x2(float2 a, float2 b, float2 c, float2 d) {
-    return add2(sub2(sub2(a, b), c), d);
-}
-__device__ __forceinline__ float get(const float2 &v, int e) { return e ? v.y : v.x; }
-__device__ __forceinline__ void set(float2 &v, int e, float x) {
-    if (e) v.y = x; else v.x = x;
 }
 
 // CPML table entry of one slab node (b, a, 1/kappa - 1).
@@ -285,6 +268,153 @@ __device__ __forceinline__ float corr(float &psi, const Coef &c, float d) {
 __device__ __forceinline__ Coef tab_coef(const float *tabs, int base, int n2, int eh, int s) {
     const float *t = tabs + base + eh * 3 * n2;
     return Coef{t[s], t[n2 + s], t[2 * n2 + s]};
+}
+
+// Four consecutive z cells.
+struct V4 {
+    float v[4];
+};
+__device__ __forceinline__ V4 lds4(const float *s) {
+    const float4 t = *reinterpret_cast<const float4 *>(s);
+    return V4{{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ void sts4(float *s, const V4 &a) {
+    *reinterpret_cast<float4 *>(s) = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
+}
+__device__ __forceinline__ bool bit(uint32_t m, int e) { return (m >> e) & 1; }
+
+// Elements q .. q+3 of a global array of n elements: the cells of mask m, as
+// one 16-byte access where vec says that the group is aligned (it then lies
+// in the array whole) and, for a store, m has all four.
+__device__ __forceinline__ V4 ldg4(const float *a, int64_t q, uint32_t m, bool vec, [[maybe_unused]] int64_t n) {
+    V4 r{};
+    if (vec) {
+        if (m && FDTD_IN(q, n) && FDTD_IN(q + 3, n)) r = lds4(a + q);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (bit(m, e) && FDTD_IN(q + e, n)) r.v[e] = a[q + e];
+    }
+    return r;
+}
+__device__ __forceinline__ void stg4(float *a, int64_t q, uint32_t m, bool vec, const V4 &r,
+                                     [[maybe_unused]] int64_t n) {
+    if (vec && m == 0xFu) {
+        if (FDTD_IN(q, n) && FDTD_IN(q + 3, n)) sts4(a + q, r);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (bit(m, e) && FDTD_IN(q + e, n)) a[q + e] = r.v[e];
+    }
+}
+
+// The z-slab nodes of a group: m its cells (bits) on front or back nodes, s(e)
+// the slab index of cell e.  A group on nodes of both sides (grids of at most
+// 2P+5 cells along z) has two bases, else one (add = 0).
+struct ZSlab {
+    uint32_t m;
+    int base, add;  // slab index of cell 0; what the back nodes add to it
+    uint32_t bm;    // cells on back nodes, where the group has both
+    __device__ __forceinline__ int s(int e) const { return base + e + (bit(bm, e) ? add : 0); }
+};
+__device__ __forceinline__ ZSlab zslab(int kk, int P, int n, int front, int back, bool e, uint32_t in) {
+    const int s0 = kk - 1, s1 = kk + P - (e ? n - P - 1 : n - P);
+    uint32_t fm = 0, bm = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const int k = kk + c;
+        fm |= (uint32_t)(P > 0 && front && k >= 1 && k <= P) << c;
+        bm |= (uint32_t)(P > 0 && back && (e ? k >= n - P - 1 && k <= n - 2 : k >= n - P && k <= n - 1)) << c;
+    }
+    fm &= in;
+    bm &= in;
+    return fm ? ZSlab{fm | bm, s0, s1 - s0, bm} : ZSlab{bm, s1, 0, 0u};
+}
+// psi of the group's z-slab cells (row: first element of the dense z-psi row):
+// one address and constant offsets but for groups with two bases
+__device__ __forceinline__ V4 ldz4(const float *a, int64_t row, uint32_t m, const ZSlab &z, [[maybe_unused]] int64_t n) {
+    V4 r{};
+    if (z.bm == 0) {
+        const float *b = a + (row + z.base);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (bit(m, e) && FDTD_IN(row + z.base + e, n)) r.v[e] = b[e];
+    } else {
+#pragma unroll 1
+        for (int e = 0; e < 4; e++)
+            if (bit(m, e) && FDTD_IN(row + z.s(e), n)) {
+                const float t = a[row + z.s(e)];
+#pragma unroll
+                for (int u = 0; u < 4; u++) r.v[u] = u == e ? t : r.v[u];
+            }
+    }
+    return r;
+}
+__device__ __forceinline__ void stz4(float *a, int64_t row, uint32_t m, const ZSlab &z, const V4 &r,
+                                     [[maybe_unused]] int64_t n) {
+    if (z.bm == 0) {
+        float *b = a + (row + z.base);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (bit(m, e) && FDTD_IN(row + z.base + e, n)) b[e] = r.v[e];
+    } else {
+#pragma unroll 1
+        for (int e = 0; e < 4; e++)
+            if (bit(m, e) && FDTD_IN(row + z.s(e), n)) {
+                float t = r.v[0];
+#pragma unroll
+                for (int u = 1; u < 4; u++) t = u == e ? r.v[u] : t;
+                a[row + z.s(e)] = t;
+            }
+    }
+}
+__device__ __forceinline__ void prefetch_l2(const float *a) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
+}
+
+// One CPML term of a group: f += S * cf * (km1 d + psi'), psi' = b psi + a d,
+// d = hi - lo, on the cells of m; without a branch a cell (values of the
+// other cells are computed and dropped).
+template <int S>
+__device__ __forceinline__ void term_cell(float &f, float cf, float &psi, const Coef &c, float d, bool in) {
+    float ps = psi;
+    const float t = fmul(cf, corr(ps, c, d));
+    const float v = S > 0 ? fadd(f, t) : fsub(f, t);
+    f = in ? v : f;
+    psi = ps;
+}
+template <int S>
+__device__ __forceinline__ void slab_term(V4 &f, const V4 &cf, V4 &psi, const Coef &c, const V4 &hi, const V4 &lo,
+                                          uint32_t m) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) term_cell<S>(f.v[e], cf.v[e], psi.v[e], c, fsub(hi.v[e], lo.v[e]), bit(m, e));
+}
+// the z slab's: coefficients by cell (tab: b of the family's tables, n2 entries
+// each; cells off the slab read a neighbouring table's entry, at most 3 floats past)
+template <int S>
+__device__ __forceinline__ void z_term(V4 &f, const V4 &cf, V4 &psi, const float *tab, int n2, const ZSlab &z,
+                                       const V4 &hi, const V4 &lo, uint32_t m) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const float *t = tab + (z.bm == 0 ? z.base + e : (bit(z.m, e) ? z.s(e) : 0));
+        const Coef c{t[0], t[n2], t[2 * n2]};
+        term_cell<S>(f.v[e], cf.v[e], psi.v[e], c, fsub(hi.v[e], lo.v[e]), bit(m, e));
+    }
+}
+// tile and x chunk of work item u: the tile rows that hold y slab cells first
+// (their planes take up to twice as long: started last, they would be the
+// launch's tail; 256^3 with y faces alone 213 -> 180 us), z tile fastest, and
+// of either kind the first and the last x chunk (x slab planes) first.  Not so
+// the z-edge tiles, which are as slow: apart from their neighbours in time,
+// they would share no halo reads through L2 (1024x1024x512: 6.1 -> 7.0 ms).
+__device__ __forceinline__ void item_tile(const Params &p, int u, int &tz, int &ty, int &xc) {
+    const int ye = p.yf + p.yb, nm = p.nty - ye, edge = p.ntz * ye * p.nxc;
+    const bool first = u < edge;
+    if (!first) u -= edge;
+    const int tiles = p.ntz * (first ? ye : nm), c = u / tiles, t = u % tiles, r = t / p.ntz;
+    tz = t % p.ntz;
+    ty = first ? (r < p.yf ? r : p.nty - ye + r) : p.yf + r;
+    xc = c == 0 ? 0 : (c == 1 ? p.nxc - 1 : c - 1);
 }
 
 // TFSF correction of one face slot: v += 0.5 (c * F1d[idx]) (kuFDTD/v0.2.0/dim3/tfsf.py:79-89)
@@ -373,118 +503,93 @@ __device__ __forceinline__ void tfsf_apply(const Params &p, int eh, uint32_t cod
     }
 }
 
-// EXT: 0 = neither the Drude box nor the TFSF faces are compiled in, 1 = the
-// Drude box, 2 = both.  A plan launches the smallest variant its grid needs:
-// code a step does not use still costs it registers and instruction-cache
-// space (the plain step ran 3.5 % slower with both compiled in).
+// EXT: bit 0: the Drude box is compiled in, bit 1: the TFSF faces, bit 2: the
+// z-slab terms (else they are the band kernels').  A plan
+// launches the variant its grid needs: code a step does not use still costs it
+// registers and instruction-cache space.
 template <int TY, int NS, bool BATCH, int EXT>
 __global__ void __launch_bounds__(Layout<TY, NS>::THREADS, Layout<TY, NS>::MINB)
 k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk, const __grid_constant__ BatchDesc bd) {
     using L = Layout<TY, NS>;
-    // A stage is released one iteration after its plane was consumed, and each
-    // iteration holds two planes: fewer than 3 stages would wait on a plane
-    // that is only issued after the wait.
-    static_assert(NS >= 3, "the fused pipeline needs at least 3 stages");
-    static_assert((2 * NS + 2) * 8 <= 128, "the mbarriers live in 128 bytes");
+    constexpr bool DRUDE = EXT & 1, TFSF = EXT & 2, ZIN = EXT & 4;
+    static_assert(NS * 8 <= 128, "the mbarriers live in 128 bytes");
     extern __shared__ unsigned char smem_raw[];
     // 128-byte aligned base, computed from the shared-window offset so the
     // pointer stays in the shared address space (shared loads, not generic ones)
     unsigned char *smem =
         smem_raw + ((128u - (static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)) & 127u)) & 127u);
-    // stage size: read from the kernel parameters at each use (a constant-bank
-    // operand) rather than held in a register
-#define FDTD_SB (BATCH ? bd.stage_bytes : pk.stage_bytes)
-    float *enew = reinterpret_cast<float *>(smem + NS * FDTD_SB);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NS * FDTD_SB + L::ENEW);
-    float *Nx = enew, *Ny = enew + L::ENEWC, *Nz = enew + 2 * L::ENEWC;
-    // psi ring (2 slots of 4 boxes), then the CPML tables:
-    // tab[(axis*2 + eh)*3 + {b,a,km}] has 2P[axis] entries
-    unsigned char *psiring = smem + NS * FDTD_SB + L::ENEW + 128;
-    float *tabs = reinterpret_cast<float *>(psiring + L::PSIRING);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L::OFF_BAR);
+    // CPML tables: tab[(axis*2 + eh)*3 + {b,a,km}] has 2P[axis] entries
+    float *tabs = reinterpret_cast<float *>(smem + L::OFF_TAB);
     // batched launches: parameters of the grid the current item belongs to
     __shared__ __align__(16) Params s_p;
-
-    __shared__ int s_abort;
-    __shared__ int s_nls;
+    __shared__ int s_nls, s_smin, s_smax;
     // sources of the current work item, list order: (i << 16 | j), (k << 2 | comp), list index
     __shared__ uint32_t s_ls_ij[MAX_LOCAL_SRC];
     __shared__ int s_ls_kc[MAX_LOCAL_SRC], s_ls_s[MAX_LOCAL_SRC];
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // Roles.  E phase: warps 0..TY-1 -> own row r = warp+1 (j = j0+warp), pair
-    // k = k0+2*lane; warp TY -> halo row r = 0 (j = j0-1); warp TY+1 -> halo
-    // column: lane r <= TY computes the pair at k0-2, k0-1 of row r (only the
-    // k0-1 value is used).  H phase: warps 0..TY-1, own pairs.
-    const bool col_warp = warp == TY + 1;
-    // producer: lane 0 of warp TY+2 waits on the mbarriers and issues the TMA
-    // copies, so that no stencil warp carries that work on its critical path
-    const bool producer = tid == (TY + 2) * 32;
-    const bool e_active = warp <= TY || (col_warp && lane <= TY);
-    const bool h_active = warp < TY;
-    const int er = warp < TY ? warp + 1 : (warp == TY ? 0 : lane);
-    const int eko = col_warp ? -2 : 2 * lane;  // pair start relative to k0
-    const bool own_row = warp < TY;
-
-    auto stage_ptr = [&](int st) { return smem + st * FDTD_SB; };
-    auto sH = [&](int st, int c) { return reinterpret_cast<float *>(stage_ptr(st) + c * L::HBOXB); };
-    auto sE = [&](int st, int c) { return reinterpret_cast<float *>(stage_ptr(st) + 3 * L::HBOXB + c * L::EBOXB); };
-    auto sC = [&](int st, int c) {
-        return reinterpret_cast<float *>(stage_ptr(st) + 3 * L::HBOXB + (3 + c) * L::EBOXB);
-    };
-    // psi box b (0, 1 = E psi, 2, 3 = H psi of the x or y slab) of ring slot sl
-    auto sP = [&](int sl, int b) { return reinterpret_cast<float *>(psiring + (sl * 4 + b) * L::EBOXB); };
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool own_t = tid < L::OWN, e_t = tid < L::OWN + L::HALO, producer = tid == L::PRODUCER;
+    // box row (row j0-1+er) and box column (first of the group) of this thread
+    int er = 0, col = 0;
+    if (own_t) {
+        er = 1 + tid / GZ;
+        col = 4 + 4 * (tid % GZ);
+    } else if (tid < L::OWN + GZ) {
+        col = 4 + 4 * (tid - L::OWN);
+    } else if (e_t) {
+        er = 1 + tid - L::OWN - GZ;
+    }
+    const float *const h_t = reinterpret_cast<const float *>(smem) + er * HC + col;
+    const float *const e_t0 = reinterpret_cast<const float *>(smem + L::OFF_E) + er * EC + col;
+    float *const n_t = reinterpret_cast<float *>(smem + L::OFF_N) + er * EC + col;
+    constexpr int HB = L::HBOXB / 4, EB = L::EBOXB / 4;  // component strides (floats)
     const Params &p = BATCH ? s_p : pk;
 
-    // stage the CPML coefficient tables of the current grid (a few hundred floats)
+    // stage the CPML coefficient tables of the current grid: the loads of all
+    // 18 tables are in flight together (in turn they cost 18 memory latencies)
     auto stage_tables = [&]() {
-        int off = 0;
-        auto copy = [&](const float *src, int n2) {
-            for (int x = tid; x < n2; x += blockDim.x) tabs[off + x] = src[x];
-            off += n2;
-        };
+        for (int x0 = 0; x0 < 2 * max(p.P[0], max(p.P[1], p.P[2])); x0 += L::THREADS) {
+            const int x = x0 + tid;
+            float v[18];
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            const int n2 = 2 * p.P[a];
-            copy(p.tb_e[a], n2);
-            copy(p.ta_e[a], n2);
-            copy(p.tk_e[a], n2);
-            copy(p.tb_h[a], n2);
-            copy(p.ta_h[a], n2);
-            copy(p.tk_h[a], n2);
+            for (int a = 0; a < 3; a++) {
+                const bool in = x < 2 * p.P[a];
+                const float *src[6] = {p.tb_e[a], p.ta_e[a], p.tk_e[a], p.tb_h[a], p.ta_h[a], p.tk_h[a]};
+#pragma unroll
+                for (int q = 0; q < 6; q++) v[6 * a + q] = in ? src[q][x] : 0.f;
+            }
+            int off = 0;
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                const int n2 = 2 * p.P[a];
+#pragma unroll
+                for (int q = 0; q < 6; q++)
+                    if (x < n2) tabs[off + q * n2 + x] = v[6 * a + q];
+                off += 6 * n2;
+            }
         }
     };
 
     if (tid == 0) {
-        // stage H barriers, stage E+CE barriers, then the 2 psi slots
-        for (int s = 0; s < 2 * NS + 2; s++) mbar_init(&bars[s], 1);
+        for (int s = 0; s < NS; s++) mbar_init(&bars[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (!BATCH) {
+    }
+    if (!BATCH) {
+        if (producer)
             for (int c = 0; c < 3; c++) {
                 prefetch_tmap(&mk.h[c]);
                 prefetch_tmap(&mk.e[c]);
                 prefetch_tmap(&mk.ce[c]);
             }
-            if (pk.xypsi)
-                for (int c = 0; c < 2; c++) {
-                    prefetch_tmap(&mk.xpe[c]);
-                    prefetch_tmap(&mk.xph[c]);
-                    prefetch_tmap(&mk.ype[c]);
-                    prefetch_tmap(&mk.yph[c]);
-                }
-        }
-        s_abort = 0;
+        stage_tables();
     }
-    // Per-grid values are read from p at each use: constant-bank operands for a
-    // single grid, shared-memory loads of the current grid's copy in a batch
-    // (held in registers they would be live across the whole item loop).
-    if (!BATCH) stage_tables();
 
-    uint32_t g0 = 0;          // planes this CTA has issued before the current item
-    uint32_t gp0 = 0;         // psi ring phases this CTA has used before the current item
-    int64_t issued_hi = -1;   // highest plane index (relative) issued in the current item (tid 0)
-    int64_t psi_hi = -1;      // highest plane whose psi boxes were issued (tid 0)
-    int64_t q_abort = 0, i_start_abort = 0;
+    // ring positions: stage slot and H slot of the current plane, parity of the stage
+    int es = 0, hs = 0;
+    uint32_t par = 0;
+    int q_abort = 0, q_issued = -1;
     bool aborted = false;
     const uint64_t wlim = (!BATCH && pk.wait_ns) ? pk.wait_ns : WAIT_NS;
     bool first_item = true;
@@ -492,8 +597,9 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
     int cur_sim = -1;
 
     // Batched launches take items from a queue (grids ordered with the longest
-    // items first, so the short ones fill the tail); a single grid walks its
-    // uniform items in a fixed stride.
+    // items first, so the short ones fill the tail); a single grid has one CTA
+    // an item (the hardware hands them out as CTAs end), or walks them in a
+    // fixed stride when the caller limits the CTAs per SM.
     __shared__ int s_item;
     int64_t gitem = blockIdx.x;
     if (BATCH) {
@@ -516,425 +622,491 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
             mp = &bd.maps[2 * lo + bd.cur];
             if (lo != cur_sim) {
                 __syncthreads();  // every thread is done with the previous grid's parameters
-                for (int w = tid; w < (int)(sizeof(Params) / 4); w += blockDim.x)
+                for (int w = tid; w < (int)(sizeof(Params) / 4); w += L::THREADS)
                     reinterpret_cast<int32_t *>(&s_p)[w] =
                         reinterpret_cast<const int32_t *>(&bd.params[2 * lo + bd.cur])[w];
                 __syncthreads();
-                if (tid == 0) {
-                    s_p.t = bd.t;
+                if (tid == 0) s_p.t = bd.t;
+                if (producer)
                     for (int c = 0; c < 3; c++) {
                         prefetch_tmap(&mp->h[c]);
                         prefetch_tmap(&mp->e[c]);
                         prefetch_tmap(&mp->ce[c]);
                     }
-                }
                 stage_tables();
-                __syncthreads();
                 cur_sim = lo;
             }
         }
         const TMaps &maps = *mp;
-        const int64_t tzi = item % p.ntz, tyi = (item / p.ntz) % p.nty, xci = item / ((int64_t)p.ntz * p.nty);
-        const int64_t k0 = tzi * TZ, j0 = tyi * TY;
-        const int64_t x0 = xci * p.x_chunk;
-        const int64_t x1 = min(x0 + (int64_t)p.x_chunk, p.nx);
-        const int64_t i_start = x0 > 0 ? x0 - 1 : 0;
-        const int64_t nplanes = x1 - i_start + 1;  // planes i_start .. x1 (H(x1) feeds E(x1-1))
-        // Tile-uniform: no grid edge and no y/z CPML slab inside the tile's E/H region.
-        // tile's E (k0-1..k0+TZ-1) or H (k0..k0+TZ-1) columns touch a z slab
-        // Tile-uniform: no y CPML slab among the tile's rows.  Grid edges are
-        // handled on the plain path by per-lane masks, and the z slab is the
-        // band kernels' work, so z-slab tiles are plain here too.
-        const bool y_plain = p.P[1] == 0 || ((j0 - 1 > p.P[1] || !((p.faces >> 2) & 1)) && (j0 + TY - 1 < p.ny - p.P[1] - 1 || !((p.faces >> 3) & 1)));
+        const int nx = (int)p.nx, ny = (int)p.ny, nz = (int)p.nz;
+        const int P0 = p.P[0], P1 = p.P[1], P2 = p.P[2], faces = p.faces;
+        int tzi, tyi, xci;
+        item_tile(p, (int)item, tzi, tyi, xci);
+        const int k0 = tzi * TZ, j0 = tyi * TY;
+        const int x0 = xci * p.x_chunk, x1 = min(x0 + p.x_chunk, nx);
+        const int i_start = x0 > 0 ? x0 - 1 : 0;
+        const int nit = x1 - i_start;  // planes i_start .. x1-1; H(x1) feeds E(x1-1)
 
-        // y psi by TMA for tiles whose y-slab rows lie on one side (box row r <-> j0-1+r)
-        const bool ye_f = ((p.faces >> 2) & 1) && p.P[1] > 0 && j0 - 1 <= p.P[1] && j0 + TY - 1 >= 1;
-        const bool ye_b = ((p.faces >> 3) & 1) && p.P[1] > 0 && j0 + TY - 1 >= p.ny - p.P[1] - 1 && j0 - 1 <= p.ny - 2;
-        const bool yh_f = ((p.faces >> 2) & 1) && p.P[1] > 0 && j0 <= p.P[1] && j0 + TY - 1 >= 1;
-        const bool yh_b = ((p.faces >> 3) & 1) && p.P[1] > 0 && j0 + TY - 1 >= p.ny - p.P[1] && j0 <= p.ny - 1;
-        const bool ytile = p.xypsi && (ye_f || ye_b || yh_f || yh_b) && !((ye_f || yh_f) && (ye_b || yh_b));
-        // the item's E region (planes i_start..x1-1, rows j0-1.., columns k0-1..) meets the Drude box
-        const bool dtile = EXT >= 1 && p.drude && i_start < p.dbox[0] + p.dbox[3] && x1 > p.dbox[0] &&
-                           j0 - 1 < p.dbox[1] + p.dbox[4] && j0 + TY > p.dbox[1] &&
-                           k0 - 1 < p.dbox[2] + p.dbox[5] && k0 + TZ > p.dbox[2];
-
-        // ---- per-item, per-thread cell description (pair at row j, columns k, k+1) ----
-        const int64_t jj = j0 - 1 + er, kk = k0 + eko;
-        const bool row_in = jj >= 0 && jj < p.ny;
-        const bool in0 = row_in && kk >= 0 && kk < p.nz, in1 = row_in && kk + 1 >= 0 && kk + 1 < p.nz;
-        const bool j_lt = jj < p.ny - 1, j_gt = jj > 0;
-        const bool k0_lt = kk < p.nz - 1, k1_lt = kk + 1 < p.nz - 1, k0_gt = kk > 0, k1_gt = kk + 1 > 0;
-        // lanes with a cell outside an update region (grid edges); the i edges are plane-uniform
-        const bool emask = !(j_lt && k0_lt && k1_lt), hmask = !(j_gt && k0_gt && k1_gt);
-        const int sye = row_in ? slab_e(jj, p.P[1], p.ny, ((p.faces >> 2) & 1), ((p.faces >> 3) & 1)) : -1;
-        const int syh = row_in ? slab_h(jj, p.P[1], p.ny, ((p.faces >> 2) & 1), ((p.faces >> 3) & 1)) : -1;
-        // H cells of the z band: left to the band kernel (no psi_h update here)
-        const bool hb0 = p.zfix && in_zband_h(kk, p.P[2], p.nz, ((p.faces >> 4) & 1), ((p.faces >> 5) & 1));
-        const bool hb1 = p.zfix && in_zband_h(kk + 1, p.P[2], p.nz, ((p.faces >> 4) & 1), ((p.faces >> 5) & 1));
-
-        auto issue = [&](int64_t q) {
-            const int64_t plane = i_start + q;
-            const int st = (int)((g0 + q) % NS);
-            uint64_t *bar = &bars[st], *bare = &bars[NS + st];
+        __syncthreads();  // previous item finished by every thread
+        // stage q into E slot se and H slot sh: E(q), CE(q), H(q+1) (and H(0) with
+        // stage 0).  Past the last plane the copies read zeros: H(nx) only feeds
+        // E components that are never updated at i = nx-1.
+        auto issue = [&](int q, int se, int sh) {
             if (!BATCH && first_item && blockIdx.x == 0 && q == pk.test_withhold) return;  // test hook
-            issued_hi = q;
-            if (plane >= p.nx) {
-                // Past the last plane: H(p.nx) only feeds E components that are
-                // never updated at i = p.nx-1; complete the phases without a copy.
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bare)) : "memory");
-                return;
+            q_issued = q;
+            uint64_t *bar = &bars[se];
+            mbar_arrive_expect_tx(bar, L::TX_E + (q == 0 ? 2 : 1) * L::TX_H);
+            const int xc = i_start + q;
+            unsigned char *hd = smem + sh * L::HSLOT, *ed = smem + L::OFF_E + se * L::ESLOT;
+            if (q == 0) {
+                unsigned char *h0 = smem + (sh == 0 ? L::NH - 1 : sh - 1) * L::HSLOT;
+                for (int c = 0; c < 3; c++) tma_load_3d(h0 + c * L::HBOXB, &maps.h[c], bar, k0 - 4, j0 - 1, xc);
             }
-            mbar_arrive_expect_tx(bar, L::TX_H);
-            mbar_arrive_expect_tx(bare, L::TX_E);
-            const int kc = (int)(k0 - 4), jc = (int)(j0 - 1), xc = (int)plane;
-            for (int c = 0; c < 3; c++) tma_load_3d(sH(st, c), &maps.h[c], bar, kc, jc, xc);
-            for (int c = 0; c < 3; c++) tma_load_3d(sE(st, c), &maps.e[c], bare, kc, jc, xc);
-            for (int c = 0; c < 3; c++) tma_load_3d(sC(st, c), &maps.ce[c], bare, kc, jc, xc);
+            for (int c = 0; c < 3; c++) tma_load_3d(hd + c * L::HBOXB, &maps.h[c], bar, k0 - 4, j0 - 1, xc + 1);
+            for (int c = 0; c < 3; c++) tma_load_3d(ed + c * L::EBOXB, &maps.e[c], bar, k0 - 4, j0 - 1, xc);
+            for (int c = 0; c < 3; c++)
+                tma_load_3d(ed + (3 + c) * L::EBOXB, &maps.ce[c], bar, k0 - 4, j0 - 1, xc);
         };
-        // psi boxes of plane q into ring slot (gp0+q)&1: the x slab's on x-slab
-        // planes, else the y slab's in y-slab tiles; otherwise a bare arrive
-        auto issue_psi = [&](int64_t q) {
-            const uint32_t Gp = gp0 + (uint32_t)q;
-            const int sl = (int)(Gp & 1);
-            uint64_t *bar = &bars[2 * NS + sl];
-            psi_hi = q;
-            const int64_t plane = i_start + q;
-            const int xse = plane < p.nx ? slab_e(plane, p.P[0], p.nx, (p.faces & 1), ((p.faces >> 1) & 1)) : -1;
-            const int xsh = plane < p.nx ? slab_h(plane, p.P[0], p.nx, (p.faces & 1), ((p.faces >> 1) & 1)) : -1;
-            const bool xm = p.xypsi && (xse >= 0 || xsh >= 0);
-            const bool ym = !xm && ytile && plane < p.nx;
-            const bool ye = ye_f || ye_b, yh = yh_f || yh_b;
-            const uint32_t nbox = xm ? 2u * (xse >= 0) + 2u * (xsh >= 0) : (ym ? 2u * ye + 2u * yh : 0u);
-            if (nbox == 0) {
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-                return;
+        if (producer) {
+            q_issued = -1;
+            for (int q = 0; q < NS && q < nit; q++) {
+                int se = es + q, sh = hs + q + 1;
+                if (se >= NS) se -= NS;
+                if (sh >= L::NH) sh -= L::NH;
+                issue(q, se, sh);
             }
-            mbar_arrive_expect_tx(bar, nbox * L::PSI_TX);
-            const int kc = (int)(k0 - 4), jc = (int)(j0 - 1), xc = (int)plane;
-            if (xm) {
-                if (xse >= 0) {
-                    tma_load_3d(sP(sl, 0), &maps.xpe[0], bar, kc, jc, xse);
-                    tma_load_3d(sP(sl, 1), &maps.xpe[1], bar, kc, jc, xse);
-                }
-                if (xsh >= 0) {
-                    tma_load_3d(sP(sl, 2), &maps.xph[0], bar, kc, jc, xsh);
-                    tma_load_3d(sP(sl, 3), &maps.xph[1], bar, kc, jc, xsh);
-                }
-            } else {
-                if (ye) {
-                    const int ys = ye_b ? (int)(p.P[1] + (j0 - 1) - (p.ny - p.P[1] - 1)) : (int)(j0 - 2);
-                    tma_load_3d(sP(sl, 0), &maps.ype[0], bar, kc, ys, xc);
-                    tma_load_3d(sP(sl, 1), &maps.ype[1], bar, kc, ys, xc);
-                }
-                if (yh) {
-                    const int ys = yh_b ? (int)(p.P[1] + (j0 - 1) - (p.ny - p.P[1])) : (int)(j0 - 2);
-                    tma_load_3d(sP(sl, 2), &maps.yph[0], bar, kc, ys, xc);
-                    tma_load_3d(sP(sl, 3), &maps.yph[1], bar, kc, ys, xc);
-                }
-            }
-        };
+        }
 
-        if (tid == 0) {
-            // sources inside the extended region of this work item, in list
-            // order (one thread: a warp-wide scan costs the kernel registers)
-            int n = 0;
+        // sources inside the extended region of this work item, in list order,
+        // found by one warp (32 a round: one memory latency for each round)
+        if (tid < 32) {
+            int n = 0, smin = 0x7fffffff, smax = -1;
             if (p.t >= 0 && p.t < p.namp) {
-                for (int s = 0; s < p.nsrc; s++) {
-                    const int64_t si = p.src_ijk[3 * s], sj = p.src_ijk[3 * s + 1], sk = p.src_ijk[3 * s + 2];
-                    if (si >= i_start && si < x1 && sj >= j0 - 1 && sj < j0 + TY && sk >= k0 - 1 && sk < k0 + TZ &&
-                        !(p.zfix && slab_e(sk, p.P[2], p.nz, ((p.faces >> 4) & 1), ((p.faces >> 5) & 1)) >= 0)) {
-                        if (n < MAX_LOCAL_SRC) {
-                            // packing: si, sj < 65536 (grid extents) and sk < 2^28 (checked at
-                            // plan creation), so neither field overflows
-                            s_ls_ij[n] = ((uint32_t)si << 16) | (uint32_t)sj;
-                            s_ls_kc[n] = (int)(sk << 2) | p.src_comp[s];
-                            s_ls_s[n] = s;
-                        }
-                        n++;
+                for (int s0 = 0; s0 < p.nsrc; s0 += 32) {
+                    const int s = s0 + lane;
+                    bool in = false;
+                    int si = 0, sj = 0, sk = 0;
+                    if (s < p.nsrc) {
+                        si = p.src_ijk[3 * s];
+                        sj = p.src_ijk[3 * s + 1];
+                        sk = p.src_ijk[3 * s + 2];
+                        in = si >= i_start && si < x1 && sj >= j0 - 1 && sj < j0 + TY && sk >= k0 - 1 && sk < k0 + TZ &&
+                             !(p.zfix && slab_e(sk, P2, nz, (faces >> 4) & 1, (faces >> 5) & 1) >= 0);
                     }
+                    const uint32_t m = __ballot_sync(0xffffffffu, in);
+                    const int at = n + __popc(m & ((1u << lane) - 1));
+                    if (in && at < MAX_LOCAL_SRC) {
+                        // packing: si, sj < 65536 (grid extents) and sk < 2^28 (checked at
+                        // plan creation), so neither field overflows
+                        s_ls_ij[at] = ((uint32_t)si << 16) | (uint32_t)sj;
+                        s_ls_kc[at] = (sk << 2) | p.src_comp[s];
+                        s_ls_s[at] = s;
+                    }
+                    if (in) {
+                        smin = min(smin, si);
+                        smax = max(smax, si);
+                    }
+                    n += __popc(m);
                 }
+                smin = __reduce_min_sync(0xffffffffu, smin);
+                smax = __reduce_max_sync(0xffffffffu, smax);
+            }
+            if (lane == 0) {
                 if (n > MAX_LOCAL_SRC) {  // the host rejects such layouts; never drop a source silently
                     atomicExch(p.status, FDTD_ERR_CAPACITY);
                     n = MAX_LOCAL_SRC;
                 }
+                s_nls = n;
+                s_smin = smin;
+                s_smax = smax;
             }
-            s_nls = n;
         }
-        __syncthreads();  // previous item finished by every thread; source list ready
-        if (producer) {
-            for (int64_t q = 0; q < NS && q < nplanes; q++) issue(q);
-            if (nplanes > 1) issue_psi(0);
+        __syncthreads();  // source list and tables ready
+        const int nls = s_nls, smin = s_smin, smax = s_smax;
+
+        // ---- per-item, per-thread description of the group (row jj, cells kk .. kk+3) ----
+        const int jj = j0 - 1 + er, kk = k0 - 4 + col;
+        const bool row_in = e_t && jj >= 0 && jj < ny;
+        const bool j_lt = jj < ny - 1, j_gt = jj > 0;
+        uint32_t inm = 0, ltm = 0, gtm = 0, hbm = 0;  // cells in the grid, with k < nz-1, with k > 0, in the H band
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int k = kk + e;
+            inm |= (uint32_t)(row_in && k >= 0 && k < nz) << e;
+            ltm |= (uint32_t)(k < nz - 1) << e;
+            gtm |= (uint32_t)(k > 0) << e;
+            hbm |= (uint32_t)(p.zfix && in_zband_h(k, P2, nz, (faces >> 4) & 1, (faces >> 5) & 1)) << e;
         }
-        const int nls = s_nls;
+        const bool emask = !(j_lt && ltm == 0xFu), hmask = !(j_gt && gtm == 0xFu);
+        const int sye = row_in ? slab_e(jj, P1, ny, (faces >> 2) & 1, (faces >> 3) & 1) : -1;
+        const int syh = own_t && row_in ? slab_h(jj, P1, ny, (faces >> 2) & 1, (faces >> 3) & 1) : -1;
+        const bool zin = ZIN && P2 > 0 && !p.zfix;
+        const ZSlab ze = zslab(kk, zin ? P2 : 0, nz, (faces >> 4) & 1, (faces >> 5) & 1, true, inm);
+        const ZSlab zh = zslab(kk, zin ? P2 : 0, nz, (faces >> 4) & 1, (faces >> 5) & 1, false, own_t ? inm : 0u);
+        const bool vpsi = p.vpsi != 0;
+        // the item's E region (planes i_start..x1-1, rows j0-1.., columns k0-1..) meets the Drude box
+        const bool dtile = DRUDE && p.drude && i_start < p.dbox[0] + p.dbox[3] && x1 > p.dbox[0] &&
+                           j0 - 1 < p.dbox[1] + p.dbox[4] && j0 + TY > p.dbox[1] &&
+                           k0 - 1 < p.dbox[2] + p.dbox[5] && k0 + TZ > p.dbox[2];
+        uint32_t dmask = 0;  // cells of the group in the box's columns, when its row is in the box
+        if (DRUDE && dtile && jj >= p.dbox[1] && jj < p.dbox[1] + p.dbox[4])
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                dmask |= (uint32_t)(bit(inm, e) && kk + e >= p.dbox[2] && kk + e < p.dbox[2] + p.dbox[5]) << e;
         // TFSF faces in this item (E faces at p1-1 and p2, H faces at p1 and p2): the tile's
         // rows and columns meet the box's y/z extent [p1-1, p2], and then either hold a y or
         // z face row/column (all planes of the box's x extent) or, per plane, an x face plane
-        const bool t_rows = EXT >= 2 && p.tfsf && j0 - 1 <= p.tp2[1] && j0 + TY - 1 >= p.tp1[1] - 1 &&
+        const bool t_rows = TFSF && p.tfsf && j0 - 1 <= p.tp2[1] && j0 + TY - 1 >= p.tp1[1] - 1 &&
                             k0 - 1 <= p.tp2[2] && k0 + TZ - 1 >= p.tp1[2] - 1;
-        auto holds = [](int64_t lo, int64_t hi, int64_t v) { return v >= lo && v <= hi; };
+        auto holds = [](int lo, int hi, int v) { return v >= lo && v <= hi; };
         const bool t_yz = t_rows && i_start <= p.tp2[0] && x1 - 1 >= p.tp1[0] - 1 &&
                           (holds(j0 - 1, j0 + TY - 1, p.tp1[1] - 1) || holds(j0 - 1, j0 + TY - 1, p.tp1[1]) ||
                            holds(j0 - 1, j0 + TY - 1, p.tp2[1]) || holds(k0 - 1, k0 + TZ - 1, p.tp1[2] - 1) ||
                            holds(k0 - 1, k0 + TZ - 1, p.tp1[2]) || holds(k0 - 1, k0 + TZ - 1, p.tp2[2]));
-        // TFSF face codes of the pair (E, H), zero outside the box's faces
-        const uint32_t tcode_e = t_rows ? tfsf_lane_codes(p, 0, jj, kk, in0, in1) : 0u;
-        const uint32_t tcode_h = t_rows && h_active ? tfsf_lane_codes(p, 1, jj, kk, in0, in1) : 0u;
-        const bool tile_plain = y_plain && nls == 0 && !dtile;
+        // plane-uniform: an x face plane; any TFSF correction on this plane
+        auto tfsf_x = [&](int i) { return i == p.tp1[0] - 1 || i == p.tp1[0] || i == p.tp2[0]; };
+        auto tfsf_plane = [&](int i) {
+            return TFSF && t_rows && (tfsf_x(i) || (t_yz && i >= p.tp1[0] - 1 && i <= p.tp2[0]));
+        };
+        // TFSF face codes of the group's two pairs (E, H), zero outside the box's faces
+        uint32_t te0 = 0, te1 = 0, th0 = 0, th1 = 0;
+        if (TFSF && t_rows) {
+            te0 = tfsf_lane_codes(p, 0, jj, kk, bit(inm, 0), bit(inm, 1));
+            te1 = tfsf_lane_codes(p, 0, jj, kk + 2, bit(inm, 2), bit(inm, 3));
+            if (own_t) {
+                th0 = tfsf_lane_codes(p, 1, jj, kk, bit(inm, 0), bit(inm, 1));
+                th1 = tfsf_lane_codes(p, 1, jj, kk + 2, bit(inm, 2), bit(inm, 3));
+            }
+        }
 
-        float2 prev_ey = make_float2(0.f, 0.f), prev_ez = make_float2(0.f, 0.f);
-        float2 oex = prev_ey, oey = prev_ey, oez = prev_ey;  // own E_new pair
-        for (int64_t q = 0; q + 1 < nplanes; q++) {
-            const int64_t i = i_start + q;
-            const uint32_t G = g0 + (uint32_t)q;
-            const int st = (int)(G % NS), st1 = (int)((G + 1) % NS);
-            const uint32_t par = (G / NS) & 1, par1 = ((G + 1) / NS) & 1;
-            const uint32_t Gp = gp0 + (uint32_t)q;
-            const int psl = (int)(Gp & 1);
-            // The producer waits for the copies; the barrier then releases the CTA
-            // (its mbarrier acquire plus bar.sync order the TMA writes before
-            // every thread's reads).  Plane q+1 is needed for its H only:
-            // its E and CE have one more iteration to arrive.
-            if (producer &&
-                (!mbar_wait_bounded(&bars[st], par, p.status, wlim) ||
-                 !mbar_wait_bounded(&bars[st1], par1, p.status, wlim) ||
-                 !mbar_wait_bounded(&bars[NS + st], par, p.status, wlim) ||
-                 !mbar_wait_bounded(&bars[2 * NS + psl], (Gp >> 1) & 1, p.status, wlim)))
-                s_abort = 1;
-            __syncthreads();  // (A) H of planes q, q+1, E and CE of q visible; iteration q-1 finished everywhere
-            if (s_abort) {
+        V4 hyc{}, hzc{};                // own hy, hz of the current plane
+        V4 prev_ey{}, prev_ez{};        // E_new of the plane before
+        int nb = 0;                     // E_new buffer
+        // planes that need more than the curl updates: all of them in tiles of a y or z
+        // slab, else the x-slab, Drude, TFSF and source planes
+        const bool tile_gen = __syncthreads_or(sye >= 0 || syh >= 0 || (ZIN && (ze.m || zh.m)));
+        // One plane: E phase, barrier, H phase.  Two copies of the code (gen: with the CPML,
+        // Drude, TFSF and source terms): most planes run the short one, which fits the
+        // instruction cache.  Returns false when a wait ran out.
+        auto plane = [&](auto gen_c, int q, bool late) -> bool {
+            constexpr bool gen = decltype(gen_c)::value;
+            const int i = i_start + q;
+            const bool i_lt = i < nx - 1, i_gt = i > 0, own = own_t && i >= x0;
+            // plane-uniform: x slab nodes
+            const int sxe = gen ? slab_e(i, P0, nx, faces & 1, (faces >> 1) & 1) : -1,
+                      sxh = gen ? slab_h(i, P0, nx, faces & 1, (faces >> 1) & 1) : -1;
+            // psi of this plane's slab cells: E psi now, H psi before the barrier below
+            // (px, py, pz: the two arrays of the x, y and z slab)
+            V4 px0{}, px1{}, py0{}, py1{}, pz0{}, pz1{};
+            const int64_t qx = ((int64_t)(sxe >= 0 ? sxe : 0) * ny + jj) * nz + kk;
+            const int64_t qy = ((int64_t)i * 2 * P1 + (sye >= 0 ? sye : 0)) * nz + kk;
+            const int64_t qz = ((int64_t)i * ny + jj) * 2 * P2;
+            if (sxe >= 0) {
+                px0 = ldg4(p.psi_e_in[0], qx, inm, vpsi, pext_y(p, 0));
+                px1 = ldg4(p.psi_e_in[1], qx, inm, vpsi, pext_y(p, 1));
+            }
+            if (gen && sye >= 0) {
+                py0 = ldg4(p.psi_e_in[2], qy, inm, vpsi, pext_y(p, 2));
+                py1 = ldg4(p.psi_e_in[3], qy, inm, vpsi, pext_y(p, 3));
+            }
+            if (ZIN && gen && ze.m) {
+                pz0 = ldz4(p.psi_e_in[4], qz, ze.m, ze, pext_y(p, 4));
+                pz1 = ldz4(p.psi_e_in[5], qz, ze.m, ze, pext_y(p, 5));
+            }
+            if (gen && q + 1 < nit) {
+                // the next plane's psi into L2: one plane is long enough for DRAM, and the
+                // loads above and before the barrier then wait for L2 only
+                const int64_t dx = (int64_t)ny * nz, dy = (int64_t)2 * P1 * nz, dz = (int64_t)ny * 2 * P2;
+                if (inm) {
+                    if (sxe >= 0 && sxe + 1 < 2 * P0) {
+                        prefetch_l2(p.psi_e_in[0] + qx + dx);
+                        prefetch_l2(p.psi_e_in[1] + qx + dx);
+                    }
+                    if (sye >= 0) {
+                        prefetch_l2(p.psi_e_in[2] + qy + dy);
+                        prefetch_l2(p.psi_e_in[3] + qy + dy);
+                    }
+                    if (ZIN && ze.m) {
+                        prefetch_l2(p.psi_e_in[4] + qz + dz + ze.s(__ffs(ze.m) - 1));
+                        prefetch_l2(p.psi_e_in[5] + qz + dz + ze.s(__ffs(ze.m) - 1));
+                    }
+                    if (own_t) {
+                        if (sxh >= 0 && sxh + 1 < 2 * P0) {
+                            const int64_t u = ((int64_t)(sxh + 1) * ny + jj) * nz + kk;
+                            prefetch_l2(p.psi_h[0] + u);
+                            prefetch_l2(p.psi_h[1] + u);
+                        }
+                        if (syh >= 0) {
+                            const int64_t u = ((int64_t)(i + 1) * 2 * P1 + syh) * nz + kk;
+                            prefetch_l2(p.psi_h[2] + u);
+                            prefetch_l2(p.psi_h[3] + u);
+                        }
+                        if (ZIN && zh.m) {
+                            prefetch_l2(p.psi_h[4] + qz + dz + zh.s(__ffs(zh.m) - 1));
+                            prefetch_l2(p.psi_h[5] + qz + dz + zh.s(__ffs(zh.m) - 1));
+                        }
+                    }
+                }
+            }
+            const bool dplane = gen && DRUDE && dmask && i >= p.dbox[0] && i < p.dbox[0] + p.dbox[3];
+            int64_t jb = 0;
+            if (gen && DRUDE && dplane) {
+                jb = ((i - p.dbox[0]) * p.dbox[4] + (jj - p.dbox[1])) * p.dbox[5] - p.dbox[2] + kk;
+                if (q + 1 < nit && i + 1 < p.dbox[0] + p.dbox[3]) {  // the next plane's box arrays into L2
+                    const int64_t u = jb + p.dbox[4] * p.dbox[5] + __ffs(dmask) - 1;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        prefetch_l2(p.dj_in[c] + u);
+                        prefetch_l2(p.dcja[c] + u);
+                        prefetch_l2(p.dcjb[c] + u);
+                    }
+                }
+            }
+
+            const float *H0 = h_t + hs * (L::HSLOT / 4);
+            const float *H1 = h_t + (hs + 1 == L::NH ? 0 : hs + 1) * (L::HSLOT / 4);
+            const float *E0 = e_t0 + es * (L::ESLOT / 4);
+            float *N0 = n_t + nb * (3 * EB);
+            // TFSF corrections on this plane; the codes of the x faces (ey, ez / hy, hz slots)
+            // count on the face planes only
+            const bool tplane = gen && TFSF && tfsf_plane(i);
+            const uint32_t tx = gen && TFSF && tfsf_x(i) ? 0xfffu : 0xfffu & ~0x330u;
+            // (a loop over the cells: one copy of the correction's code a phase)
+            auto tfsf_group = [&](int eh, uint32_t c0, uint32_t c1, V4 &vx, V4 &vy, V4 &vz) {
+                if (!(c0 | c1)) return;
+#pragma unroll 1
+                for (int e = 0; e < 4; e++) {
+                    const uint32_t c = ((e < 2 ? c0 : c1) >> (e & 1 ? 12 : 0)) & tx;
+                    if (!c) continue;
+                    float x = vx.v[0], y = vy.v[0], z = vz.v[0];
+#pragma unroll
+                    for (int u = 1; u < 4; u++) {
+                        x = u == e ? vx.v[u] : x;
+                        y = u == e ? vy.v[u] : y;
+                        z = u == e ? vz.v[u] : z;
+                    }
+                    tfsf_apply(p, eh, c, i, jj, kk + e, x, y, z);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        vx.v[u] = u == e ? x : vx.v[u];
+                        vy.v[u] = u == e ? y : vy.v[u];
+                        vz.v[u] = u == e ? z : vz.v[u];
+                    }
+                }
+            };
+            // ---- E phase ----
+            V4 hx{}, hy1{}, hz1{}, ex{}, ey{}, ez{};
+            if (e_t) {
+                if (q == 0) {
+                    hyc = lds4(H0 + HB);
+                    hzc = lds4(H0 + 2 * HB);
+                }
+                hx = lds4(H0);
+                hy1 = lds4(H1 + HB);
+                hz1 = lds4(H1 + 2 * HB);
+                const V4 hxj = lds4(H0 + HC), hzj = lds4(H0 + 2 * HB + HC);
+                const float hxk4 = H0[4], hyk4 = H0[HB + 4];
+                const V4 ex0 = lds4(E0), ey0 = lds4(E0 + EB), ez0 = lds4(E0 + 2 * EB);
+                const V4 cx = lds4(E0 + 3 * EB), cy = lds4(E0 + 4 * EB), cz = lds4(E0 + 5 * EB);
+                auto hxk = [&](int e) { return e < 3 ? hx.v[e + 1] : hxk4; };
+                auto hyk = [&](int e) { return e < 3 ? hyc.v[e + 1] : hyk4; };
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    ex.v[e] = fadd(ex0.v[e], fmul(cx.v[e], curl4(hzj.v[e], hzc.v[e], hyk(e), hyc.v[e])));
+                    ey.v[e] = fadd(ey0.v[e], fmul(cy.v[e], curl4(hxk(e), hx.v[e], hz1.v[e], hzc.v[e])));
+                    ez.v[e] = fadd(ez0.v[e], fmul(cz.v[e], curl4(hy1.v[e], hyc.v[e], hxj.v[e], hx.v[e])));
+                }
+                if (!i_lt || emask) {
+                    // component masks (cells the reference does not update keep their value)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        if (!(j_lt && bit(ltm, e))) ex.v[e] = ex0.v[e];
+                        if (!(i_lt && bit(ltm, e))) ey.v[e] = ey0.v[e];
+                        if (!(i_lt && j_lt)) ez.v[e] = ez0.v[e];
+                    }
+                }
+                if (gen && DRUDE && dplane) {  // Drude ADE, before the CPML terms
+                    [[maybe_unused]] const int64_t nd = p.dbox[3] * p.dbox[4] * p.dbox[5];
+                    const bool dv = p.dvec != 0;
+                    V4 dj[3], da[3], db[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        dj[c] = ldg4(p.dj_in[c], jb, dmask, dv, nd);
+                        da[c] = ldg4(p.dcja[c], jb, dmask, dv, nd);
+                        db[c] = ldg4(p.dcjb[c], jb, dmask, dv, nd);
+                    }
+                    auto ade = [&](V4 &v, const V4 &cf, int c) {
+                        V4 jn;
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const float n = drude_cell(v.v[e], cf.v[e], dj[c].v[e], da[c].v[e], db[c].v[e], jn.v[e]);
+                            v.v[e] = bit(dmask, e) ? n : v.v[e];
+                        }
+                        if (own) stg4(p.dj_out[c], jb, dmask, dv, jn, nd);
+                    };
+                    ade(ex, cx, 0);
+                    ade(ey, cy, 1);
+                    ade(ez, cz, 2);
+                }
+                if (gen && sxe >= 0) {  // x slab: ey -= cey (..dHz/dx..), ez += cez (..dHy/dx..)
+                    const Coef c = tab_coef(tabs, 0, 2 * P0, 0, sxe);
+                    const uint32_t m0 = inm & ltm, m1 = j_lt ? inm : 0u;
+                    slab_term<-1>(ey, cy, px0, c, hz1, hzc, m0);
+                    slab_term<+1>(ez, cz, px1, c, hy1, hyc, m1);
+                    if (own) {
+                        stg4(p.psi_e_out[0], qx, m0, vpsi, px0, pext_y(p, 0));
+                        stg4(p.psi_e_out[1], qx, m1, vpsi, px1, pext_y(p, 1));
+                    }
+                }
+                if (gen && sye >= 0) {  // y slab: ez -= cez (..dHx/dy..), ex += cex (..dHz/dy..)
+                    const Coef c = tab_coef(tabs, 12 * P0, 2 * P1, 0, sye);
+                    const uint32_t m0 = i_lt ? inm : 0u, m1 = inm & ltm;
+                    slab_term<-1>(ez, cz, py0, c, hxj, hx, m0);
+                    slab_term<+1>(ex, cx, py1, c, hzj, hzc, m1);
+                    if (own) {
+                        stg4(p.psi_e_out[2], qy, m0, vpsi, py0, pext_y(p, 2));
+                        stg4(p.psi_e_out[3], qy, m1, vpsi, py1, pext_y(p, 3));
+                    }
+                }
+                if (ZIN && gen && ze.m) {  // z slab: ex -= cex (..dHy/dz..), ey += cey (..dHx/dz..)
+                    const uint32_t m0 = j_lt ? ze.m : 0u, m1 = i_lt ? ze.m : 0u;
+                    const V4 hxs{{hx.v[1], hx.v[2], hx.v[3], hxk4}}, hys{{hyc.v[1], hyc.v[2], hyc.v[3], hyk4}};
+                    z_term<-1>(ex, cx, pz0, tabs + 12 * (P0 + P1), 2 * P2, ze, hys, hyc, m0);
+                    z_term<+1>(ey, cy, pz1, tabs + 12 * (P0 + P1), 2 * P2, ze, hxs, hx, m1);
+                    if (own) {
+                        stz4(p.psi_e_out[4], qz, m0, ze, pz0, pext_y(p, 4));
+                        stz4(p.psi_e_out[5], qz, m1, ze, pz1, pext_y(p, 5));
+                    }
+                }
+                // TFSF: E += 0.5 (c * H1d), after the CPML terms, before the sources
+                if (gen && TFSF && tplane) tfsf_group(0, te0, te1, ex, ey, ez);
+                if (gen && i >= smin && i <= smax) {  // soft sources, list order
+                    const uint32_t ij_here = ((uint32_t)i << 16) | (uint32_t)jj;
+                    for (int s = 0; s < nls; s++) {
+                        if (s_ls_ij[s] != ij_here) continue;
+                        const int kc = s_ls_kc[s], d = (kc >> 2) - kk;
+                        if (d < 0 || d > 3) continue;
+                        const float v = p.src_amp[(int64_t)s_ls_s[s] * p.namp + p.t];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            if (e != d) continue;
+                            if ((kc & 3) == 0) ex.v[e] = fadd(ex.v[e], v);
+                            else if ((kc & 3) == 1) ey.v[e] = fadd(ey.v[e], v);
+                            else ez.v[e] = fadd(ez.v[e], v);
+                        }
+                    }
+                }
+                sts4(N0, ex);
+                sts4(N0 + EB, ey);
+                sts4(N0 + 2 * EB, ez);
+            }
+            // H psi of the slab cells (in place: only this thread touches them)
+            const int64_t ux = ((int64_t)(sxh >= 0 ? sxh : 0) * ny + jj) * nz + kk;
+            const int64_t uy = ((int64_t)i * 2 * P1 + (syh >= 0 ? syh : 0)) * nz + kk;
+            if (own) {
+                if (gen && sxh >= 0) {
+                    px0 = ldg4(p.psi_h[0], ux, inm, vpsi, pext_y(p, 0));
+                    px1 = ldg4(p.psi_h[1], ux, inm, vpsi, pext_y(p, 1));
+                }
+                if (gen && syh >= 0) {
+                    py0 = ldg4(p.psi_h[2], uy, inm, vpsi, pext_y(p, 2));
+                    py1 = ldg4(p.psi_h[3], uy, inm, vpsi, pext_y(p, 3));
+                }
+                if (ZIN && gen && zh.m) {
+                    pz0 = ldz4(p.psi_h[4], qz, zh.m, zh, pext_y(p, 4));
+                    pz1 = ldz4(p.psi_h[5], qz, zh.m, zh, pext_y(p, 5));
+                }
+            }
+            // E_new of plane i visible; E(q), CE(q) and H(q) read by every thread; the
+            // barrier also agrees on whether any thread's wait ran out
+            if (__syncthreads_or(late)) {
+                return false;
+            }
+            if (producer && q + NS < nit) issue(q + NS, es, hs);
+
+            // ---- H phase ----
+            if (own) {
+                const V4 ez_j = lds4(N0 + 2 * EB - EC), ex_j = lds4(N0 - EC);
+                const float eyk0 = N0[EB - 1], exk0 = N0[-1];
+                auto ey_k = [&](int e) { return e ? ey.v[e - 1] : eyk0; };
+                auto ex_k = [&](int e) { return e ? ex.v[e - 1] : exk0; };
+                V4 ox, oy, oz;  // H_new
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    ox.v[e] = fsub(hx.v[e], fmul(0.5f, curl4(ez.v[e], ez_j.v[e], ey.v[e], ey_k(e))));
+                    oy.v[e] = fsub(hyc.v[e], fmul(0.5f, curl4(ex.v[e], ex_k(e), ez.v[e], prev_ez.v[e])));
+                    oz.v[e] = fsub(hzc.v[e], fmul(0.5f, curl4(ey.v[e], prev_ey.v[e], ex.v[e], ex_j.v[e])));
+                }
+                if (!i_gt || hmask) {
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        if (!(j_gt && bit(gtm, e))) ox.v[e] = hx.v[e];
+                        if (!(i_gt && bit(gtm, e))) oy.v[e] = hyc.v[e];
+                        if (!(i_gt && j_gt)) oz.v[e] = hzc.v[e];
+                    }
+                }
+                const V4 half{{0.5f, 0.5f, 0.5f, 0.5f}};
+                if (gen && sxh >= 0) {  // x slab: hy += (..dEz/dx..), hz -= (..dEy/dx..)
+                    const Coef c = tab_coef(tabs, 0, 2 * P0, 1, sxh);
+                    const uint32_t m0 = inm & gtm & ~hbm, m1 = j_gt ? inm & ~hbm : 0u;
+                    slab_term<+1>(oy, half, px0, c, ez, prev_ez, m0);
+                    slab_term<-1>(oz, half, px1, c, ey, prev_ey, m1);
+                    stg4(p.psi_h[0], ux, m0, vpsi, px0, pext_y(p, 0));
+                    stg4(p.psi_h[1], ux, m1, vpsi, px1, pext_y(p, 1));
+                }
+                if (gen && syh >= 0) {  // y slab: hz += (..dEx/dy..), hx -= (..dEz/dy..)
+                    const Coef c = tab_coef(tabs, 12 * P0, 2 * P1, 1, syh);
+                    const uint32_t m0 = i_gt ? inm & ~hbm : 0u, m1 = inm & gtm & ~hbm;
+                    slab_term<+1>(oz, half, py0, c, ex, ex_j, m0);
+                    slab_term<-1>(ox, half, py1, c, ez, ez_j, m1);
+                    stg4(p.psi_h[2], uy, m0, vpsi, py0, pext_y(p, 2));
+                    stg4(p.psi_h[3], uy, m1, vpsi, py1, pext_y(p, 3));
+                }
+                if (ZIN && gen && zh.m) {  // z slab: hx += (..dEy/dz..), hy -= (..dEx/dz..)
+                    const uint32_t m0 = j_gt ? zh.m : 0u, m1 = i_gt ? zh.m : 0u;
+                    const V4 eys{{eyk0, ey.v[0], ey.v[1], ey.v[2]}}, exs{{exk0, ex.v[0], ex.v[1], ex.v[2]}};
+                    z_term<+1>(ox, half, pz0, tabs + 12 * (P0 + P1) + 6 * P2, 2 * P2, zh, ey, eys, m0);
+                    z_term<-1>(oy, half, pz1, tabs + 12 * (P0 + P1) + 6 * P2, 2 * P2, zh, ex, exs, m1);
+                    stz4(p.psi_h[4], qz, m0, zh, pz0, pext_y(p, 4));
+                    stz4(p.psi_h[5], qz, m1, zh, pz1, pext_y(p, 5));
+                }
+                // TFSF: H += 0.5 (c * E1d), after the CPML terms
+                if (gen && TFSF && tplane) tfsf_group(1, th0, th1, ox, oy, oz);
+                const int64_t gi = (int64_t)i * p.sx + (int64_t)jj * p.sy + kk;
+                stg4(p.out[0], gi, inm, true, ex, fext_y(p));
+                stg4(p.out[1], gi, inm, true, ey, fext_y(p));
+                stg4(p.out[2], gi, inm, true, ez, fext_y(p));
+                stg4(p.out[3], gi, inm, true, ox, fext_y(p));
+                stg4(p.out[4], gi, inm, true, oy, fext_y(p));
+                stg4(p.out[5], gi, inm, true, oz, fext_y(p));
+            }
+            prev_ey = ey;
+            prev_ez = ez;
+            hyc = hy1;
+            hzc = hz1;
+            nb ^= 1;
+            return true;
+        };
+        for (int q = 0; q < nit; q++) {
+            const int i = i_start + q;
+            // E(q), CE(q) and H(q+1) have arrived (H(q) with the stage before)
+            const bool late = !mbar_wait_bounded(&bars[es], par, p.status, wlim);
+            const bool gen = tile_gen || (P0 > 0 && (i <= P0 || i >= nx - P0 - 1)) || (i >= smin && i <= smax) ||
+                             (DRUDE && dtile && i >= p.dbox[0] && i < p.dbox[0] + p.dbox[3]) || (TFSF && tfsf_plane(i));
+            if (!(gen ? plane(std::true_type{}, q, late) : plane(std::false_type{}, q, late))) {
                 aborted = true;
                 q_abort = q;
-                i_start_abort = i_start;
                 break;
             }
-            if (producer) {
-                if (q >= 1 && q - 1 + NS < nplanes) issue(q - 1 + NS);  // reuse plane q-1's stage
-                if (q + 2 < nplanes) issue_psi(q + 1);                  // reuse plane q-1's psi slot
+            if (++es == NS) {
+                es = 0;
+                par ^= 1;
             }
-
-            // plane-uniform CPML (x) and masks
-            const int sxe = slab_e(i, p.P[0], p.nx, (p.faces & 1), ((p.faces >> 1) & 1)), sxh = slab_h(i, p.P[0], p.nx, (p.faces & 1), ((p.faces >> 1) & 1));
-            const bool i_lt = i < p.nx - 1, i_gt = i > 0;
-            // plane-uniform: TFSF corrections on this plane
-            const bool ttile = t_rows && ((t_yz && i >= p.tp1[0] - 1 && i <= p.tp2[0]) ||
-                                          i == p.tp1[0] - 1 || i == p.tp1[0] || i == p.tp2[0]);
-            const bool e_plain = tile_plain && i_lt && sxe < 0 && !ttile;
-            const bool h_plain = tile_plain && i_gt && sxh < 0 && !ttile;
-            // where this plane's x/y psi come from (the choice of issue_psi)
-            const bool xm = p.xypsi && (sxe >= 0 || sxh >= 0);
-            const bool ym = !xm && ytile;
-
-            // ---- E phase ----
-            if (e_active) {
-                const int hc = 4 + eko;
-                const float *HX = sH(st, 0) + er * HC + hc, *HY = sH(st, 1) + er * HC + hc,
-                            *HZ = sH(st, 2) + er * HC + hc;
-                const float2 hx = ld2(HX), hy = ld2(HY), hz = ld2(HZ);
-                const float2 hxj1 = ld2(HX + HC), hzj1 = ld2(HZ + HC);
-                const float2 hxk1 = make_float2(HX[1], HX[2]), hyk1 = make_float2(HY[1], HY[2]);
-                const float2 hy1 = ld2(sH(st1, 1) + er * HC + hc), hz1 = ld2(sH(st1, 2) + er * HC + hc);
-                const int ei = er * EC + hc;
-                const float2 ex0 = ld2(sE(st, 0) + ei), ey0 = ld2(sE(st, 1) + ei), ez0 = ld2(sE(st, 2) + ei);
-                const float2 cex = ld2(sC(st, 0) + ei), cey = ld2(sC(st, 1) + ei), cez = ld2(sC(st, 2) + ei);
-                float2 ex = add2(ex0, mul2(cex, curl4x2(hzj1, hz, hyk1, hy)));
-                float2 ey = add2(ey0, mul2(cey, curl4x2(hxk1, hx, hz1, hz)));
-                float2 ez = add2(ez0, mul2(cez, curl4x2(hy1, hy, hxj1, hx)));
-                if (!e_plain || emask) {
-                    // component masks (cells the reference does not update keep their value)
-                    if (!(j_lt && k0_lt)) ex.x = ex0.x;
-                    if (!(j_lt && k1_lt)) ex.y = ex0.y;
-                    if (!(i_lt && k0_lt)) ey.x = ey0.x;
-                    if (!(i_lt && k1_lt)) ey.y = ey0.y;
-                    if (!(i_lt && j_lt)) {
-                        ez.x = ez0.x;
-                        ez.y = ez0.y;
-                    }
-                }
-                if (!e_plain) {
-                    const bool own = own_row && i >= x0;
-                    if (dtile && i >= p.dbox[0] && i < p.dbox[0] + p.dbox[3] && jj >= p.dbox[1] &&
-                        jj < p.dbox[1] + p.dbox[4]) {  // Drude ADE, before the CPML terms
-                        const int64_t jb = ((i - p.dbox[0]) * p.dbox[4] + (jj - p.dbox[1])) * p.dbox[5] - p.dbox[2];
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const int64_t k = kk + e;
-                            if (!(e ? in1 : in0) || k < p.dbox[2] || k >= p.dbox[2] + p.dbox[5]) continue;
-                            float jn;
-                            set(ex, e, drude_cell(get(ex, e), get(cex, e), p.dj_in[0][jb + k], p.dcja[0][jb + k],
-                                                  p.dcjb[0][jb + k], jn));
-                            if (own) p.dj_out[0][jb + k] = jn;
-                            set(ey, e, drude_cell(get(ey, e), get(cey, e), p.dj_in[1][jb + k], p.dcja[1][jb + k],
-                                                  p.dcjb[1][jb + k], jn));
-                            if (own) p.dj_out[1][jb + k] = jn;
-                            set(ez, e, drude_cell(get(ez, e), get(cez, e), p.dj_in[2][jb + k], p.dcja[2][jb + k],
-                                                  p.dcjb[2][jb + k], jn));
-                            if (own) p.dj_out[2][jb + k] = jn;
-                        }
-                    }
-                    if (sxe >= 0) {  // x slab: ey -= cey (..dHz/dx..), ez += cez (..dHy/dx..)
-                        const Coef c = tab_coef(tabs, 0, 2 * p.P[0], 0, sxe);
-                        const int64_t qb = ((int64_t)sxe * p.ny + jj) * p.nz + kk;
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            if (!(e ? in1 : in0)) continue;
-                            if (e ? k1_lt : k0_lt) {
-                                float psi = xm ? sP(psl, 0)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 0)) ? p.psi_e_in[0][qb + e] : 0.f);
-                                const float tc = corr(psi, c, fsub(get(hz1, e), get(hz, e)));
-                                if (own) if (FDTD_IN(qb + e, pext_y(p, 0))) p.psi_e_out[0][qb + e] = psi;
-                                set(ey, e, fsub(get(ey, e), fmul(get(cey, e), tc)));
-                            }
-                            if (j_lt) {
-                                float psi = xm ? sP(psl, 1)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 1)) ? p.psi_e_in[1][qb + e] : 0.f);
-                                const float tc = corr(psi, c, fsub(get(hy1, e), get(hy, e)));
-                                if (own) if (FDTD_IN(qb + e, pext_y(p, 1))) p.psi_e_out[1][qb + e] = psi;
-                                set(ez, e, fadd(get(ez, e), fmul(get(cez, e), tc)));
-                            }
-                        }
-                    }
-                    if (sye >= 0) {  // y slab: ez -= cez (..dHx/dy..), ex += cex (..dHz/dy..)
-                        const Coef cye = tab_coef(tabs, (12 * p.P[0]), 2 * p.P[1], 0, sye);
-                        const int64_t qb = (i * 2 * p.P[1] + sye) * p.nz + kk;
-#pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            if (!(e ? in1 : in0)) continue;
-                            if (i_lt) {
-                                float psi = ym ? sP(psl, 0)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 2)) ? p.psi_e_in[2][qb + e] : 0.f);
-                                const float tc = corr(psi, cye, fsub(get(hxj1, e), get(hx, e)));
-                                if (own) if (FDTD_IN(qb + e, pext_y(p, 2))) p.psi_e_out[2][qb + e] = psi;
-                                set(ez, e, fsub(get(ez, e), fmul(get(cez, e), tc)));
-                            }
-                            if (e ? k1_lt : k0_lt) {
-                                float psi = ym ? sP(psl, 1)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 3)) ? p.psi_e_in[3][qb + e] : 0.f);
-                                const float tc = corr(psi, cye, fsub(get(hzj1, e), get(hz, e)));
-                                if (own) if (FDTD_IN(qb + e, pext_y(p, 3))) p.psi_e_out[3][qb + e] = psi;
-                                set(ex, e, fadd(get(ex, e), fmul(get(cex, e), tc)));
-                            }
-                        }
-                    }
-                    if (ttile && tcode_e) {  // TFSF: E += 0.5 (c * H1d), after the CPML terms, before the sources
-                        tfsf_apply(p, 0, tcode_e & 0xfff, i, jj, kk, ex.x, ey.x, ez.x);
-                        tfsf_apply(p, 0, tcode_e >> 12, i, jj, kk + 1, ex.y, ey.y, ez.y);
-                    }
-                    const uint32_t ij_here = ((uint32_t)i << 16) | (uint32_t)jj;
-                    for (int s = 0; s < nls; s++) {  // soft sources, list order
-                        if (s_ls_ij[s] != ij_here) continue;
-                        const int kc = s_ls_kc[s];
-                        const int64_t sk = kc >> 2;
-                        if (sk != kk && sk != kk + 1) continue;
-                        const int e = (int)(sk - kk);
-                        const float v = p.src_amp[(int64_t)s_ls_s[s] * p.namp + p.t];
-                        const int comp = kc & 3;
-                        if (comp == 0) set(ex, e, fadd(get(ex, e), v));
-                        else if (comp == 1) set(ey, e, fadd(get(ey, e), v));
-                        else set(ez, e, fadd(get(ez, e), v));
-                    }
-                }
-                const int o = er * NCW + 2 + eko;
-                st2(Nx + o, ex);
-                st2(Ny + o, ey);
-                st2(Nz + o, ez);
-                oex = ex;
-                oey = ey;
-                oez = ez;
-            }
-            __syncthreads();  // (B) E_new of plane i visible
-
-            // ---- H phase: own rows ----
-            if (h_active) {
-                if (i >= x0) {
-                    const int o = er * NCW + 2 + eko;
-                    const float2 ez_jm = ld2(Nz + o - NCW), ex_jm = ld2(Nx + o - NCW);
-                    const float2 ey_km = make_float2(Ny[o - 1], oey.x), ex_km = make_float2(Nx[o - 1], oex.x);
-                    const int hi = er * HC + 4 + eko;
-                    const float2 hx0 = ld2(sH(st, 0) + hi), hy0 = ld2(sH(st, 1) + hi), hz0 = ld2(sH(st, 2) + hi);
-                    const float2 half = make_float2(0.5f, 0.5f);
-                    float2 hx = sub2(hx0, mul2(half, curl4x2(oez, ez_jm, oey, ey_km)));
-                    float2 hy = sub2(hy0, mul2(half, curl4x2(oex, ex_km, oez, prev_ez)));
-                    float2 hz = sub2(hz0, mul2(half, curl4x2(oey, prev_ey, oex, ex_jm)));
-                    if (!h_plain || hmask) {
-                        if (!(j_gt && k0_gt)) hx.x = hx0.x;
-                        if (!(j_gt && k1_gt)) hx.y = hx0.y;
-                        if (!(i_gt && k0_gt)) hy.x = hy0.x;
-                        if (!(i_gt && k1_gt)) hy.y = hy0.y;
-                        if (!(i_gt && j_gt)) {
-                            hz.x = hz0.x;
-                            hz.y = hz0.y;
-                        }
-                    }
-                    if (!h_plain) {
-                        if (sxh >= 0) {  // x slab: hy += (..dEz/dx..), hz -= (..dEy/dx..)
-                            const Coef c = tab_coef(tabs, 0, 2 * p.P[0], 1, sxh);
-                            const int64_t qb = ((int64_t)sxh * p.ny + jj) * p.nz + kk;
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                if (!(e ? in1 : in0) || (e ? hb1 : hb0)) continue;
-                                if (e ? k1_gt : k0_gt) {
-                                    float psi = xm ? sP(psl, 2)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 0)) ? p.psi_h[0][qb + e] : 0.f);
-                                    const float tc = corr(psi, c, fsub(get(oez, e), get(prev_ez, e)));
-                                    if (FDTD_IN(qb + e, pext_y(p, 0))) p.psi_h[0][qb + e] = psi;
-                                    set(hy, e, fadd(get(hy, e), fmul(0.5f, tc)));
-                                }
-                                if (j_gt) {
-                                    float psi = xm ? sP(psl, 3)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 1)) ? p.psi_h[1][qb + e] : 0.f);
-                                    const float tc = corr(psi, c, fsub(get(oey, e), get(prev_ey, e)));
-                                    if (FDTD_IN(qb + e, pext_y(p, 1))) p.psi_h[1][qb + e] = psi;
-                                    set(hz, e, fsub(get(hz, e), fmul(0.5f, tc)));
-                                }
-                            }
-                        }
-                        if (syh >= 0) {  // y slab: hz += (..dEx/dy..), hx -= (..dEz/dy..)
-                            const Coef cyh = tab_coef(tabs, (12 * p.P[0]), 2 * p.P[1], 1, syh);
-                            const int64_t qb = (i * 2 * p.P[1] + syh) * p.nz + kk;
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                if (!(e ? in1 : in0) || (e ? hb1 : hb0)) continue;
-                                if (i_gt) {
-                                    float psi = ym ? sP(psl, 2)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 2)) ? p.psi_h[2][qb + e] : 0.f);
-                                    const float tc = corr(psi, cyh, fsub(get(oex, e), get(ex_jm, e)));
-                                    if (FDTD_IN(qb + e, pext_y(p, 2))) p.psi_h[2][qb + e] = psi;
-                                    set(hz, e, fadd(get(hz, e), fmul(0.5f, tc)));
-                                }
-                                if (e ? k1_gt : k0_gt) {
-                                    float psi = ym ? sP(psl, 3)[er * EC + 4 + eko + e] : (FDTD_IN(qb + e, pext_y(p, 3)) ? p.psi_h[3][qb + e] : 0.f);
-                                    const float tc = corr(psi, cyh, fsub(get(oez, e), get(ez_jm, e)));
-                                    if (FDTD_IN(qb + e, pext_y(p, 3))) p.psi_h[3][qb + e] = psi;
-                                    set(hx, e, fsub(get(hx, e), fmul(0.5f, tc)));
-                                }
-                            }
-                        }
-                    }
-                    if (ttile && tcode_h) {  // TFSF: H += 0.5 (c * E1d), after the CPML terms
-                        tfsf_apply(p, 1, tcode_h & 0xfff, i, jj, kk, hx.x, hy.x, hz.x);
-                        tfsf_apply(p, 1, tcode_h >> 12, i, jj, kk + 1, hx.y, hy.y, hz.y);
-                    }
-                    const int64_t gi = i * p.sx + jj * p.sy + kk;
-                    if (in1) {
-                        if (FDTD_IN(gi + 1, fext_y(p))) st2(p.out[0] + gi, oex);
-                        if (FDTD_IN(gi + 1, fext_y(p))) st2(p.out[1] + gi, oey);
-                        if (FDTD_IN(gi + 1, fext_y(p))) st2(p.out[2] + gi, oez);
-                        if (FDTD_IN(gi + 1, fext_y(p))) st2(p.out[3] + gi, hx);
-                        if (FDTD_IN(gi + 1, fext_y(p))) st2(p.out[4] + gi, hy);
-                        if (FDTD_IN(gi + 1, fext_y(p))) st2(p.out[5] + gi, hz);
-                    } else if (in0) {
-                        if (FDTD_IN(gi, fext_y(p))) p.out[0][gi] = oex.x;
-                        if (FDTD_IN(gi, fext_y(p))) p.out[1][gi] = oey.x;
-                        if (FDTD_IN(gi, fext_y(p))) p.out[2][gi] = oez.x;
-                        if (FDTD_IN(gi, fext_y(p))) p.out[3][gi] = hx.x;
-                        if (FDTD_IN(gi, fext_y(p))) p.out[4][gi] = hy.x;
-                        if (FDTD_IN(gi, fext_y(p))) p.out[5][gi] = hz.x;
-                    }
-                }
-                prev_ey = oey;
-                prev_ez = oez;
-            }
+            if (++hs == L::NH) hs = 0;
         }
         if (aborted) break;
         first_item = false;
-        g0 += (uint32_t)nplanes;
-        gp0 += (uint32_t)(nplanes - 1);  // one psi phase per iteration
-        issued_hi = -1;
-        psi_hi = -1;
+        if (++hs == L::NH) hs = 0;  // an item uses one H plane more than stages
         if (BATCH) {
             __syncthreads();  // every thread has read s_item
             if (tid == 0) s_item = atomicAdd(&bd.queue[0], 1);
@@ -959,21 +1131,18 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
             atomicExch(p.status, FDTD_ERR_TIMEOUT);
             // Let the copies still in flight land before the CTA's shared
             // memory is released (each wait bounded).
-            for (int64_t q = q_abort; q <= issued_hi; q++) {
-                if (i_start_abort + q >= p.nx) continue;
-                const uint32_t G = g0 + (uint32_t)q;
-                mbar_wait_bounded(&bars[G % NS], (G / NS) & 1, nullptr, wlim);
-                mbar_wait_bounded(&bars[NS + G % NS], (G / NS) & 1, nullptr, wlim);
-            }
-            for (int64_t q = q_abort; q <= psi_hi; q++) {
-                const uint32_t Gp = gp0 + (uint32_t)q;
-                mbar_wait_bounded(&bars[2 * NS + (Gp & 1)], (Gp >> 1) & 1, nullptr, wlim);
+            for (int q = q_abort; q <= q_issued; q++) {
+                mbar_wait_bounded(&bars[es], par, nullptr, wlim);
+                if (++es == NS) {
+                    es = 0;
+                    par ^= 1;
+                }
             }
         }
         __syncthreads();
     }
 }
-#undef FDTD_SB
+
 
 // ---------------------------------------------------------------------------
 // z band kernels (single-grid plans).  The fused kernel treats z-slab tiles
@@ -990,25 +1159,16 @@ __device__ __forceinline__ Coef gcoef(const float *b, const float *a, const floa
     return Coef{b[s], a[s], k[s]};
 }
 
-// band cell counts of one grid: E (E z-slab nodes) and H (k in the H band)
-__host__ __device__ __forceinline__ int64_t zband_e_cells(const Params &p) {
-    const int P = p.P[2], f = (p.faces >> 4) & 1, b = (p.faces >> 5) & 1;
-    return p.zfix ? p.nx * p.ny * (int64_t)((f + b) * P) : 0;
-}
+// first k of the back H band
 __host__ __device__ __forceinline__ int64_t zband_h_start(const Params &p) {
     const int P = p.P[2], f = (p.faces >> 4) & 1, b = (p.faces >> 5) & 1;
     const int64_t fend = f ? P + 1 : 0;
     return b ? (p.nz - P - 1 > fend + 1 ? p.nz - P - 1 : fend + 1) : p.nz;
 }
-__host__ __device__ __forceinline__ int64_t zband_h_cells(const Params &p) {
-    const int P = p.P[2], f = (p.faces >> 4) & 1;
-    const int64_t fend = f ? P + 1 : 0;
-    return p.zfix ? p.nx * p.ny * (fend + p.nz - zband_h_start(p)) : 0;
-}
 
-// E band cell number t of grid p at step tstep.  All loads come first, then
-// the arithmetic, then the stores: a store could alias a later load as far as
-// the compiler knows, so loads placed after stores would not be overlapped.
+// All loads come first, then the arithmetic, then the stores: a store could
+// alias a later load as far as the compiler knows, so loads placed after
+// stores would not be overlapped.
 // E band cells per (i, j) row: the front slab's nodes, then the back slab's
 __device__ __forceinline__ int zband_e_row(const Params &p) {
     return (((p.faces >> 4) & 1) ? p.P[2] : 0) + (((p.faces >> 5) & 1) ? p.P[2] : 0);
@@ -1057,12 +1217,6 @@ __device__ __forceinline__ void zband_e_at(const Params &p, int64_t tstep, int64
     }
 }
 
-// E band cell number t of grid p (rows of zband_e_row cells, z fastest)
-__device__ __forceinline__ void zband_e_cell(const Params &p, int64_t tstep, int64_t t) {
-    const int nk = zband_e_row(p);
-    zband_e_at(p, tstep, t / ((int64_t)nk * p.ny), (t / nk) % p.ny, (int)(t % nk));
-}
-
 // H band cells per (i, j) row: k = 1 .. P+1 (front), then bstart .. nz-1 (back)
 __device__ __forceinline__ int zband_h_row(const Params &p) {
     const int64_t fend = ((p.faces >> 4) & 1) ? p.P[2] + 1 : 0;
@@ -1081,8 +1235,8 @@ __device__ __forceinline__ void zband_h_at(const Params &p, int64_t i, int64_t j
     const int64_t k = kb < nf ? 1 + kb : bstart + (kb - nf);
     const int64_t c = i * p.sx + j * p.sy + k;
     const int f0 = p.faces & 1, b0 = (p.faces >> 1) & 1, f1 = (p.faces >> 2) & 1, b1 = (p.faces >> 3) & 1;
-    const int sxh = slab_h(i, p.P[0], nx, f0, b0), syh = slab_h(j, p.P[1], ny, f1, b1);
-    const int szh = slab_h(k, P, nz, front, back);
+    const int sxh = slab_h((int)i, p.P[0], (int)nx, f0, b0), syh = slab_h((int)j, p.P[1], (int)ny, f1, b1);
+    const int szh = slab_h((int)k, P, (int)nz, front, back);
     const int P1 = p.P[1];
     const bool ux = j > 0 && k > 0, uy = i > 0 && k > 0, uz = i > 0 && j > 0;  // update masks
     // ---- loads
@@ -1151,30 +1305,6 @@ __device__ __forceinline__ void zband_h_at(const Params &p, int64_t i, int64_t j
     }
 }
 
-// H band cell number t of grid p (rows of zband_h_row cells, z fastest)
-__device__ __forceinline__ void zband_h_cell(const Params &p, int64_t t) {
-    const int nk = zband_h_row(p);
-    zband_h_at(p, t / ((int64_t)nk * p.ny), (t / nk) % p.ny, (int)(t % nk));
-}
-
-struct BandBatch {
-    int32_t nsims, cur;
-    int64_t t;
-    const Params *params;   // [2*nsims], as BatchDesc
-    const int64_t *off;     // [nsims + 1]
-};
-
-__device__ __forceinline__ int band_sim(const BandBatch &d, int64_t t) {
-    int lo = 0, hi = d.nsims - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (d.off[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-
 // Host stub of one fused-kernel instantiation (launched through a pointer).
 typedef void (*FusedKernel)(const TMaps, const Params, const BatchDesc);
 
@@ -1182,9 +1312,11 @@ typedef void (*FusedKernel)(const TMaps, const Params, const BatchDesc);
 #define FDTD_FUSED_TILES(X) X(4, 3) X(4, 4) X(4, 6) X(8, 3) X(8, 4) X(16, 3)
 
 // Instantiations compiled in separate translation units (the build compiles
-// them in parallel): single-grid kernels (EXT 0..2) and batched kernels
-// (EXT 0..1).  false when (ty, ns) is not compiled in.
-bool single_kernels(int ty, int ns, FusedKernel out[3]);
+// them in parallel): single-grid kernels without (EXT 0..3) and with (EXT 4..7)
+// the z-slab terms, batched kernels (EXT 4, 5).  false when (ty, ns) is not
+// compiled in.
+bool single_kernels(int ty, int ns, FusedKernel out[4]);
+bool single_kernels_z(int ty, int ns, FusedKernel out[4]);
 bool batch_kernels(int ty, int ns, FusedKernel out[2]);
 
 }  // namespace fused

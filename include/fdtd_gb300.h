@@ -230,12 +230,12 @@ typedef struct {
 
 /* Launch shape of the fused kernel (0 = default): tile height in y (4, 8
  * or 16 cells; the tile is 64 cells wide in z), x planes per work item,
- * resident CTAs per SM (persistent grid), pipeline stages (planes staged in
+ * resident CTAs per SM (0: one CTA per work item; else a persistent grid of
+ * that many CTAs per SM at most), pipeline stages (planes staged in
  * shared memory), L2 promotion of the tile loads (0 = 256 B, 1 = none,
- * 2 = 64 B, 3 = 128 B).  x_chunk 0 picks a chunk that gives every SM
- * about three work items, and for a grid without CPML (work items of equal
- * cost) the chunk of 128 .. 8 planes whose persistent launch is shortest
- * (ceil(items / CTAs) items of chunk + 3 plane steps). */
+ * 2 = 64 B, 3 = 128 B).  x_chunk 0: the split of the x planes whose launch is
+ * shortest when the resident CTAs work through tiles x chunks items of chunk
+ * + 4 plane steps (a batched plan: one chunk for all its grids). */
 typedef struct {
     int32_t tile_y;
     int32_t x_chunk;
@@ -266,8 +266,8 @@ int fdtd_yee_plan_set_current(fdtd_yee_plan *plan, int32_t cur);
  * every copy.  The aborted step leaves the output buffer partly written. */
 int fdtd_yee_plan_test_timeout(fdtd_yee_plan *plan, int64_t wait_ns, int32_t withhold_plane);
 /* info[0..5] = tile_y, stages, x_chunk, CTAs launched, threads/CTA, shared bytes/CTA;
- * with n >= 8 also info[6] = 1 when the z slab runs on the band kernels and
- * info[7] = kernel launches per step */
+ * with n >= 8 also info[6] = 1 when the z slab runs on the band kernels (else
+ * the fused kernel applies its terms) and info[7] = kernel launches per step */
 int fdtd_yee_plan_info(const fdtd_yee_plan *plan, int32_t *info, int32_t n);
 int fdtd_yee_plan_destroy(fdtd_yee_plan *plan);
 
