@@ -62,6 +62,36 @@ inline int check_launch() {
     return FDTD_OK;
 }
 
+// Launch with programmatic stream serialization: the kernel may start while
+// the one before it in the stream drains, and must execute grid_wait() before
+// it touches global memory (a kernel that calls grid_release() lets its own
+// successor start as soon as its last blocks are resident).  cluster: blocks
+// of a thread-block cluster (the grid a multiple of it), 1: none.
+template <typename... P, typename... A>
+inline void launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cluster,
+                           const A &...args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = cluster > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&c, fn, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+// all work of the kernels before this one in the stream is done and visible
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the stream may start (its grid_wait still waits for this grid's end)
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 #define FDTD_TRY(expr)                  \
     do {                                \
         int _st = (expr);               \

@@ -88,6 +88,7 @@ struct fdtd_yee_plan {
     int x_chunk;
     int64_t nitems;
     int nblocks;
+    int cluster;  // CTAs of a cluster (consecutive work items)
     int cur;
     TMaps maps[2];
     Params base;
@@ -119,18 +120,20 @@ static int encode_map(EncodeTiledFn enc, CUtensorMap *m, const float *ptr, const
 
 // Default launch shape: tile rows and pipeline stages.
 constexpr int kTileY = 8, kStages = 3;
+constexpr int kCluster = 8;
 
 // Whether a single grid's z slab is left to the band kernels.  In the fused
 // kernel a z-edge tile takes twice the time of a plain one a plane (its row
-// warps run the z code for a quarter of their lanes); the band kernels cost two
-// launches and a second pass over the row ends.  Measured, fused / bands, us a
-// step with CPML on all faces: 64^3 16.6 / 24.9, 80^3 33 / 38, 128^3 65 / 66,
-// 256x256x128 186 / 167, 256^3 315 / 260, 400x300x200 633 / 429, 512^3 1739 /
-// 1655, 1024x1024x512 6083 / 6596.  Grids of few (i, j) rows keep the bands'
-// three launches, which plan_info reports and the tests of it expect.
+// warps run the z code for a quarter of their lanes), and its neighbours then
+// share no halo reads with it; the band kernels cost two launches and a second
+// pass over the row ends.  Measured, fused / bands, us a step with CPML on all
+// faces: 64^3 15 / 23, 80^3 33 / 35, 128^3 65 / 62, 256x256x128 186 / 160,
+// 256^3 315 / 247, 400x300x200 633 / 412, 512^3 1739 / 1545, 1024x1024x512
+// 6078 / 5843.  Grids of few (i, j) rows keep the bands' three
+// launches, which plan_info reports and the tests of it expect.
 static bool use_bands(const Grid &g) {
-    const int64_t rows = g.nx * g.ny, cells = rows * g.nz;
-    return rows < 2048 || (cells >= ((int64_t)1 << 21) && cells < ((int64_t)1 << 28));
+    const int64_t rows = g.nx * g.ny;
+    return rows < 2048 || rows * g.nz >= ((int64_t)1 << 21);
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -306,6 +309,17 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
     if (pl->nitems >= ((int64_t)1 << 31)) { delete pl; return FDTD_ERR_UNSUPPORTED; }
     // one CTA an item, or a persistent grid where the caller limits the CTAs per SM
     pl->nblocks = (int)(max_ctas > 0 ? std::min<int64_t>(pl->nitems, (int64_t)nsm * occ) : pl->nitems);
+    // Launches of several rounds: clusters of 8 consecutive items.  A cluster's CTAs
+    // start together, so neighbouring tiles stay on nearby planes and share their halo
+    // reads through L2, which items that start one by one do not after the first
+    // rounds.  Measured without / with, us a step (27 rounds: 1024x1024x512, 6.7:
+    // 512^3): 5098 / 4837 plain and 6563 / 6015 with CPML; 1241 / 1223 and 1652 / 1587.
+    // With 3 rounds (256^3) the slots that wait for 8 to be free cost more: 164 / 172.
+    pl->cluster = 1;
+    if (max_ctas <= 0 && pl->nitems >= 4 * (int64_t)nsm * occ) {
+        pl->cluster = kCluster;
+        pl->nblocks = (pl->nblocks + kCluster - 1) / kCluster * kCluster;  // the excess CTAs find no item
+    }
     if (src && src->nsrc > 0) {
         if (!all_nonnull(src->ijk, src->comp, src->amp) || src->namp < 0) { delete pl; return FDTD_ERR_ARG; }
         p.nsrc = src->nsrc; p.src_ijk = src->ijk; p.src_comp = src->comp; p.src_amp = src->amp; p.namp = src->namp;
@@ -432,10 +446,13 @@ int fdtd_yee_plan_run(fdtd_yee_plan *pl, int64_t t0, int64_t nsteps, void *strea
         }
         p.t = t0 + n;
         BatchDesc bd{};
-        pl->fn<<<pl->nblocks, pl->k->threads, pl->smem, st>>>(pl->maps[in], p, bd);
+        launch_chained(pl->fn, dim3((unsigned)pl->nblocks), dim3((unsigned)pl->k->threads), (size_t)pl->smem, st,
+                       (unsigned)pl->cluster, pl->maps[in], p, bd);
         if (p.zfix) {
             for (int q = 0; q < 6; q++) p.in[q] = pl->f[in][q];
             const dim3 rows((unsigned)((p.ny + 3) / 4), (unsigned)p.nx);
+            // launched the plain way: started early, their waiting blocks hold back the
+            // kernel before them (256^3 253 -> 261 us a step)
             k_zband_e<<<rows, 128, 0, st>>>(p);
             k_zband_h<<<rows, 128, 0, st>>>(p);
         }
@@ -662,7 +679,8 @@ int fdtd_batch_plan_run(fdtd_batch_plan *bp, int64_t t0, int64_t nsteps, void *s
         bd.maps = bp->d_maps;
         bd.item_off = bp->d_off;
         bd.queue = bp->d_queue;
-        bp->fn<<<bp->nblocks, bp->k->threads, bp->smem, st>>>(dummy_maps, dummy, bd);
+        launch_chained(bp->fn, dim3((unsigned)bp->nblocks), dim3((unsigned)bp->k->threads), (size_t)bp->smem, st, 1,
+                       dummy_maps, dummy, bd);
         FDTD_TRY(check_launch());
         bp->cur = 1 - bp->cur;
     }

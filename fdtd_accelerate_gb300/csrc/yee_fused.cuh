@@ -528,6 +528,10 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
     __shared__ uint32_t s_ls_ij[MAX_LOCAL_SRC];
     __shared__ int s_ls_kc[MAX_LOCAL_SRC], s_ls_s[MAX_LOCAL_SRC];
 
+    // the next step's CTAs may set up while this launch drains (not the band kernels,
+    // which wait for its end)
+    if (BATCH || !pk.zfix) grid_release();
+
     const int tid = threadIdx.x, lane = tid & 31;
     const bool own_t = tid < L::OWN, e_t = tid < L::OWN + L::HALO, producer = tid == L::PRODUCER;
     // box row (row j0-1+er) and box column (first of the group) of this thread
@@ -583,7 +587,10 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                 prefetch_tmap(&mk.e[c]);
                 prefetch_tmap(&mk.ce[c]);
             }
+        grid_wait();
         stage_tables();
+    } else {
+        grid_wait();
     }
 
     // ring positions: stage slot and H slot of the current plane, parity of the stage

@@ -55,6 +55,7 @@ def _check(a, b, n=6):
     ((45, 47, 64), 8, 0x20, (16, 5, 0, 3)),
     ((45, 47, 70), 8, 0x1F, (4, 6, 2, 4)),     # persistent grid, no z back face
     ((64, 32, 72), 3, 0x0C, None),             # y faces alone
+    ((161, 72, 70), 4, 0x3F, (8, 2, 0, 3)),    # 1458 items: clusters of 8, the last one not full
 ])
 def test_z_terms_in_kernel(shape, npml, faces, tile):
     a, b = _pair(shape, npml, faces, tile)
