@@ -189,10 +189,8 @@ __device__ __forceinline__ bool near_h(const Args &A, int a, int x, int n) {
 //    would wait for them).  Cells with no CPML node skip the slab code.
 // ---------------------------------------------------------------------------
 template <typename I>
-__global__ void __launch_bounds__(kB) k_adj_e(Args A) {
-    const int k = blockIdx.x * kB + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
+__device__ __forceinline__ void adj_e_cell(const Args &A, int i, int j, int k) {
     const int nx = (int)A.g.nx, ny = (int)A.g.ny, nz = (int)A.g.nz;
-    if (k >= nz) return;
     const I X = (I)A.g.sx, Y = (I)A.g.sy, c = (I)i * X + (I)j * Y + k;
     // E update masks (2nd_order-Yee/Numpy/fdtd3d.py:10-13)
     const bool e0 = j < ny - 1 && k < nz - 1, e1 = i < nx - 1 && k < nz - 1, e2 = i < nx - 1 && j < ny - 1;
@@ -335,10 +333,8 @@ __global__ void __launch_bounds__(kB) k_adj_e(Args A) {
 //    first, as in k_adj_e; cells with no CPML node skip the slab code.
 // ---------------------------------------------------------------------------
 template <typename I>
-__global__ void __launch_bounds__(kB) k_adj_h(Args A) {
-    const int k = blockIdx.x * kB + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
+__device__ __forceinline__ void adj_h_cell(const Args &A, int i, int j, int k) {
     const int nx = (int)A.g.nx, ny = (int)A.g.ny, nz = (int)A.g.nz;
-    if (k >= nz) return;
     const I X = (I)A.g.sx, Y = (I)A.g.sy, c = (I)i * X + (I)j * Y + k;
     // H update masks (2nd_order-Yee/Numpy/fdtd3d.py:4-7)
     const bool h0 = j > 0 && k > 0, h1 = i > 0 && k > 0, h2 = i > 0 && j > 0;
@@ -418,6 +414,273 @@ __global__ void __launch_bounds__(kB) k_adj_h(Args A) {
     }
 }
 
+template <typename I>
+__global__ void __launch_bounds__(kB) k_adj_e(Args A) {
+    const int k = blockIdx.x * kB + threadIdx.x;
+    if (k < (int)A.g.nz) adj_e_cell<I>(A, blockIdx.z, blockIdx.y, k);
+}
+template <typename I>
+__global__ void __launch_bounds__(kB) k_adj_h(Args A) {
+    const int k = blockIdx.x * kB + threadIdx.x;
+    if (k < (int)A.g.nz) adj_h_cell<I>(A, blockIdx.z, blockIdx.y, k);
+}
+
+// ---------------------------------------------------------------------------
+// The two cell kernels with 4 z cells a thread, for fields whose rows start on
+// 16-byte boundaries and 32-bit offsets: the same expressions per cell, field
+// accesses 16 bytes wide.  One cell a thread was bound by its instructions
+// (85-90 % issue-active, ~500 a cell): at 256x256x128 with 12 CPML cells and a
+// gradient box of 1/8 of the cells E 123 and H 125 us a launch; this form 77 and
+// 68 (H: 48 bytes a cell at 5.9 TB/s).  Threads run over the (j, group) pairs of
+// an x plane.  The ragged end of a row goes cell by cell.
+// ---------------------------------------------------------------------------
+struct F4 {
+    float v[4];
+};
+__device__ __forceinline__ F4 ld4(const float *p) {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+    return F4{{t.x, t.y, t.z, t.w}};
+}
+__device__ __forceinline__ F4 ld4(const float *p, bool on) { return on ? ld4(p) : F4{}; }
+// 4 consecutive elements of a psi-shaped array: one access when the rows are aligned
+__device__ __forceinline__ F4 ldp(const float *p, bool on, bool vec) {
+    if (!on) return F4{};
+    if (vec) return ld4(p);
+    return F4{{__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3)}};
+}
+// elements lo .. hi-1
+__device__ __forceinline__ void st4(float *p, const F4 &r, int lo, int hi) {
+    if (lo == 0 && hi == 4) {
+        *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (e >= lo && e < hi) p[e] = r.v[e];
+    }
+}
+__device__ __forceinline__ float get(const F4 &a, int e, float past) { return e < 3 ? a.v[e < 3 ? e + 1 : 3] : past; }
+__device__ __forceinline__ float got(const F4 &a, int e, float before) { return e ? a.v[e ? e - 1 : 0] : before; }
+
+// A pair of slab terms of one component: d += w[s0] (s0 >= 0), d -= w[s1] (s1 >= 0)
+__device__ __forceinline__ void slab_pair(F4 &d, const F4 &w0, bool s0, const F4 &w1, bool s1) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        if (s0) d.v[e] = fadd(d.v[e], w0.v[e]);
+        if (s1) d.v[e] = fsub(d.v[e], w1.v[e]);
+    }
+}
+// the same along z: the node below / at cell e is in the slab where bit e / e+1 of m is set
+__device__ __forceinline__ void slab_pair_z(F4 &d, const float w[5], uint32_t m) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const float a = fadd(d.v[e], w[e]);
+        d.v[e] = (m >> e) & 1 ? a : d.v[e];
+        const float b = fsub(d.v[e], w[e + 1]);
+        d.v[e] = (m >> (e + 1)) & 1 ? b : d.v[e];
+    }
+}
+
+__global__ void __launch_bounds__(kB) k_adj_e4(Args A, uint32_t ng, int vec) {
+    const int nx = (int)A.g.nx, ny = (int)A.g.ny, nz = (int)A.g.nz, i = blockIdx.y;
+    const uint32_t t = blockIdx.x * kB + threadIdx.x;
+    const int j = (int)(t / ng), k = 4 * (int)(t - (uint32_t)j * ng);
+    if (j >= ny) return;
+    if (nz - k < 4) {
+        for (int q = k; q < nz; q++) adj_e_cell<int32_t>(A, i, j, q);
+        return;
+    }
+    const int X = (int)A.g.sx, Y = (int)A.g.sy, c = i * X + j * Y + k;
+    const int Px = A.P[0], Py = A.P[1], Pz = A.P[2];
+    const bool jl = j < ny - 1, il = i < nx - 1, jg = j > 0, ig = i > 0, last = k + 4 == nz, first = k == 0;
+    // adjoint H through the H update masks
+    const float *lhx = A.lf[3], *lhy = A.lf[4], *lhz = A.lf[5];
+    F4 hx0 = ld4(lhx + c, jg), hy0 = ld4(lhy + c, ig);
+    const F4 hz0 = ld4(lhz + c, ig && jg), hzj = ld4(lhz + c + Y, jl && ig), hzi = ld4(lhz + c + X, il && jg);
+    F4 hyi = ld4(lhy + c + X, il && jl), hxj = ld4(lhx + c + Y, il && jl);
+    const float hxk4 = jg && !last ? __ldg(lhx + c + 4) : 0.f, hyk4 = ig && !last ? __ldg(lhy + c + 4) : 0.f;
+    F4 l0 = ld4(A.lf[0] + c), l1 = ld4(A.lf[1] + c), l2 = ld4(A.lf[2] + c);
+    if (first) hx0.v[0] = hy0.v[0] = hyi.v[0] = hxj.v[0] = 0.f;  // (k > 0 masks; k+1 neighbours are unaffected)
+    F4 d0, d1, d2;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        d0.v[e] = fmul(-0.5f, curl4(hzj.v[e], hz0.v[e], get(hy0, e, hyk4), hy0.v[e]));
+        d1.v[e] = fmul(-0.5f, curl4(get(hx0, e, hxk4), hx0.v[e], hzi.v[e], hz0.v[e]));
+        d2.v[e] = fmul(-0.5f, curl4(hyi.v[e], hy0.v[e], hxj.v[e], hx0.v[e]));
+    }
+    // slab terms, per component in the order x or y, then z (or x, then y)
+    const bool nxs = near_e(A, 0, i, nx), nys = near_e(A, 1, j, ny);
+    const bool nzs = Pz > 0 && ((A.front[2] && k <= Pz) || (A.back[2] && k + 3 >= nz - Pz - 1));
+    int sxe = -1, sye = -1;
+    if (nxs) {
+        const int s0 = slab_h(i, Px, nx, A.front[0], A.back[0]), s1 = slab_h(i + 1, Px, nx, A.front[0], A.back[0]);
+        sxe = slab_e(i, Px, nx, A.front[0], A.back[0]);
+        const int o0 = psi_x<int>(ny, nz, s0, j, k), o1 = psi_x<int>(ny, nz, s1, j, k);
+        slab_pair(d1, ldp(A.wh[1] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.wh[1] + o1, s1 >= 0, vec), s1 >= 0);
+        slab_pair(d2, ldp(A.wh[0] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.wh[0] + o1, s1 >= 0, vec), s1 >= 0);
+    }
+    if (nys) {
+        const int s0 = slab_h(j, Py, ny, A.front[1], A.back[1]), s1 = slab_h(j + 1, Py, ny, A.front[1], A.back[1]);
+        sye = slab_e(j, Py, ny, A.front[1], A.back[1]);
+        const int o0 = psi_y<int>(nz, Py, i, s0, k), o1 = psi_y<int>(nz, Py, i, s1, k);
+        slab_pair(d0, ldp(A.wh[2] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.wh[2] + o1, s1 >= 0, vec), s1 >= 0);
+        slab_pair(d2, ldp(A.wh[3] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.wh[3] + o1, s1 >= 0, vec), s1 >= 0);
+    }
+    if (nzs) {
+        uint32_t m = 0;
+        float w5[5], w4[5];
+#pragma unroll
+        for (int e = 0; e < 5; e++) {
+            const int sz = slab_h(k + e, Pz, nz, A.front[2], A.back[2]), o = psi_z<int>(ny, Pz, i, j, sz);
+            m |= (uint32_t)(sz >= 0) << e;
+            w5[e] = sz >= 0 ? __ldg(A.wh[5] + o) : 0.f;
+            w4[e] = sz >= 0 ? __ldg(A.wh[4] + o) : 0.f;
+        }
+        slab_pair_z(d0, w5, m);
+        slab_pair_z(d1, w4, m);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        l0.v[e] = fadd(l0.v[e], d0.v[e]);
+        l1.v[e] = fadd(l1.v[e], d1.v[e]);
+        l2.v[e] = fadd(l2.v[e], d2.v[e]);
+    }
+    const int hi = last ? 3 : 4;  // cells with k < nz-1
+    if (jl) st4(A.lf[0] + c, l0, 0, hi);
+    if (il) st4(A.lf[1] + c, l1, 0, hi);
+    if (il && jl) st4(A.lf[2] + c, l2, 0, 4);
+
+    // gradient, on the cells glo .. ghi-1 of the box
+    int glo = 0, ghi = 4;
+    if (A.gbox) {
+        glo = (int)max((int64_t)0, A.gb0[2] - k);
+        ghi = (int)min((int64_t)4, A.gb1[2] - k);
+        if (i < A.gb0[0] || i >= A.gb1[0] || j < A.gb0[1] || j >= A.gb1[1] || glo >= ghi) return;
+    }
+    const float *hx = A.hp[0], *hy = A.hp[1], *hz = A.hp[2];
+    const F4 Hx0 = ld4(hx + c), Hy0 = ld4(hy + c), Hz0 = ld4(hz + c), Hzj = ld4(hz + c + Y, jl),
+             Hzi = ld4(hz + c + X, il), Hyi = ld4(hy + c + X, il && jl), Hxj = ld4(hx + c + Y, il && jl);
+    const float Hxk4 = last ? 0.f : __ldg(hx + c + 4), Hyk4 = last ? 0.f : __ldg(hy + c + 4);
+    F4 g0, g1, g2;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        g0.v[e] = curl4(Hzj.v[e], Hz0.v[e], get(Hy0, e, Hyk4), Hy0.v[e]);
+        g1.v[e] = curl4(get(Hx0, e, Hxk4), Hx0.v[e], Hzi.v[e], Hz0.v[e]);
+        g2.v[e] = curl4(Hyi.v[e], Hy0.v[e], Hxj.v[e], Hx0.v[e]);
+    }
+    // G += or -= km1 d + psi_e
+    auto term = [&](F4 &G, bool add, const F4 &ps, float km1, const F4 &a, const F4 &b) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float v = fadd(fmul(km1, fsub(a.v[e], b.v[e])), ps.v[e]);
+            G.v[e] = add ? fadd(G.v[e], v) : fsub(G.v[e], v);
+        }
+    };
+    if (sxe >= 0) {
+        const int o = psi_x<int>(ny, nz, sxe, j, k);
+        const float km1 = __ldg(A.ke[0] + sxe);
+        term(g1, false, ldp(A.pe[0] + o, true, vec), km1, Hzi, Hz0);
+        term(g2, true, ldp(A.pe[1] + o, true, vec), km1, Hyi, Hy0);
+    }
+    if (sye >= 0) {
+        const int o = psi_y<int>(nz, Py, i, sye, k);
+        const float km1 = __ldg(A.ke[1] + sye);
+        term(g0, true, ldp(A.pe[3] + o, true, vec), km1, Hzj, Hz0);
+        term(g2, false, ldp(A.pe[2] + o, true, vec), km1, Hxj, Hx0);
+    }
+    if (nzs) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int sz = slab_e(k + e, Pz, nz, A.front[2], A.back[2]);
+            if (sz < 0) continue;
+            const int o = psi_z<int>(ny, Pz, i, j, sz);
+            const float km1 = __ldg(A.ke[2] + sz);
+            g0.v[e] = fsub(g0.v[e], fadd(fmul(km1, fsub(get(Hy0, e, Hyk4), Hy0.v[e])), __ldg(A.pe[4] + o)));
+            g1.v[e] = fadd(g1.v[e], fadd(fmul(km1, fsub(get(Hx0, e, Hxk4), Hx0.v[e])), __ldg(A.pe[5] + o)));
+        }
+    }
+    auto accumulate = [&](float *gp, const F4 &l, const F4 &G, int top) {
+        F4 a = ld4(gp + c);
+#pragma unroll
+        for (int e = 0; e < 4; e++) a.v[e] = fadd(a.v[e], fmul(l.v[e], G.v[e]));
+        st4(gp + c, a, glo, min(ghi, top));
+    };
+    if (jl) accumulate(A.gce[0], l0, g0, hi);
+    if (il) accumulate(A.gce[1], l1, g1, hi);
+    if (il && jl) accumulate(A.gce[2], l2, g2, 4);
+}
+
+__global__ void __launch_bounds__(kB) k_adj_h4(Args A, uint32_t ng, int vec) {
+    const int nx = (int)A.g.nx, ny = (int)A.g.ny, nz = (int)A.g.nz, i = blockIdx.y;
+    const uint32_t t = blockIdx.x * kB + threadIdx.x;
+    const int j = (int)(t / ng), k = 4 * (int)(t - (uint32_t)j * ng);
+    if (j >= ny) return;
+    if (nz - k < 4) {
+        for (int q = k; q < nz; q++) adj_h_cell<int32_t>(A, i, j, q);
+        return;
+    }
+    const int X = (int)A.g.sx, Y = (int)A.g.sy, c = i * X + j * Y + k;
+    const int Px = A.P[0], Py = A.P[1], Pz = A.P[2];
+    const bool jl = j < ny - 1, il = i < nx - 1, jg = j > 0, ig = i > 0, last = k + 4 == nz, first = k == 0;
+    // nu = CE * lE of component q at offset o, zero outside q's update mask
+    auto nu4 = [&](int q, int o, bool on) {
+        F4 r{};
+        if (on) {
+            const F4 a = ld4(A.ce[q] + c + o), b = ld4(A.lf[q] + c + o);
+#pragma unroll
+            for (int e = 0; e < 4; e++) r.v[e] = fmul(a.v[e], b.v[e]);
+        }
+        return r;
+    };
+    auto nu1 = [&](int q, bool on) { return on ? fmul(__ldg(A.ce[q] + c - 1), __ldg(A.lf[q] + c - 1)) : 0.f; };
+    F4 n0 = nu4(0, 0, jl), n1 = nu4(1, 0, il), n1i = nu4(1, -X, ig && jg), n0j = nu4(0, -Y, ig && jg);
+    const F4 n2 = nu4(2, 0, il && jl), n2j = nu4(2, -Y, jg && il), n2i = nu4(2, -X, ig && jl);
+    const float n1k = nu1(1, il && !first), n0k = nu1(0, jl && !first);
+    F4 h0 = ld4(A.lf[3] + c), h1 = ld4(A.lf[4] + c), h2 = ld4(A.lf[5] + c);
+    if (last) n0.v[3] = n1.v[3] = n1i.v[3] = n0j.v[3] = 0.f;  // (k < nz-1 masks)
+    F4 d0, d1, d2;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        d0.v[e] = curl4(n2.v[e], n2j.v[e], n1.v[e], got(n1, e, n1k));
+        d1.v[e] = curl4(n0.v[e], got(n0, e, n0k), n2.v[e], n2i.v[e]);
+        d2.v[e] = curl4(n1.v[e], n1i.v[e], n0.v[e], n0j.v[e]);
+    }
+    if (near_h(A, 0, i, nx)) {
+        const int s0 = slab_e(i - 1, Px, nx, A.front[0], A.back[0]), s1 = slab_e(i, Px, nx, A.front[0], A.back[0]);
+        const int o0 = psi_x<int>(ny, nz, s0, j, k), o1 = psi_x<int>(ny, nz, s1, j, k);
+        slab_pair(d1, ldp(A.we[1] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.we[1] + o1, s1 >= 0, vec), s1 >= 0);
+        slab_pair(d2, ldp(A.we[0] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.we[0] + o1, s1 >= 0, vec), s1 >= 0);
+    }
+    if (near_h(A, 1, j, ny)) {
+        const int s0 = slab_e(j - 1, Py, ny, A.front[1], A.back[1]), s1 = slab_e(j, Py, ny, A.front[1], A.back[1]);
+        const int o0 = psi_y<int>(nz, Py, i, s0, k), o1 = psi_y<int>(nz, Py, i, s1, k);
+        slab_pair(d0, ldp(A.we[2] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.we[2] + o1, s1 >= 0, vec), s1 >= 0);
+        slab_pair(d2, ldp(A.we[3] + o0, s0 >= 0, vec), s0 >= 0, ldp(A.we[3] + o1, s1 >= 0, vec), s1 >= 0);
+    }
+    if (Pz > 0 && ((A.front[2] && k <= Pz + 1) || (A.back[2] && k + 3 >= nz - Pz - 1))) {
+        uint32_t m = 0;
+        float w5[5], w4[5];
+#pragma unroll
+        for (int e = 0; e < 5; e++) {
+            const int sz = slab_e(k + e - 1, Pz, nz, A.front[2], A.back[2]), o = psi_z<int>(ny, Pz, i, j, sz);
+            m |= (uint32_t)(sz >= 0) << e;
+            w5[e] = sz >= 0 ? __ldg(A.we[5] + o) : 0.f;
+            w4[e] = sz >= 0 ? __ldg(A.we[4] + o) : 0.f;
+        }
+        slab_pair_z(d0, w5, m);
+        slab_pair_z(d1, w4, m);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        h0.v[e] = fadd(h0.v[e], d0.v[e]);
+        h1.v[e] = fadd(h1.v[e], d1.v[e]);
+        h2.v[e] = fadd(h2.v[e], d2.v[e]);
+    }
+    const int lo = first ? 1 : 0;  // cells with k > 0
+    if (jg) st4(A.lf[3] + c, h0, lo, 4);
+    if (ig) st4(A.lf[4] + c, h1, lo, 4);
+    if (ig && jg) st4(A.lf[5] + c, h2, 0, 4);
+}
+
 // ---------------------------------------------------------------------------
 // point lists: gather (monitors) and add (adjoint injection), list order
 // ---------------------------------------------------------------------------
@@ -442,19 +705,29 @@ __global__ void k_gather_points(Grid g, fdtd_points pts, fdtd_fields6 f, float *
 // points: one thread per point, one block.  A point whose cell and component
 // an earlier point also names is skipped by its thread; the thread of the
 // first such point adds the values of all of them in list order.
+// (The list is staged in shared memory: read from global memory in the two
+// loops it cost a memory latency a point, 8 us for 16 points.)
 constexpr int kAddThreads = 1024;
-__global__ void k_add_points(Grid g, fdtd_points pts, fdtd_fields6 f, const float *vals) {
+__global__ void __launch_bounds__(kAddThreads)
+k_add_points(Grid g, fdtd_points pts, fdtd_fields6 f, const float *vals) {
+    __shared__ int64_t s_c[kAddThreads];  // 8 * cell offset + component, -1: out of range
+    __shared__ float s_v[kAddThreads];
     const int p = threadIdx.x;
-    if (blockIdx.x != 0 || p >= pts.n) return;
-    const int64_t c = point_offset(g, pts, p);
-    if (c < 0) return;
-    const int q = pts.comp[p];
+    int64_t key = -1;
+    if (p < pts.n) {
+        const int64_t c = point_offset(g, pts, p);
+        if (c >= 0) key = 8 * c + pts.comp[p];
+        s_c[p] = key;
+        s_v[p] = vals[p];
+    }
+    __syncthreads();
+    if (key < 0) return;
     for (int r = 0; r < p; r++)
-        if (pts.comp[r] == q && point_offset(g, pts, r) == c) return;
-    float *fp = f.f[q] + c;
+        if (s_c[r] == key) return;
+    float *fp = f.f[key & 7] + (key >> 3);
     float v = *fp;
     for (int r = p; r < pts.n; r++)
-        if (pts.comp[r] == q && point_offset(g, pts, r) == c) v = fadd(v, vals[r]);
+        if (s_c[r] == key) v = fadd(v, s_v[r]);
     *fp = v;
 }
 // longer lists: one thread walks the list
@@ -576,13 +849,25 @@ static int adjoint_step(const fdtd_grid *gp, const fdtd_cpml *cp, const fdtd_adj
         if (i32) k_adj_psi3<false, int32_t><<<R.nb[2], kB, 0, st>>>(A, R);
         else k_adj_psi3<false, int64_t><<<R.nb[2], kB, 0, st>>>(A, R);
     }
-    if (i32) k_adj_e<int32_t><<<cells(g), kB, 0, st>>>(A);
+    // 4 cells a thread where the rows of every field array start on 16-byte
+    // boundaries; psi rows then load as vectors when nz is a multiple of 4
+    auto a16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    bool v4 = i32 && g.sx % 4 == 0 && g.sy % 4 == 0, vec = g.nz % 4 == 0;
+    for (int q = 0; q < 6; q++) v4 = v4 && a16(A.lf[q]);
+    for (int q = 0; q < 3; q++) v4 = v4 && a16(A.gce[q]) && a16(A.hp[q]) && a16(A.ce[q]);
+    for (int q = 0; q < 4; q++)
+        if (A.P[q / 2] > 0) vec = vec && a16(A.we[q]) && a16(A.wh[q]) && a16(A.pe[q]);
+    const uint32_t ng = (uint32_t)((g.nz + 3) / 4);
+    const dim3 grid4((unsigned)((g.ny * (int64_t)ng + kB - 1) / kB), (unsigned)g.nx);
+    if (v4) k_adj_e4<<<grid4, kB, 0, st>>>(A, ng, vec);
+    else if (i32) k_adj_e<int32_t><<<cells(g), kB, 0, st>>>(A);
     else k_adj_e<int64_t><<<cells(g), kB, 0, st>>>(A);
     if (R.nb[2] > 0) {
         if (i32) k_adj_psi3<true, int32_t><<<R.nb[2], kB, 0, st>>>(A, R);
         else k_adj_psi3<true, int64_t><<<R.nb[2], kB, 0, st>>>(A, R);
     }
-    if (i32) k_adj_h<int32_t><<<cells(g), kB, 0, st>>>(A);
+    if (v4) k_adj_h4<<<grid4, kB, 0, st>>>(A, ng, vec);
+    else if (i32) k_adj_h<int32_t><<<cells(g), kB, 0, st>>>(A);
     else k_adj_h<int64_t><<<cells(g), kB, 0, st>>>(A);
     return check_launch();
 }
