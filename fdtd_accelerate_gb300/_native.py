@@ -157,6 +157,13 @@ _SIGS = {
 
 _lib = None
 
+try:  # the raw handle of a device's current stream, without a Stream object around it
+    from torch._C import _cuda_getCurrentRawStream as raw_stream
+except ImportError:
+    def raw_stream(device):
+        import torch
+        return torch.cuda.current_stream(device).cuda_stream
+
 
 def lib():
     """Load the library (once).  Raises if it has not been built."""
@@ -202,5 +209,6 @@ def check(st, fn):
 
 
 def call(name, *args):
-    st = getattr(lib(), name)(*args)
-    check(st, name)
+    st = getattr(_lib or lib(), name)(*args)
+    if st:
+        check(st, name)

@@ -27,6 +27,18 @@ __all__ = ["update_e", "update_h", "update_pbc_e", "update_pbc_h", "grid_of", "s
 
 def check_field_tensors(names, tensors):
     """Validate a group of field tensors: float32, CUDA, 3-D, one layout."""
+    # the usual case in one pass: every tensor like the first (a call on a small
+    # grid takes longer on the host than on the GPU, and most of that in here)
+    first = tensors[0] if len(tensors) else None
+    if isinstance(first, torch.Tensor) and first.dtype is torch.float32 and first.is_cuda and first.dim() == 3:
+        shape, stride, dev = first.shape, first.stride(), first.get_device()
+        if stride[2] == 1 and stride[1] >= shape[2] and stride[0] >= shape[1] * stride[1]:
+            for t in tensors:
+                if not (isinstance(t, torch.Tensor) and t.dtype is torch.float32 and t.is_cuda
+                        and t.shape == shape and t.stride() == stride and t.get_device() == dev):
+                    break
+            else:
+                return first
     ref = None
     for name, t in zip(names, tensors):
         if not isinstance(t, torch.Tensor):
@@ -53,8 +65,8 @@ def check_field_tensors(names, tensors):
 
 
 def grid_of(t):
-    nx, ny, nz = t.shape
-    return N.Grid(nx, ny, nz, t.stride(0), t.stride(1))
+    sx, sy, _ = t.stride()
+    return N.Grid(*t.shape, sx, sy)
 
 
 def stream_of(t):
@@ -62,7 +74,17 @@ def stream_of(t):
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
+
+
+def _call(ref, name, *args):
+    """N.call on ref's device, its current stream as the last argument."""
+    dev = ref.get_device()
+    if torch.cuda.current_device() == dev:
+        N.call(name, *args, N.raw_stream(dev))
+    else:
+        with torch.cuda.device(dev):
+            N.call(name, *args, N.raw_stream(dev))
 
 
 def update_e(ex, ey, ez, hx, hy, hz, cex, cey, cez):
@@ -70,8 +92,7 @@ def update_e(ex, ey, ez, hx, hy, hz, cex, cey, cez):
     ts = (ex, ey, ez, hx, hy, hz, cex, cey, cez)
     ref = check_field_tensors(names, ts)
     g = grid_of(ref)
-    with torch.cuda.device(ref.device):
-        N.call("fdtd_update_e_f32", C.byref(g), *map(_ptr, ts), stream_of(ref))
+    _call(ref, "fdtd_update_e_f32", C.byref(g), *map(_ptr, ts))
 
 
 def update_h(ex, ey, ez, hx, hy, hz, chx=None, chy=None, chz=None):
@@ -85,9 +106,7 @@ def update_h(ex, ey, ez, hx, hy, hz, chx=None, chy=None, chz=None):
         ts += list(chs)
     ref = check_field_tensors(names, ts)
     g = grid_of(ref)
-    with torch.cuda.device(ref.device):
-        N.call("fdtd_update_h_f32", C.byref(g), *map(_ptr, (ex, ey, ez, hx, hy, hz, chx, chy, chz)),
-               stream_of(ref))
+    _call(ref, "fdtd_update_h_f32", C.byref(g), *map(_ptr, (ex, ey, ez, hx, hy, hz, chx, chy, chz)))
 
 
 def _axes(directions):
@@ -103,13 +122,11 @@ def update_pbc_e(directions, ex, ey, ez):
     axes = _axes(directions)
     ref = check_field_tensors(("ex", "ey", "ez"), (ex, ey, ez))
     g = grid_of(ref)
-    with torch.cuda.device(ref.device):
-        N.call("fdtd_update_pbc_e_f32", C.byref(g), axes, _ptr(ex), _ptr(ey), _ptr(ez), stream_of(ref))
+    _call(ref, "fdtd_update_pbc_e_f32", C.byref(g), axes, _ptr(ex), _ptr(ey), _ptr(ez))
 
 
 def update_pbc_h(directions, hx, hy, hz):
     axes = _axes(directions)
     ref = check_field_tensors(("hx", "hy", "hz"), (hx, hy, hz))
     g = grid_of(ref)
-    with torch.cuda.device(ref.device):
-        N.call("fdtd_update_pbc_h_f32", C.byref(g), axes, _ptr(hx), _ptr(hy), _ptr(hz), stream_of(ref))
+    _call(ref, "fdtd_update_pbc_h_f32", C.byref(g), axes, _ptr(hx), _ptr(hy), _ptr(hz))

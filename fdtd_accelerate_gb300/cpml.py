@@ -124,16 +124,18 @@ class CpmlLayer:
             c.npml[a] = self.npml[a]
         c.faces = self.faces
         for a in range(3):
-            t = self.tables[a]
-            for key in ("b_e", "a_e", "km1_e", "b_h", "a_h", "km1_h"):
-                getattr(c, key)[a] = t[key].data_ptr() if self.npml[a] else None
+            if self.npml[a]:
+                t = self.tables[a]
+                for key in ("b_e", "a_e", "km1_e", "b_h", "a_h", "km1_h"):
+                    getattr(c, key)[a] = t[key].data_ptr()
         return c
 
     def psi_struct(self, buf=0):
         p = N.Psi()
-        for q in range(6):
-            p.e[q] = self.psi_e[buf][q].data_ptr() if self.psi_e[buf][q] is not None else None
-            p.h[q] = self.psi_h[q].data_ptr() if self.psi_h[q] is not None else None
+        pe, ph = p.e, p.h
+        for q, (e, h) in enumerate(zip(self.psi_e[buf], self.psi_h)):
+            if e is not None:
+                pe[q], ph[q] = e.data_ptr(), h.data_ptr()
         return p
 
     def reset(self):
@@ -148,19 +150,17 @@ class CpmlLayer:
     # -- reference-shaped per-call updates (kuFDTD CpmlNonKappa.updateE/H,
     #    kuFDTD/v0.2.0/dim3/cpu/cpml.py:129-203; KEMP Pml.update_e/h) -------
     def update_e(self, ex, ey, ez, hx, hy, hz, cex, cey, cez):
-        from .api import check_field_tensors, grid_of, stream_of
+        from .api import _call, check_field_tensors, grid_of
         ts = (ex, ey, ez, hx, hy, hz, cex, cey, cez)
         ref = check_field_tensors(("ex", "ey", "ez", "hx", "hy", "hz", "cex", "cey", "cez"), ts)
         self._check_shape(ref)
         g = grid_of(ref)
         c = self.struct()
         psi = self.psi_struct(0)
-        with torch.cuda.device(ref.device):
-            N.call("fdtd_cpml_e_f32", C.byref(g), C.byref(c), *[C.c_void_p(t.data_ptr()) for t in ts],
-                   C.byref(psi), stream_of(ref))
+        _call(ref, "fdtd_cpml_e_f32", C.byref(g), C.byref(c), *[t.data_ptr() for t in ts], C.byref(psi))
 
     def update_h(self, ex, ey, ez, hx, hy, hz, chx=None, chy=None, chz=None):
-        from .api import check_field_tensors, grid_of, stream_of
+        from .api import _call, check_field_tensors, grid_of
         ts = [ex, ey, ez, hx, hy, hz]
         names = ["ex", "ey", "ez", "hx", "hy", "hz"]
         if chx is not None:
@@ -171,10 +171,8 @@ class CpmlLayer:
         g = grid_of(ref)
         c = self.struct()
         psi = self.psi_struct(0)
-        ptrs = [C.c_void_p(t.data_ptr()) for t in (ex, ey, ez, hx, hy, hz)]
-        ptrs += [C.c_void_p(t.data_ptr()) if t is not None else None for t in (chx, chy, chz)]
-        with torch.cuda.device(ref.device):
-            N.call("fdtd_cpml_h_f32", C.byref(g), C.byref(c), *ptrs, C.byref(psi), stream_of(ref))
+        ptrs = [t.data_ptr() if t is not None else None for t in (ex, ey, ez, hx, hy, hz, chx, chy, chz)]
+        _call(ref, "fdtd_cpml_h_f32", C.byref(g), C.byref(c), *ptrs, C.byref(psi))
 
     def _check_shape(self, t):
         if tuple(t.shape) != self.shape:

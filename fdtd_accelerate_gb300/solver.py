@@ -78,8 +78,7 @@ class YeeSolver:
 
     # ------------------------------------------------------------------ views
     def _views(self, b):
-        nz = self.shape[2]
-        return [self._state[b, q, :, :, :nz] for q in range(6)]
+        return list(self._state[b].narrow(3, 0, self.shape[2]).unbind(0))
 
     @property
     def fields(self):
@@ -165,10 +164,13 @@ class YeeSolver:
                 self.close()
         plan = self.plan()
         L = N.lib()
-        L.fdtd_yee_plan_set_current(plan, self.cur)
-        with torch.cuda.device(self.device):
-            stream = C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-            N.call("fdtd_yee_plan_run", plan, int(self.tstep), int(n), stream)
+        L.fdtd_yee_plan_set_current(plan, self._cur)
+        dev = self._state.get_device()
+        if torch.cuda.current_device() == dev:
+            N.call("fdtd_yee_plan_run", plan, int(self.tstep), int(n), N.raw_stream(dev))
+        else:
+            with torch.cuda.device(dev):
+                N.call("fdtd_yee_plan_run", plan, int(self.tstep), int(n), N.raw_stream(dev))
         self.cur = L.fdtd_yee_plan_current(plan)
         self.tstep += n
 
