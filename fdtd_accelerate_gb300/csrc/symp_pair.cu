@@ -973,8 +973,10 @@ static int map3(EncodeFn enc, CUtensorMap *m, const float *ptr, const Grid &g, i
 }
 
 // x planes per work item when the caller leaves the choice to the plan: of
-// the chunks 48 .. 256 (steps of 8), the one whose greedy schedule of a
-// pass's items over the resident CTAs ends first.  The queue hands items out
+// the chunks 48 .. 256 (steps of 8; from 8 on where chunks of 48 make fewer
+// items than two rounds of CTAs: with 48 planes at least, 150x171x163 filled
+// half of them), the one whose greedy schedule of a pass's items over the
+// resident CTAs ends first.  The queue hands items out
 // x chunk by x chunk; an item costs its planes (x-slab planes, which carry
 // the CPML terms, twice) plus the 6 iterations that fill the pipeline.  The
 // largest chunk wins ties (fewer fills).
@@ -983,7 +985,8 @@ static int choose_x_chunk(int nx, int64_t tiles, int slots, int pf, int pb) {
     int64_t best_t = -1;
     std::vector<int64_t> heap;
     int last = -1;
-    for (int xc = 256; xc >= 48; xc -= 8) {
+    const int least = tiles * ((nx + 47) / 48) < 2 * (int64_t)slots ? 8 : 48;
+    for (int xc = 256; xc >= least; xc -= 8) {
         const int c = std::min(xc, nx);
         if (c == last) continue;  // chunks past nx are all the whole grid
         last = c;

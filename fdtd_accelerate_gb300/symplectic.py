@@ -26,6 +26,7 @@ import torch
 from . import _native as N
 from .api import check_field_tensors, grid_of, stream_of
 from .cpml import parse_faces, sigma_max_from_reflection
+from .solver import padded_nz
 from .sources import PointSources
 
 __all__ = ["C1", "C2", "C3", "D1", "D2", "CL", "DL", "COURANT", "update_h", "update_e",
@@ -200,7 +201,7 @@ class SymplecticSolver:
         self.S = S
         # state buffers: buf[cur] holds the fields; the stage-pair path writes
         # buf[1 - cur] from buf[cur] (the second buffer is allocated on first use)
-        self._buf = [torch.zeros((6,) + self.shape, dtype=torch.float32, device=dev), None]
+        self._buf = [self._rows(6), None]
         self._cur = 0
         self.fused = fused
         self.x_chunk = int(x_chunk)
@@ -208,10 +209,9 @@ class SymplecticSolver:
         self._pair_src = None
         if ce is None:
             ce = [np.full(self.shape, S / 24.0)] * 3
-        self.ce = [torch.as_tensor(c, dtype=torch.float32, device=dev).contiguous() for c in ce]
+        self.ce = self._as_rows(ce)
         self.ch = float(S / 24.0) if ch is None else (
-            float(ch) if isinstance(ch, (int, float)) else
-            [torch.as_tensor(c, dtype=torch.float32, device=dev).contiguous() for c in ch])
+            float(ch) if isinstance(ch, (int, float)) else self._as_rows(ch))
         self.cpml = SymplecticCpml(self.shape, npml, faces, S, device=dev, **(cpml_params or {}))
         self.src_spec = list(sources)
         self.max_steps = max_steps
@@ -219,6 +219,22 @@ class SymplecticSolver:
         self._src = None
         self._stage_args = None
         self._build_sources(max(max_steps, 1))
+
+    def _rows(self, n):
+        """n zeroed arrays of the grid's shape whose rows start on 16-byte
+        boundaries (the pitch is nz rounded up to 4 floats), as the TMA copies
+        of the stage-pair path need them."""
+        nx, ny, nz = self.shape
+        return torch.zeros((n, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)[..., :nz]
+
+    def _as_rows(self, arrays):
+        """Three coefficient arrays in the fields' layout."""
+        if self.shape[2] % 4 == 0:
+            return [torch.as_tensor(c, dtype=torch.float32, device=self.device).contiguous() for c in arrays]
+        out = list(self._rows(3).unbind(0))
+        for dst, c in zip(out, arrays):
+            dst.copy_(torch.as_tensor(c, dtype=torch.float32, device=self.device))
+        return out
 
     def _build_sources(self, nsteps):
         tabs = []
@@ -241,19 +257,33 @@ class SymplecticSolver:
         return dict(zip(("ex", "ey", "ez", "hx", "hy", "hz"), self.f))
 
     def pair_path(self):
-        """True when step() runs the fused stage pairs: uniform ch, rows of a
-        multiple of 4 floats (16-byte TMA rows), fewer than 2^31 cells, every
-        extent at least 4."""
+        """True when step() runs the fused stage pairs: uniform ch, fewer than
+        2^31 elements (with the rows' padding), every extent at least 4, and
+        on rows that are no multiple of 4 floats at least 65 % of the grid
+        clear of the y/z CPML shell (below that the stage kernels are faster:
+        80x80x81 with 8 cells, 45 % clear, 568 us for 4 steps against 778;
+        150x171x163, 69 %, 607 us a step against 563; 300x300x301 with 10,
+        82 %, 2908 against 2180; 200x200x201 without CPML 805 against 496)."""
         nx, ny, nz = self.shape
-        return (self.fused and isinstance(self.ch, float) and nz % 4 == 0 and min(self.shape) >= 4
-                and nx * ny * nz < 2 ** 31)
+        return (self.fused and isinstance(self.ch, float) and min(self.shape) >= 4
+                and nx * ny * padded_nz(nz) < 2 ** 31 and (nz % 4 == 0 or self._inside() >= 0.65))
+
+    def _inside(self):
+        """Share of the grid that the pair kernel advances: rows P+2 and more
+        from a y face, columns from a z face likewise, in steps of 16."""
+        _, ny, nz = self.shape
+        (_, py, pz), f = self.cpml.npml, self.cpml.faces
+        j0, j1 = (py + 2 if py and f & 4 else 0), (ny - py - 2 if py and f & 8 else ny)
+        k0 = (pz + 17) // 16 * 16 if pz and f & 16 else 0
+        k1 = (nz - pz - 2) // 16 * 16 if pz and f & 32 else nz
+        return max(0, j1 - j0) * max(0, k1 - k0) / (ny * nz)
 
     def _pair_plan(self):
         if self._pair is not None and self._pair_src is self._src:
             return self._pair
         self.close()
         if self._buf[1] is None:
-            self._buf[1] = torch.zeros_like(self._buf[0])
+            self._buf[1] = self._rows(6)
         hb = self.cpml.second_h_buffer()
         st = N.SympState()
         for b in range(2):
@@ -341,7 +371,7 @@ class SymplecticSolver:
         stage.  Fields of 2^31 or more elements (the stage kernel's offsets are
         32-bit) take the per-call path of step_unfused."""
         f = self.f
-        if f[0].numel() >= 2 ** 31:
+        if f[0].shape[0] * f[0].stride(0) >= 2 ** 31:
             return self.step_unfused(n)
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)

@@ -288,8 +288,8 @@ int fdtd_yee_step_f32(const fdtd_grid *g, const fdtd_yee_state *st, const fdtd_c
 /* State in two buffers (ping-pong): f[b] = ex,ey,ez,hx,hy,hz of buffer b,
  * psi_h[b] the H psi slabs of buffer b (layouts of fdtd_psi); the E psi
  * slabs psi_e are updated in place.  Requirements: C-order arrays with
- * 16-byte aligned bases and rows (nz a multiple of 4 floats), fewer than
- * 2^31 elements each, nx, ny, nz >= 4, a uniform ch. */
+ * 16-byte aligned bases and rows (strides of a multiple of 4 floats; nz may
+ * be any), fewer than 2^31 elements each, nx, ny, nz >= 4, a uniform ch. */
 typedef struct {
     float *f[2][6];
     float *psi_e[6];
