@@ -178,12 +178,22 @@ static int single_chunk(int64_t nx, int64_t tiles, int64_t slots) {
     return (int)best;
 }
 
-// batch: a grid of a batched plan, which pools every grid's items over one
-// launch (x_chunk comes from the batched plan) and whose kernel applies the
-// z-slab terms itself
+// The chunk for which the number of sources an item may hold is counted when the
+// caller gives none: 128 planes, halved down to 8 until there are 3 items an SM.
+// It fixes which source layouts are refused, whatever chunk the step then takes;
+// a longer chunk's items may hold more than their list does, and scan all sources.
+static int capacity_chunk(int64_t nx, int64_t tiles, int nsm) {
+    int xc = 128;
+    while (xc > 8 && tiles * ((nx + xc - 1) / xc) < 3 * (int64_t)nsm) xc /= 2;
+    return xc;
+}
+
+// batch_chunk > 0: a grid of a batched plan, which pools every grid's items over
+// one launch (with that chunk unless the caller gives one) and whose kernel
+// applies the z-slab terms itself
 static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_yee_state *s, const fdtd_cpml *c,
                            const fdtd_sources *src, const fdtd_tile *tile, int32_t *status_dev, int32_t cur,
-                           void *stream, bool batch) {
+                           void *stream, int batch_chunk) {
     if (!out || !s || !status_dev) return FDTD_ERR_ARG;
     *out = nullptr;
     Grid g;
@@ -282,7 +292,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         p.th1d = t.h1d;
     }
     // the z slab (when a z face has CPML): inside the fused kernel or by the band kernels
-    p.zfix = (!batch && p.P[2] > 0 && ((p.faces >> 4) & 3) && use_bands(g)) ? 1 : 0;
+    p.zfix = (!batch_chunk && p.P[2] > 0 && ((p.faces >> 4) & 3) && use_bands(g)) ? 1 : 0;
     // tile rows with y slab cells (rows j0-1 .. j0+ty-1), counted from either end
     if (p.P[1] > 0)
         for (int t = 0; t < p.nty; t++) {
@@ -302,7 +312,8 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
     }
     const int max_ctas = tile ? (int)tile->ctas_per_sm : 0;
     if (max_ctas > 0) occ = std::min(occ, max_ctas);
-    if (!xch) xch = single_chunk(g.nx, (int64_t)p.ntz * p.nty, (int64_t)nsm * occ);
+    const int cap_chunk = xch ? xch : capacity_chunk(g.nx, (int64_t)p.ntz * p.nty, nsm);
+    if (!xch) xch = batch_chunk ? batch_chunk : single_chunk(g.nx, (int64_t)p.ntz * p.nty, (int64_t)nsm * occ);
     pl->x_chunk = p.x_chunk = (int)std::min<int64_t>(xch, g.nx);
     p.nxc = (int)((g.nx + pl->x_chunk - 1) / pl->x_chunk);
     pl->nitems = (int64_t)p.ntz * p.nty * p.nxc;
@@ -323,7 +334,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
     if (src && src->nsrc > 0) {
         if (!all_nonnull(src->ijk, src->comp, src->amp) || src->namp < 0) { delete pl; return FDTD_ERR_ARG; }
         p.nsrc = src->nsrc; p.src_ijk = src->ijk; p.src_comp = src->comp; p.src_amp = src->amp; p.namp = src->namp;
-        // capacity: sources per work item's extended region (checked on the host)
+        // capacity: sources per work item's extended region, in chunks of cap_chunk planes
         // read on the caller's stream (after any pending write of the list), then wait for it
         int32_t *hijk = new int32_t[3 * (size_t)src->nsrc];
         cudaError_t ce = cudaMemcpyAsync(hijk, src->ijk, sizeof(int32_t) * 3 * src->nsrc, cudaMemcpyDeviceToHost,
@@ -352,7 +363,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         // (x in [i_start, x1), y in [j0-1, j0+TY), z in [k0-1, k0+TZ)); a source
         // lies in at most two chunks/tiles per axis
         std::unordered_map<int64_t, int> per_item;
-        const int64_t xc = pl->x_chunk;
+        const int64_t xc = std::min<int64_t>(cap_chunk, g.nx);
         const int64_t ntz = (g.nz + TZ - 1) / TZ, nty = (g.ny + ty - 1) / ty;
         for (int a = 0; a < src->nsrc; a++) {
             const int64_t si = hijk[3 * a], sj = hijk[3 * a + 1], sk = hijk[3 * a + 2];
@@ -418,7 +429,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
 int fdtd_yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_yee_state *s, const fdtd_cpml *c,
                          const fdtd_sources *src, const fdtd_tile *tile, int32_t *status_dev, int32_t cur,
                          void *stream) {
-    return yee_plan_create(out, gp, s, c, src, tile, status_dev, cur, stream, false);
+    return yee_plan_create(out, gp, s, c, src, tile, status_dev, cur, stream, 0);
 }
 
 int fdtd_yee_plan_run(fdtd_yee_plan *pl, int64_t t0, int64_t nsteps, void *stream) {
@@ -568,8 +579,8 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     int tab_bytes = 0;
     bool any_drude = false;
     const int ty = tile && tile->tile_y ? tile->tile_y : kTileY;
-    fdtd_tile bt = tile ? *tile : fdtd_tile{0, 0, 0, 0, 0};
-    if (ty > 0 && !bt.x_chunk) {
+    int chunk = tile ? tile->x_chunk : 0;
+    if (ty > 0 && !chunk) {
         // default chunk for all grids: of 8 .. 128 planes, the one for which the
         // items (planes + kItemPlanes each) of all grids, spread evenly over
         // the CTAs, plus one last item end first
@@ -589,7 +600,7 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
             const double t = work / (2.0 * nsm) + (double)longest;
             if (best_t < 0 || t < best_t) {
                 best_t = t;
-                bt.x_chunk = c;
+                chunk = c;
             }
         }
     }
@@ -597,7 +608,7 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     std::vector<int32_t> order((size_t)nsims);
     for (int32_t s = 0; s < nsims; s++) order[s] = s;
     auto item_len = [&](int32_t s) {
-        return std::min<int64_t>(bt.x_chunk, grids[s].nx) * 65536 + std::min<int64_t>(grids[s].ny, 65535);
+        return std::min<int64_t>(chunk, grids[s].nx) * 65536 + std::min<int64_t>(grids[s].ny, 65535);
     };
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return item_len(a) > item_len(b); });
     for (int32_t s = 0; s < nsims; s++)
@@ -606,7 +617,7 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
         const int32_t u = order[s];
         fdtd_yee_plan *pl = nullptr;
         const int st = yee_plan_create(&pl, &grids[u], &states[u], cpmls ? &cpmls[u] : nullptr,
-                                       srcs ? &srcs[u] : nullptr, &bt, status_dev, cur, stream, true);
+                                       srcs ? &srcs[u] : nullptr, tile, status_dev, cur, stream, std::max(chunk, 1));
         if (st != FDTD_OK) return st;
         ke = pl->k;
         any_drude = any_drude || pl->base.drude;

@@ -719,11 +719,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                 smax = __reduce_max_sync(0xffffffffu, smax);
             }
             if (lane == 0) {
-                if (n > MAX_LOCAL_SRC) {  // the host rejects such layouts; never drop a source silently
-                    atomicExch(p.status, FDTD_ERR_CAPACITY);
-                    n = MAX_LOCAL_SRC;
-                }
-                s_nls = n;
+                s_nls = n > MAX_LOCAL_SRC ? -1 : n;  // -1: more than the list holds, the planes scan all sources
                 s_smin = smin;
                 s_smax = smax;
             }
@@ -989,11 +985,21 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                 if (gen && TFSF && tplane) tfsf_group(0, te0, te1, ex, ey, ez);
                 if (gen && i >= smin && i <= smax) {  // soft sources, list order
                     const uint32_t ij_here = ((uint32_t)i << 16) | (uint32_t)jj;
-                    for (int s = 0; s < nls; s++) {
-                        if (s_ls_ij[s] != ij_here) continue;
-                        const int kc = s_ls_kc[s], d = (kc >> 2) - kk;
+                    const int ns = nls >= 0 ? nls : p.nsrc;
+                    for (int s = 0; s < ns; s++) {
+                        int kc, ls = s;
+                        if (nls >= 0) {
+                            if (s_ls_ij[s] != ij_here) continue;
+                            kc = s_ls_kc[s];
+                            ls = s_ls_s[s];
+                        } else {
+                            if (p.src_ijk[3 * s] != i || p.src_ijk[3 * s + 1] != jj) continue;
+                            kc = (p.src_ijk[3 * s + 2] << 2) | p.src_comp[s];
+                            if (p.zfix && slab_e(kc >> 2, P2, nz, (faces >> 4) & 1, (faces >> 5) & 1) >= 0) continue;
+                        }
+                        const int d = (kc >> 2) - kk;
                         if (d < 0 || d > 3) continue;
-                        const float v = p.src_amp[(int64_t)s_ls_s[s] * p.namp + p.t];
+                        const float v = p.src_amp[(int64_t)ls * p.namp + p.t];
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
                             if (e != d) continue;

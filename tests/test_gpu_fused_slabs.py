@@ -98,3 +98,45 @@ def test_band_range_and_plain_chunks():
             for s in (a, b):
                 s.set_fields(**{k: np.random.default_rng(1).standard_normal(shape) for k in NAMES})
         _check(a, b, 4)
+
+
+def _cluster(ranges, n, seed, ny=128, nz=128):
+    """n sources in each x range, rows 9..14, columns 70..100 of one tile, and n/4 repeats."""
+    rng = np.random.default_rng(seed)
+    amp = rng.standard_normal((n, 8))
+    src = []
+    for x0, x1 in ranges:
+        for m in range(n):
+            at = (int(rng.integers(x0, x1)), int(rng.integers(9, 15)), int(rng.integers(70, 101)))
+            src.append((("ex", "ey", "ez")[m % 3], at if m % 4 else (x0, 9, 70), amp[m]))
+    return src
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_sources_counted_per_default_chunk(batch):
+    """Sources are counted against the capacity of an item in chunks of 8 planes on these
+    grids (3 items an SM), not in the longer chunks the step takes: 120 in planes 1..6 and
+    120 in 9..14 are accepted, and applied although they share an item; 129 in 1..6 are refused."""
+    import fdtd_accelerate_gb300 as F
+    shape = (96, 128, 128) if batch else (128, 128, 128)
+
+    def build(src):
+        s = [F.YeeSolver(shape, npml=6, sources=src) for _ in range(2)]
+        for u in s:
+            u.set_fields(**{k: np.random.default_rng(5).standard_normal(shape).astype(np.float32) for k in NAMES})
+        if not batch:
+            return s, s[0]
+        return s, F.BatchSolver([s[0]] + [F.YeeSolver(shape, npml=6) for _ in range(7)])
+
+    s, run = build(_cluster(((1, 7), (9, 15)), 120, 7))
+    run.step(4)
+    s[1].step_unfused(4)
+    torch.cuda.synchronize()
+    run.check_status()
+    if not batch:
+        assert run.plan_info()["x_chunk"] > 8
+    for k in NAMES:
+        assert torch.equal(s[0].fields[k], s[1].fields[k]), k
+    with pytest.raises(ValueError):
+        s, run = build(_cluster(((1, 7),), 129, 8))
+        run.step(1)
