@@ -417,90 +417,69 @@ __device__ __forceinline__ void item_tile(const Params &p, int u, int &tz, int &
     xc = c == 0 ? 0 : (c == 1 ? p.nxc - 1 : c - 1);
 }
 
-// TFSF correction of one face slot: v += 0.5 (c * F1d[idx]) (kuFDTD/v0.2.0/dim3/tfsf.py:79-89)
-__device__ __forceinline__ void tfsf_add(const Params &p, int half, int f, int slot, const float *f1d, int64_t ax,
-                                         float &v) {
-    const int32_t ix = p.tix[half][f][slot];
-    const float c = p.tcoef[half][f][slot];
-    // the 1-D grid is read-only inside the fused kernel: read-only data cache
-    v = fadd(v, fmul(0.5f, fmul(c, __ldg(f1d + (ix >= 0 ? (int64_t)ix : ax + p.tvo)))));
-}
 __device__ __forceinline__ bool tin(int64_t x, int32_t lo, int32_t hi) { return x >= lo && x <= hi; }
 
-// Per item and lane: for each cell e of the pair, component and face family
-// (the two face axes that can correct that component, in face order), a
-// 2-bit code from the cell's (j, k): 0 none, 1 front face, 2 back face, 3 one of
-// the two x faces (decided per plane).  Layout: bit (e*12 + (comp*2 + fam)*2).
-// E (tfsf.py:154-186 e1/e2 slices): ex (y face, z face), ey (x face, z face),
-// ez (x face, y face); H: hx (y, z), hy (x, z), hz (x, y).
-__device__ __forceinline__ uint32_t tfsf_lane_codes(const Params &p, int eh, int64_t j, int64_t k0c, bool in0,
-                                                    bool in1) {
-    const int32_t j1 = p.tp1[1], k1 = p.tp1[2], j2 = p.tp2[1], k2 = p.tp2[2];
-    const int32_t f = p.tfaces;
-    auto code = [&](bool cand, bool back, int face_front) -> uint32_t {
-        if (!cand) return 0;
-        const int face = face_front + (back ? 1 : 0);
-        return ((f >> face) & 1) ? (back ? 2u : 1u) : 0u;
-    };
+// TFSF corrections (kuFDTD/v0.2.0/dim3/tfsf.py:79-89, e1/e2 slices :154-186).  Two face
+// families can correct a component, in this order: ex, hx the y then the z face; ey, hy
+// x, z; ez, hz x, y: families 0 .. 5.  E faces lie at p1-1 and p2, H faces at p1 and p2.
+//
+// Cells of the group (row j, cells k .. k+3) that each family corrects on the planes it
+// acts on: 4 bits a family, from bit 0.
+__device__ __forceinline__ uint32_t tfsf_masks(const Params &p, int eh, int64_t j, int64_t k, uint32_t inm) {
+    const int32_t j1 = p.tp1[1], k1 = p.tp1[2], j2 = p.tp2[1], k2 = p.tp2[2], f = p.tfaces;
+    // components that run along an axis end one cell before p2: E in the face's slot, H in the other
+    const bool ja = tin(j, j1, eh ? j2 : j2 - 1), jb = tin(j, j1, eh ? j2 - 1 : j2);
+    const bool yon = (j == (eh ? j1 : j1 - 1) && ((f >> 2) & 1)) || (j == j2 && ((f >> 3) & 1));
     uint32_t m = 0;
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-        if (!(e ? in1 : in0)) continue;
-        const int64_t k = k0c + e;
-        uint32_t c[6];
-        if (eh == 0) {
-            const int32_t je0 = j1 - 1, ke0 = k1 - 1;  // E faces at p1-1 and p2
-            c[0] = code((j == je0 || j == j2) && tin(k, k1, k2 - 1), j == j2, 2);     // ex, y face
-            c[1] = code((k == ke0 || k == k2) && tin(j, j1, j2 - 1), k == k2, 4);     // ex, z face
-            c[2] = tin(j, j1, j2) && tin(k, k1, k2 - 1) ? 3u : 0u;                    // ey, x face
-            c[3] = code((k == ke0 || k == k2) && tin(j, j1, j2), k == k2, 4);         // ey, z face
-            c[4] = tin(j, j1, j2 - 1) && tin(k, k1, k2) ? 3u : 0u;                    // ez, x face
-            c[5] = code((j == je0 || j == j2) && tin(k, k1, k2), j == j2, 2);         // ez, y face
-        } else {                                       // H faces at p1 and p2
-            c[0] = code((j == j1 || j == j2) && tin(k, k1, k2), j == j2, 2);          // hx, y face
-            c[1] = code((k == k1 || k == k2) && tin(j, j1, j2), k == k2, 4);          // hx, z face
-            c[2] = tin(j, j1, j2 - 1) && tin(k, k1, k2) ? 3u : 0u;                    // hy, x face
-            c[3] = code((k == k1 || k == k2) && tin(j, j1, j2 - 1), k == k2, 4);      // hy, z face
-            c[4] = tin(j, j1, j2) && tin(k, k1, k2 - 1) ? 3u : 0u;                    // hz, x face
-            c[5] = code((j == j1 || j == j2) && tin(k, k1, k2 - 1), j == j2, 2);      // hz, y face
-        }
-#pragma unroll
-        for (int q = 0; q < 6; q++) m |= c[q] << (e * 12 + q * 2);
+    for (int e = 0; e < 4; e++) {
+        if (!((inm >> e) & 1)) continue;
+        const int64_t kc = k + e;
+        const bool ka = tin(kc, k1, eh ? k2 : k2 - 1), kb = tin(kc, k1, eh ? k2 - 1 : k2);
+        const bool zon = (kc == (eh ? k1 : k1 - 1) && ((f >> 4) & 1)) || (kc == k2 && ((f >> 5) & 1));
+        m |= ((uint32_t)(yon && ka) | (uint32_t)(zon && ja) << 4 | (uint32_t)(jb && ka) << 8 |
+              (uint32_t)(zon && jb) << 12 | (uint32_t)(ja && kb) << 16 | (uint32_t)(yon && kb) << 20)
+             << e;
     }
     return m;
 }
 
-// Apply the TFSF terms of one cell (codes = its 12 bits) to the three
-// components of the E (eh = 0) or H (eh = 1) field just updated at plane i.
-// Slot and face of each family as tfsf.py:154-186; the x faces of E at p1-1 and
-// p2, of H at p1 and p2; for H the two families apply in face order.
-__device__ __forceinline__ void tfsf_apply(const Params &p, int eh, uint32_t codes, int64_t i, int64_t j, int64_t k,
-                                           float &vx, float &vy, float &vz) {
+// v += 0.5 (c * F1d[idx]) on the cells m of the group: one face, slot 0 or 1 of it
+__device__ __forceinline__ void tfsf_term(const Params &p, int eh, int face, int slot, int ax, uint32_t m, V4 &v) {
+    const float *f1d = eh == 0 ? p.th1d : p.te1d;  // read-only inside the fused kernel
+    const float c = p.tcoef[eh][face][slot];
+    const int ix = p.tix[eh][face][slot];
+    const int at = ix >= 0 ? ix : ax + p.tvo, step = ix < 0 && p.taxis == 2 ? 1 : 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if ((m >> e) & 1) v.v[e] = fadd(v.v[e], fmul(0.5f, fmul(c, __ldg(f1d + at + e * step))));
+}
+
+// The terms of one group (m: its masks) on plane i, E (eh = 0) or H (eh = 1).  A family
+// at a time, 4 cells each: one cell at a time, with the family's face and table looked up
+// for each, a plane of a tile with a y face row took 3 times as long (256^3, 12-cell
+// CPML, all faces of a 128^3 box: 404 us a step, now 340; the same step without a wave 247).
+__device__ __forceinline__ void tfsf_group(const Params &p, int eh, uint32_t m, int i, int j, int k, V4 &vx, V4 &vy,
+                                           V4 &vz) {
     const int32_t i1 = p.tp1[0], i2 = p.tp2[0];
-    const int64_t ax = p.taxis == 0 ? i : (p.taxis == 1 ? j : k);
-    const float *f1d = eh == 0 ? p.th1d : p.te1d;
-    const bool xf = eh == 0 ? i == i1 - 1 : i == i1, xb = i == i2;  // x face planes
-    const bool xface = (xf && (p.tfaces & 1)) || (xb && ((p.tfaces >> 1) & 1));
-    const int xid = xf ? 0 : 1;
-    // x-range of the y and z families: [i1, i2] or [i1, i2-1] per component
-    const bool ir = tin(i, i1, i2), irm = tin(i, i1, i2 - 1);
-    const uint32_t c0 = codes & 3, c1 = (codes >> 2) & 3, c2 = (codes >> 4) & 3, c3 = (codes >> 6) & 3,
-                   c4 = (codes >> 8) & 3, c5 = (codes >> 10) & 3;
-    if (eh == 0) {
-        if (c0 && ir) tfsf_add(p, 0, 2 + (int)c0 - 1, 1, f1d, ax, vx);      // ex += y face (slot e2)
-        if (c1 && ir) tfsf_add(p, 0, 4 + (int)c1 - 1, 0, f1d, ax, vx);      // ex += z face (e1)
-        if (c2 && xface) tfsf_add(p, 0, xid, 0, f1d, ax, vy);               // ey += x face (e1)
-        if (c3 && irm) tfsf_add(p, 0, 4 + (int)c3 - 1, 1, f1d, ax, vy);     // ey += z face (e2)
-        if (c4 && xface) tfsf_add(p, 0, xid, 1, f1d, ax, vz);               // ez += x face (e2)
-        if (c5 && irm) tfsf_add(p, 0, 2 + (int)c5 - 1, 0, f1d, ax, vz);     // ez += y face (e1)
-    } else {
-        if (c0 && irm) tfsf_add(p, 1, 2 + (int)c0 - 1, 1, f1d, ax, vx);     // hx += y face (h2)
-        if (c1 && irm) tfsf_add(p, 1, 4 + (int)c1 - 1, 0, f1d, ax, vx);     //    then z face (h1)
-        if (c2 && xface) tfsf_add(p, 1, xid, 0, f1d, ax, vy);               // hy += x face (h1)
-        if (c3 && ir) tfsf_add(p, 1, 4 + (int)c3 - 1, 1, f1d, ax, vy);      //    then z face (h2)
-        if (c4 && xface) tfsf_add(p, 1, xid, 1, f1d, ax, vz);               // hz += x face (h2)
-        if (c5 && ir) tfsf_add(p, 1, 2 + (int)c5 - 1, 0, f1d, ax, vz);      //    then y face (h1)
-    }
+    const bool xb = i == i2, xface = (i == (eh ? i1 : i1 - 1) && (p.tfaces & 1)) || (xb && ((p.tfaces >> 1) & 1));
+    if (!tin(i, i1, eh ? i2 - 1 : i2)) m &= ~0x0000ffu;  // y, z faces of the x component
+    if (!xface) m &= ~0x0f0f00u;
+    if (!tin(i, i1, eh ? i2 : i2 - 1)) m &= ~0xf0f000u;  // y, z faces of the z, y component
+    if (!m) return;
+    const int ax = p.taxis == 0 ? i : (p.taxis == 1 ? j : k);
+    const int fx = xb ? 1 : 0, fy = j == p.tp2[1] ? 3 : 2;
+    const uint32_t back = k <= p.tp2[2] && p.tp2[2] < k + 4 ? 1u << (p.tp2[2] - k) : 0u;
+    auto zfaces = [&](uint32_t z, int slot, V4 &v) {
+        if (z & ~back) tfsf_term(p, eh, 4, slot, ax, z & ~back, v);
+        if (z & back) tfsf_term(p, eh, 5, slot, ax, z & back, v);
+    };
+    if (m & 15u) tfsf_term(p, eh, fy, 1, ax, m & 15u, vx);
+    if ((m >> 4) & 15u) zfaces((m >> 4) & 15u, 0, vx);
+    if ((m >> 8) & 15u) tfsf_term(p, eh, fx, 0, ax, (m >> 8) & 15u, vy);
+    if ((m >> 12) & 15u) zfaces((m >> 12) & 15u, 1, vy);
+    if ((m >> 16) & 15u) tfsf_term(p, eh, fx, 1, ax, (m >> 16) & 15u, vz);
+    if (m >> 20) tfsf_term(p, eh, fy, 0, ax, m >> 20, vz);
 }
 
 // EXT: bit 0: the Drude box is compiled in, bit 1: the TFSF faces, bit 2: the
@@ -771,15 +750,10 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
         auto tfsf_plane = [&](int i) {
             return TFSF && t_rows && (tfsf_x(i) || (t_yz && i >= p.tp1[0] - 1 && i <= p.tp2[0]));
         };
-        // TFSF face codes of the group's two pairs (E, H), zero outside the box's faces
-        uint32_t te0 = 0, te1 = 0, th0 = 0, th1 = 0;
+        uint32_t te = 0, th = 0;  // TFSF cells of the group, zero outside the box's faces
         if (TFSF && t_rows) {
-            te0 = tfsf_lane_codes(p, 0, jj, kk, bit(inm, 0), bit(inm, 1));
-            te1 = tfsf_lane_codes(p, 0, jj, kk + 2, bit(inm, 2), bit(inm, 3));
-            if (own_t) {
-                th0 = tfsf_lane_codes(p, 1, jj, kk, bit(inm, 0), bit(inm, 1));
-                th1 = tfsf_lane_codes(p, 1, jj, kk + 2, bit(inm, 2), bit(inm, 3));
-            }
+            te = tfsf_masks(p, 0, jj, kk, inm);
+            if (own_t) th = tfsf_masks(p, 1, jj, kk, inm);
         }
 
         V4 hyc{}, hzc{};                // own hy, hz of the current plane
@@ -870,33 +844,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
             const float *H1 = h_t + (hs + 1 == L::NH ? 0 : hs + 1) * (L::HSLOT / 4);
             const float *E0 = e_t0 + es * (L::ESLOT / 4);
             float *N0 = n_t + nb * (3 * EB);
-            // TFSF corrections on this plane; the codes of the x faces (ey, ez / hy, hz slots)
-            // count on the face planes only
-            const bool tplane = gen && TFSF && tfsf_plane(i);
-            const uint32_t tx = gen && TFSF && tfsf_x(i) ? 0xfffu : 0xfffu & ~0x330u;
-            // (a loop over the cells: one copy of the correction's code a phase)
-            auto tfsf_group = [&](int eh, uint32_t c0, uint32_t c1, V4 &vx, V4 &vy, V4 &vz) {
-                if (!(c0 | c1)) return;
-#pragma unroll 1
-                for (int e = 0; e < 4; e++) {
-                    const uint32_t c = ((e < 2 ? c0 : c1) >> (e & 1 ? 12 : 0)) & tx;
-                    if (!c) continue;
-                    float x = vx.v[0], y = vy.v[0], z = vz.v[0];
-#pragma unroll
-                    for (int u = 1; u < 4; u++) {
-                        x = u == e ? vx.v[u] : x;
-                        y = u == e ? vy.v[u] : y;
-                        z = u == e ? vz.v[u] : z;
-                    }
-                    tfsf_apply(p, eh, c, i, jj, kk + e, x, y, z);
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        vx.v[u] = u == e ? x : vx.v[u];
-                        vy.v[u] = u == e ? y : vy.v[u];
-                        vz.v[u] = u == e ? z : vz.v[u];
-                    }
-                }
-            };
+            const bool tplane = gen && TFSF && tfsf_plane(i);  // TFSF corrections on this plane
             // ---- E phase ----
             V4 hx{}, hy1{}, hz1{}, ex{}, ey{}, ez{};
             if (e_t) {
@@ -982,7 +930,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     }
                 }
                 // TFSF: E += 0.5 (c * H1d), after the CPML terms, before the sources
-                if (gen && TFSF && tplane) tfsf_group(0, te0, te1, ex, ey, ez);
+                if (gen && TFSF && tplane && te) tfsf_group(p, 0, te, i, jj, kk, ex, ey, ez);
                 if (gen && i >= smin && i <= smax) {  // soft sources, list order
                     const uint32_t ij_here = ((uint32_t)i << 16) | (uint32_t)jj;
                     const int ns = nls >= 0 ? nls : p.nsrc;
@@ -1084,7 +1032,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     stz4(p.psi_h[5], qz, m1, zh, pz1, pext_y(p, 5));
                 }
                 // TFSF: H += 0.5 (c * E1d), after the CPML terms
-                if (gen && TFSF && tplane) tfsf_group(1, th0, th1, ox, oy, oz);
+                if (gen && TFSF && tplane && th) tfsf_group(p, 1, th, i, jj, kk, ox, oy, oz);
                 const int64_t gi = (int64_t)i * p.sx + (int64_t)jj * p.sy + kk;
                 stg4(p.out[0], gi, inm, true, ex, fext_y(p));
                 stg4(p.out[1], gi, inm, true, ey, fext_y(p));
