@@ -762,16 +762,16 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
         // planes that need more than the curl updates: all of them in tiles of a y or z
         // slab, else the x-slab, Drude, TFSF and source planes
         const bool tile_gen = __syncthreads_or(sye >= 0 || syh >= 0 || (ZIN && (ze.m || zh.m)));
-        // One plane: E phase, barrier, H phase.  Two copies of the code (gen: with the CPML,
-        // Drude, TFSF and source terms): most planes run the short one, which fits the
-        // instruction cache.  Returns false when a wait ran out.
-        auto plane = [&](auto gen_c, int q, bool late) -> bool {
-            constexpr bool gen = decltype(gen_c)::value;
+        // One plane: E phase, barrier, H phase.  Copies of the code (gen: with the Drude, TFSF
+        // and source terms; slab: with the CPML terms too): most planes run the shortest one,
+        // which fits the instruction cache.  Returns false when a wait ran out.
+        auto plane = [&](auto gen_c, auto slab_c, int q, bool late) -> bool {
+            constexpr bool gen = decltype(gen_c)::value, slab = decltype(slab_c)::value;
             const int i = i_start + q;
             const bool i_lt = i < nx - 1, i_gt = i > 0, own = own_t && i >= x0;
             // plane-uniform: x slab nodes
-            const int sxe = gen ? slab_e(i, P0, nx, faces & 1, (faces >> 1) & 1) : -1,
-                      sxh = gen ? slab_h(i, P0, nx, faces & 1, (faces >> 1) & 1) : -1;
+            const int sxe = slab ? slab_e(i, P0, nx, faces & 1, (faces >> 1) & 1) : -1,
+                      sxh = slab ? slab_h(i, P0, nx, faces & 1, (faces >> 1) & 1) : -1;
             // psi of this plane's slab cells: E psi now, H psi before the barrier below
             // (px, py, pz: the two arrays of the x, y and z slab)
             V4 px0{}, px1{}, py0{}, py1{}, pz0{}, pz1{};
@@ -782,15 +782,15 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                 px0 = ldg4(p.psi_e_in[0], qx, inm, vpsi, pext_y(p, 0));
                 px1 = ldg4(p.psi_e_in[1], qx, inm, vpsi, pext_y(p, 1));
             }
-            if (gen && sye >= 0) {
+            if (slab && sye >= 0) {
                 py0 = ldg4(p.psi_e_in[2], qy, inm, vpsi, pext_y(p, 2));
                 py1 = ldg4(p.psi_e_in[3], qy, inm, vpsi, pext_y(p, 3));
             }
-            if (ZIN && gen && ze.m) {
+            if (ZIN && slab && ze.m) {
                 pz0 = ldz4(p.psi_e_in[4], qz, ze.m, ze, pext_y(p, 4));
                 pz1 = ldz4(p.psi_e_in[5], qz, ze.m, ze, pext_y(p, 5));
             }
-            if (gen && q + 1 < nit) {
+            if (slab && q + 1 < nit) {
                 // the next plane's psi into L2: one plane is long enough for DRAM, and the
                 // loads above and before the barrier then wait for L2 only
                 const int64_t dx = (int64_t)ny * nz, dy = (int64_t)2 * P1 * nz, dz = (int64_t)ny * 2 * P2;
@@ -899,7 +899,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     ade(ey, cy, 1);
                     ade(ez, cz, 2);
                 }
-                if (gen && sxe >= 0) {  // x slab: ey -= cey (..dHz/dx..), ez += cez (..dHy/dx..)
+                if (slab && sxe >= 0) {  // x slab: ey -= cey (..dHz/dx..), ez += cez (..dHy/dx..)
                     const Coef c = tab_coef(tabs, 0, 2 * P0, 0, sxe);
                     const uint32_t m0 = inm & ltm, m1 = j_lt ? inm : 0u;
                     slab_term<-1>(ey, cy, px0, c, hz1, hzc, m0);
@@ -909,7 +909,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                         stg4(p.psi_e_out[1], qx, m1, vpsi, px1, pext_y(p, 1));
                     }
                 }
-                if (gen && sye >= 0) {  // y slab: ez -= cez (..dHx/dy..), ex += cex (..dHz/dy..)
+                if (slab && sye >= 0) {  // y slab: ez -= cez (..dHx/dy..), ex += cex (..dHz/dy..)
                     const Coef c = tab_coef(tabs, 12 * P0, 2 * P1, 0, sye);
                     const uint32_t m0 = i_lt ? inm : 0u, m1 = inm & ltm;
                     slab_term<-1>(ez, cz, py0, c, hxj, hx, m0);
@@ -919,7 +919,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                         stg4(p.psi_e_out[3], qy, m1, vpsi, py1, pext_y(p, 3));
                     }
                 }
-                if (ZIN && gen && ze.m) {  // z slab: ex -= cex (..dHy/dz..), ey += cey (..dHx/dz..)
+                if (ZIN && slab && ze.m) {  // z slab: ex -= cex (..dHy/dz..), ey += cey (..dHx/dz..)
                     const uint32_t m0 = j_lt ? ze.m : 0u, m1 = i_lt ? ze.m : 0u;
                     const V4 hxs{{hx.v[1], hx.v[2], hx.v[3], hxk4}}, hys{{hyc.v[1], hyc.v[2], hyc.v[3], hyk4}};
                     z_term<-1>(ex, cx, pz0, tabs + 12 * (P0 + P1), 2 * P2, ze, hys, hyc, m0);
@@ -965,15 +965,15 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
             const int64_t ux = ((int64_t)(sxh >= 0 ? sxh : 0) * ny + jj) * nz + kk;
             const int64_t uy = ((int64_t)i * 2 * P1 + (syh >= 0 ? syh : 0)) * nz + kk;
             if (own) {
-                if (gen && sxh >= 0) {
+                if (slab && sxh >= 0) {
                     px0 = ldg4(p.psi_h[0], ux, inm, vpsi, pext_y(p, 0));
                     px1 = ldg4(p.psi_h[1], ux, inm, vpsi, pext_y(p, 1));
                 }
-                if (gen && syh >= 0) {
+                if (slab && syh >= 0) {
                     py0 = ldg4(p.psi_h[2], uy, inm, vpsi, pext_y(p, 2));
                     py1 = ldg4(p.psi_h[3], uy, inm, vpsi, pext_y(p, 3));
                 }
-                if (ZIN && gen && zh.m) {
+                if (ZIN && slab && zh.m) {
                     pz0 = ldz4(p.psi_h[4], qz, zh.m, zh, pext_y(p, 4));
                     pz1 = ldz4(p.psi_h[5], qz, zh.m, zh, pext_y(p, 5));
                 }
@@ -1007,7 +1007,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     }
                 }
                 const V4 half{{0.5f, 0.5f, 0.5f, 0.5f}};
-                if (gen && sxh >= 0) {  // x slab: hy += (..dEz/dx..), hz -= (..dEy/dx..)
+                if (slab && sxh >= 0) {  // x slab: hy += (..dEz/dx..), hz -= (..dEy/dx..)
                     const Coef c = tab_coef(tabs, 0, 2 * P0, 1, sxh);
                     const uint32_t m0 = inm & gtm & ~hbm, m1 = j_gt ? inm & ~hbm : 0u;
                     slab_term<+1>(oy, half, px0, c, ez, prev_ez, m0);
@@ -1015,7 +1015,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     stg4(p.psi_h[0], ux, m0, vpsi, px0, pext_y(p, 0));
                     stg4(p.psi_h[1], ux, m1, vpsi, px1, pext_y(p, 1));
                 }
-                if (gen && syh >= 0) {  // y slab: hz += (..dEx/dy..), hx -= (..dEz/dy..)
+                if (slab && syh >= 0) {  // y slab: hz += (..dEx/dy..), hx -= (..dEz/dy..)
                     const Coef c = tab_coef(tabs, 12 * P0, 2 * P1, 1, syh);
                     const uint32_t m0 = i_gt ? inm & ~hbm : 0u, m1 = inm & gtm & ~hbm;
                     slab_term<+1>(oz, half, py0, c, ex, ex_j, m0);
@@ -1023,7 +1023,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     stg4(p.psi_h[2], uy, m0, vpsi, py0, pext_y(p, 2));
                     stg4(p.psi_h[3], uy, m1, vpsi, py1, pext_y(p, 3));
                 }
-                if (ZIN && gen && zh.m) {  // z slab: hx += (..dEy/dz..), hy -= (..dEx/dz..)
+                if (ZIN && slab && zh.m) {  // z slab: hx += (..dEy/dz..), hy -= (..dEx/dz..)
                     const uint32_t m0 = j_gt ? zh.m : 0u, m1 = i_gt ? zh.m : 0u;
                     const V4 eys{{eyk0, ey.v[0], ey.v[1], ey.v[2]}}, exs{{exk0, ex.v[0], ex.v[1], ex.v[2]}};
                     z_term<+1>(ox, half, pz0, tabs + 12 * (P0 + P1) + 6 * P2, 2 * P2, zh, ey, eys, m0);
@@ -1052,9 +1052,19 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
             const int i = i_start + q;
             // E(q), CE(q) and H(q+1) have arrived (H(q) with the stage before)
             const bool late = !mbar_wait_bounded(&bars[es], par, p.status, wlim);
-            const bool gen = tile_gen || (P0 > 0 && (i <= P0 || i >= nx - P0 - 1)) || (i >= smin && i <= smax) ||
+            const bool slab = tile_gen || (P0 > 0 && (i <= P0 || i >= nx - P0 - 1));
+            const bool ext = (i >= smin && i <= smax) ||
                              (DRUDE && dtile && i >= p.dbox[0] && i < p.dbox[0] + p.dbox[3]) || (TFSF && tfsf_plane(i));
-            if (!(gen ? plane(std::true_type{}, q, late) : plane(std::false_type{}, q, late))) {
+            // Drude and TFSF planes off the slabs run a copy without the CPML terms (256^3 with
+            // bands: 343 -> 310 us a step with a 128^3 wave box, 295 -> 287 with a 128^3 Drude
+            // box).  Not where the kernel has the z terms: those grids are small, their planes
+            // of all kinds alternate, and a third copy costs more (64^3, Drude: 17.1 -> 19.0).
+            using std::true_type, std::false_type;
+            constexpr bool own_copy = (DRUDE || TFSF) && !ZIN;
+            const bool ok = slab || (!own_copy && ext) ? plane(true_type{}, true_type{}, q, late)
+                            : own_copy && ext          ? plane(true_type{}, std::bool_constant<!own_copy>{}, q, late)
+                                                       : plane(false_type{}, false_type{}, q, late);
+            if (!ok) {
                 aborted = true;
                 q_abort = q;
                 break;
