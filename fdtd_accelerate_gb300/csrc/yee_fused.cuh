@@ -56,6 +56,7 @@ constexpr int GZ = TZ / 4;   // groups of 4 z cells in a tile row
 constexpr int HC = TZ + 8;   // H box:    k0-4 .. k0+TZ+3 (needs k0-1 .. k0+TZ)
 constexpr int EC = TZ + 4;   // E/CE box: k0-4 .. k0+TZ-1 (needs k0-1 .. k0+TZ-1); E_new rows too
 constexpr int MAX_LOCAL_SRC = 128;
+constexpr int MAX_ORDERED = 32;     // x chunks whose order a plan holds
 constexpr int MAX_BAND_SRC = 32;
 constexpr uint64_t WAIT_NS = 1000000000ull;  // a wait gives up after 1 s
 
@@ -97,6 +98,7 @@ struct Params {
     int32_t ntz, nty, nxc, x_chunk;
     // tile rows at either end that hold y slab cells (item order)
     int32_t yf, yb;
+    uint8_t xorder[MAX_ORDERED];  // the x chunks in item order, when there are no more than that
     float *out[6];  // ex, ey, ez, hx, hy, hz of the output buffer
     const float *psi_e_in[6];
     float *psi_e_out[6];
@@ -404,7 +406,8 @@ __device__ __forceinline__ void z_term(V4 &f, const V4 &cf, V4 &psi, const float
 // tile and x chunk of work item u: the tile rows that hold y slab cells first
 // (their planes take up to twice as long: started last, they would be the
 // launch's tail; 256^3 with y faces alone 213 -> 180 us), z tile fastest, and
-// of either kind the first and the last x chunk (x slab planes) first.  Not so
+// of either kind the x chunks with most slab, Drude and TFSF planes first (the
+// first and the last one, where there are too many for the table).  Not so
 // the z-edge tiles, which are as slow: apart from their neighbours in time,
 // they would share no halo reads through L2 (1024x1024x512: 6.1 -> 7.0 ms).
 __device__ __forceinline__ void item_tile(const Params &p, int u, int &tz, int &ty, int &xc) {
@@ -414,7 +417,7 @@ __device__ __forceinline__ void item_tile(const Params &p, int u, int &tz, int &
     const int tiles = p.ntz * (first ? ye : nm), c = u / tiles, t = u % tiles, r = t / p.ntz;
     tz = t % p.ntz;
     ty = first ? (r < p.yf ? r : p.nty - ye + r) : p.yf + r;
-    xc = c == 0 ? 0 : (c == 1 ? p.nxc - 1 : c - 1);
+    xc = p.nxc <= MAX_ORDERED ? p.xorder[c] : c == 0 ? 0 : (c == 1 ? p.nxc - 1 : c - 1);
 }
 
 __device__ __forceinline__ bool tin(int64_t x, int32_t lo, int32_t hi) { return x >= lo && x <= hi; }
