@@ -18,8 +18,9 @@
 //    k_lo rounded up to 4): E_new there needs H_new of rows j_lo-1 .. j_hi+1,
 //    where no y or z CPML node lies.  So the pair kernel carries the x-slab
 //    terms only.  The rest of the grid (the y and z slabs plus two cells) is
-//    the edge shell, advanced by one-thread-per-cell kernels (k_edge_*), out
-//    of place, after the pair kernel has written the inside H_new.
+//    the edge shell, advanced by kernels of 4 cells a thread (k_edge_*), out
+//    of place; their E stage runs after the pair kernel has written the inside
+//    H_new.  Small grids are all shell.
 //  * Pair kernel, 2.5-D blocking: a CTA owns TZ = 32 (z) x TY = 16 (y) cells
 //    for a chunk of x planes and marches along x.  E_new(i) needs H_new on
 //    planes i-1 .. i+2 and on the rows/columns -1 .. +2 around the tile, so
@@ -46,11 +47,11 @@
 #include <cuda.h>
 
 #include <algorithm>
-#include <functional>
-#include <queue>
+#include <map>
 #include <vector>
 
 #include "common.cuh"
+#include "symp_group.cuh"
 
 namespace fdtd {
 namespace sp {
@@ -111,6 +112,7 @@ struct Params {
     int32_t kt0;              // first z tile origin (k_lo rounded down to TZ)
     const float *in[6];       // ex, ey, ez, hx, hy, hz of the input buffer (edge kernels)
     const float *ce[3];
+    int32_t vpsi;             // the x and y psi arrays' rows are 16-byte multiples (edge kernels)
     int32_t nsrc;
     const int32_t *src_ijk, *src_comp;
     const float *src_amp;
@@ -177,21 +179,11 @@ __device__ __forceinline__ int slab(const Axis &A, int x, int n, bool e) {
     if (A.back && x >= b0 && x <= b1) return A.P + x - b0;
     return -1;
 }
-// psi element of slab s along ax at (i, j, k)
-__device__ __forceinline__ uint32_t psi_index(const Params &p, int ax, int s, int i, int j, int k, int P) {
-    const uint32_t twoP = 2u * (uint32_t)P;
-    return ax == 0 ? ((uint32_t)s * p.ny + j) * p.nz + k
-                   : (ax == 1 ? ((uint32_t)i * twoP + s) * p.nz + k : ((uint32_t)i * p.ny + j) * twoP + s);
-}
 // CPML tables of one stage along one axis
 struct Tab {
     const float *b, *a, *km1;
 };
 __device__ __forceinline__ Tab tab(const Axis &A) { return Tab{A.b, A.a, A.km1}; }
-// the tables of H stage b (st = 1) or a, selected by value
-__device__ __forceinline__ Tab tab_h(const Params &p, int st, int ax) {
-    return Tab{st ? p.hb[ax].b : p.ha[ax].b, st ? p.hb[ax].a : p.ha[ax].a, st ? p.hb[ax].km1 : p.ha[ax].km1};
-}
 // psi <- b psi + a d; returns (coef * cv) * (km1 d + psi)
 __device__ __forceinline__ float sterm(const Tab &T, int s, float &psi, float d, float coef, float cv) {
     psi = fadd(fmul(__ldg(T.b + s), psi), fmul(__ldg(T.a + s), d));
@@ -282,6 +274,10 @@ k_symp_pair(const __grid_constant__ Maps mk, const __grid_constant__ Params p) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         s_abort = 0;
     }
+    // nothing above touches global memory; the edge kernel may start beside this one, whose
+    // CTAs (never more than are resident) have all seen the launches before it end
+    grid_wait();
+    grid_release();
     // the group of this thread: H row hr (j0-1+hr), group g (columns
     // k0-4+4g .. k0-1+4g).  Tile groups first (row hr = 1 + tid/8, groups
     // 1 .. 8), then the halo: rows 0, TY+1, TY+2 (all groups), then groups 0
@@ -718,7 +714,7 @@ k_symp_pair(const __grid_constant__ Maps mk, const __grid_constant__ Params p) {
 
 // ---------------------------------------------------------------------------
 // Edge shell: the cells outside the pair kernel's tiles (the y and z CPML
-// slabs and a tile of margin), one thread per cell, out of place:
+// slabs and a tile of margin), 4 z cells a thread (symp_group.cuh), out of place:
 //   k_edge_h         H_out = H_in - clch_a curl4(E_in) with its CPML terms
 //                    (psi_h_in -> psi_h_out); in a two-H pass the second
 //                    stage follows in registers (same E_in, psi carried);
@@ -733,193 +729,77 @@ k_symp_pair(const __grid_constant__ Maps mk, const __grid_constant__ Params p) {
 struct Edge {
     int32_t n;                           // boxes
     int32_t j0[4], j1[4], k0[4], k1[4];  // rows [j0, j1), columns [k0, k1), every x plane
-    uint32_t off[5];                     // first cell of each box within one x plane
-    uint32_t rcp[4];                     // ceil(2^32 / width) of each box (division by the width)
+    uint32_t off[5];                     // first group of 4 cells of each box within one x plane
+    uint32_t rcp[4];                     // ceil(2^32 / groups a row) of each box (division by it)
 };
 constexpr int EDGE_BLOCK = 128;
 
-// launch: blockIdx.y = x plane, blockIdx.x * EDGE_BLOCK + threadIdx.x = cell of
-// the plane's part of the shell (box by box, z fastest)
-__device__ __forceinline__ bool edge_cell(const Edge &eb, int &i, int &j, int &k) {
+// launch: blockIdx.y = x plane, blockIdx.x * EDGE_BLOCK + threadIdx.x = group of
+// the plane's part of the shell (box by box, z fastest; every box starts at a
+// multiple of 4 columns and ends at one or at nz)
+__device__ __forceinline__ bool edge_group(const Edge &eb, int &i, int &j, int &k) {
     const uint32_t u = blockIdx.x * EDGE_BLOCK + threadIdx.x;
     if (u >= eb.off[eb.n]) return false;
     int b = 0;
     while (b + 1 < eb.n && u >= eb.off[b + 1]) b++;
-    const uint32_t v = u - eb.off[b], nk = (uint32_t)(eb.k1[b] - eb.k0[b]);
-    uint32_t r = __umulhi(v, eb.rcp[b]);  // v / nk, or one off
-    if (r * nk > v) r--;
-    else if ((r + 1) * nk <= v) r++;
-    k = eb.k0[b] + (int)(v - r * nk);
+    const uint32_t v = u - eb.off[b], ng = (uint32_t)(eb.k1[b] - eb.k0[b] + 3) / 4;
+    uint32_t r = __umulhi(v, eb.rcp[b]);  // v / ng, or one off
+    if (r * ng > v) r--;
+    else if ((r + 1) * ng <= v) r++;
+    k = eb.k0[b] + 4 * (int)(v - r * ng);
     j = eb.j0[b] + (int)r;
     i = blockIdx.y;
     return true;
 }
 
+// the edge kernels' stages (sg::stage): E or the H stages a, b of a pass
+template <bool E>
+struct EdgeStage {
+    const Params &p;
+    __device__ __forceinline__ const Axis &axis(int st, int ax) const { return E ? p.ea[ax] : st ? p.hb[ax] : p.ha[ax]; }
+    __device__ __forceinline__ const float *fin(int q) const { return p.in[(E ? 0 : 3) + q]; }
+    __device__ __forceinline__ float *fout(int q) const { return p.out[(E ? 0 : 3) + q]; }
+    __device__ __forceinline__ const float *g(int q) const { return E ? p.out[3 + q] : p.in[q]; }
+    __device__ __forceinline__ const float *psi_in(int a) const { return E ? p.psi_e[a] : p.psi_h_in[a]; }
+    __device__ __forceinline__ float *psi_out(int a) const { return E ? p.psi_e[a] : p.psi_h_out[a]; }
+    __device__ __forceinline__ bool vpsi() const { return p.vpsi != 0; }
+    __device__ __forceinline__ int P(int ax) const { return axis(0, ax).P; }
+    __device__ __forceinline__ bool front(int ax) const { return axis(0, ax).front; }
+    __device__ __forceinline__ bool back(int ax) const { return axis(0, ax).back; }
+    __device__ __forceinline__ sg::Tab tab(int st, int ax) const {
+        const Axis &A = axis(st, ax);
+        return sg::Tab{A.b, A.a, A.km1};
+    }
+    __device__ __forceinline__ float coef(int st) const { return E ? p.dl : st ? p.cl_b : p.cl_a; }
+    __device__ __forceinline__ sg::F4 cv(int q, const sg::Group &g) const {
+        return E ? g.ldg(p.ce[q], g.c) : sg::F4{{p.ch, p.ch, p.ch, p.ch}};
+    }
+    __device__ __forceinline__ float main(int st, float v, float cv, float d27) const {
+        return E ? fadd(v, fmul(fmul(p.dl, cv), d27)) : fsub(v, fmul(st ? p.clch_b : p.clch_a, d27));
+    }
+};
+
 template <bool HH>
 __global__ void __launch_bounds__(EDGE_BLOCK)
-k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
+k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb, int32_t beside) {
+    // beside: started by the pair kernel's release, so the launches before that one have
+    // ended, and this one reads nothing that the pair kernel writes.  Its own end stands for
+    // both kernels': its last block waits for the pair kernel.
+    if (!beside) grid_wait();
+    grid_release();
     int i, j, k;
-    if (!edge_cell(eb, i, j, k)) return;
-    const uint32_t X = p.sx, Y = p.sy, c = (uint32_t)i * X + (uint32_t)j * Y + (uint32_t)k;
-    const float *ex = p.in[0], *ey = p.in[1], *ez = p.in[2];
-    [[maybe_unused]] const int64_t FE = fext(p);
-    [[maybe_unused]] const int64_t PE0 = pext(p, 0, p.ha[0].P), PE1 = PE0, PE2 = pext(p, 1, p.ha[1].P),
-                                   PE3 = PE2, PE4 = pext(p, 2, p.ha[2].P), PE5 = PE4;
-    const bool jin = j > 1 && j < p.ny - 1, kin = k > 1 && k < p.nz - 1, iin = i > 1 && i < p.nx - 1;
-    const int sx = slab(p.ha[0], i, p.nx, false), sy = slab(p.ha[1], j, p.ny, false),
-              sz = slab(p.ha[2], k, p.nz, false);
-    // One component: the input H, then per stage (a, then b in a two-H pass)
-    // the main term and the two CPML terms (signs s1, s2: +1 adds), psi
-    // carried from stage a to stage b in registers; E_in is the same for both
-    // stages, so are d27 and the one-axis differences.
-    auto comp = [&](int q, bool upd, float d27, int a1, int s1, int q1, float d1, int a2, int s2, int q2, float d2) {
-        float v = LDG(p.in[3 + q], c, FE);
-        if (upd) {
-            const int sl1 = a1 == 0 ? sx : (a1 == 1 ? sy : sz), sl2 = a2 == 0 ? sx : (a2 == 1 ? sy : sz);
-            [[maybe_unused]] const int64_t pe1 = a1 == 0 ? PE0 : (a1 == 1 ? PE2 : PE4),
-                                           pe2 = a2 == 0 ? PE0 : (a2 == 1 ? PE2 : PE4);
-            uint32_t i1 = 0, i2 = 0;
-            float ps1 = 0.f, ps2 = 0.f;
-            if (sl1 >= 0) {
-                i1 = psi_index(p, a1, sl1, i, j, k, p.ha[a1].P);
-                ps1 = FDTD_IN(i1, pe1) ? p.psi_h_in[q1][i1] : 0.f;
-            }
-            if (sl2 >= 0) {
-                i2 = psi_index(p, a2, sl2, i, j, k, p.ha[a2].P);
-                ps2 = FDTD_IN(i2, pe2) ? p.psi_h_in[q2][i2] : 0.f;
-            }
-#pragma unroll
-            for (int st = 0; st < (HH ? 2 : 1); st++) {
-                const float clch = st ? p.clch_b : p.clch_a, cl = st ? p.cl_b : p.cl_a;
-                v = fsub(v, fmul(clch, d27));
-                if (sl1 >= 0) {
-                    const float t = sterm(tab_h(p, st, a1), sl1, ps1, d1, cl, p.ch);
-                    v = s1 > 0 ? fadd(v, t) : fsub(v, t);
-                }
-                if (sl2 >= 0) {
-                    const float t = sterm(tab_h(p, st, a2), sl2, ps2, d2, cl, p.ch);
-                    v = s2 > 0 ? fadd(v, t) : fsub(v, t);
-                }
-            }
-            if (sl1 >= 0 && FDTD_IN(i1, pe1)) p.psi_h_out[q1][i1] = ps1;
-            if (sl2 >= 0 && FDTD_IN(i2, pe2)) p.psi_h_out[q2][i2] = ps2;
-        }
-        if (FDTD_IN(c, FE)) p.out[3 + q][c] = v;
-    };
-    {   // hx: y term subtracted, z term added
-        float d27 = 0.f, dy = 0.f, dz = 0.f;
-        if (jin && kin) {
-            const float n = curl4(LDG(ez, c, FE), LDG(ez, c - Y, FE), LDG(ey, c, FE), LDG(ey, c - 1, FE));
-            const float f = curl4(LDG(ez, c + Y, FE), LDG(ez, c - 2 * Y, FE), LDG(ey, c + 1, FE), LDG(ey, c - 2, FE));
-            d27 = fsub(fmul(27.0f, n), f);
-            if (sy >= 0) dy = d4h(LDG(ez, c - 2 * Y, FE), LDG(ez, c - Y, FE), LDG(ez, c, FE), LDG(ez, c + Y, FE));
-            if (sz >= 0) dz = d4h(LDG(ey, c - 2, FE), LDG(ey, c - 1, FE), LDG(ey, c, FE), LDG(ey, c + 1, FE));
-        }
-        comp(0, jin && kin, d27, 1, -1, 3, dy, 2, +1, 4, dz);
-    }
-    {   // hy: x term added, z term subtracted
-        float d27 = 0.f, dx = 0.f, dz = 0.f;
-        if (iin && kin) {
-            const float n = curl4(LDG(ex, c, FE), LDG(ex, c - 1, FE), LDG(ez, c, FE), LDG(ez, c - X, FE));
-            const float f = curl4(LDG(ex, c + 1, FE), LDG(ex, c - 2, FE), LDG(ez, c + X, FE), LDG(ez, c - 2 * X, FE));
-            d27 = fsub(fmul(27.0f, n), f);
-            if (sx >= 0) dx = d4h(LDG(ez, c - 2 * X, FE), LDG(ez, c - X, FE), LDG(ez, c, FE), LDG(ez, c + X, FE));
-            if (sz >= 0) dz = d4h(LDG(ex, c - 2, FE), LDG(ex, c - 1, FE), LDG(ex, c, FE), LDG(ex, c + 1, FE));
-        }
-        comp(1, iin && kin, d27, 0, +1, 0, dx, 2, -1, 5, dz);
-    }
-    {   // hz: x term subtracted, y term added
-        float d27 = 0.f, dx = 0.f, dy = 0.f;
-        if (iin && jin) {
-            const float n = curl4(LDG(ey, c, FE), LDG(ey, c - X, FE), LDG(ex, c, FE), LDG(ex, c - Y, FE));
-            const float f = curl4(LDG(ey, c + X, FE), LDG(ey, c - 2 * X, FE), LDG(ex, c + Y, FE), LDG(ex, c - 2 * Y, FE));
-            d27 = fsub(fmul(27.0f, n), f);
-            if (sx >= 0) dx = d4h(LDG(ey, c - 2 * X, FE), LDG(ey, c - X, FE), LDG(ey, c, FE), LDG(ey, c + X, FE));
-            if (sy >= 0) dy = d4h(LDG(ex, c - 2 * Y, FE), LDG(ex, c - Y, FE), LDG(ex, c, FE), LDG(ex, c + Y, FE));
-        }
-        comp(2, iin && jin, d27, 0, -1, 1, dx, 1, +1, 2, dy);
-    }
+    if (beside && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && threadIdx.x == 0) grid_wait();
+    if (!edge_group(eb, i, j, k)) return;
+    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false>{p});
 }
 
 __global__ void __launch_bounds__(EDGE_BLOCK)
 k_edge_e(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
+    grid_wait();
+    grid_release();
     int i, j, k;
-    if (!edge_cell(eb, i, j, k)) return;
-    const uint32_t X = p.sx, Y = p.sy, c = (uint32_t)i * X + (uint32_t)j * Y + (uint32_t)k;
-    const float *hx = p.out[3], *hy = p.out[4], *hz = p.out[5];
-    [[maybe_unused]] const int64_t FE = fext(p);
-    [[maybe_unused]] const int64_t PE0 = pext(p, 0, p.ea[0].P), PE1 = PE0, PE2 = pext(p, 1, p.ea[1].P),
-                                   PE3 = PE2, PE4 = pext(p, 2, p.ea[2].P), PE5 = PE4;
-    const Tab T0 = tab(p.ea[0]), T1 = tab(p.ea[1]), T2 = tab(p.ea[2]);
-    const bool jin = j > 0 && j < p.ny - 2, kin = k > 0 && k < p.nz - 2, iin = i > 0 && i < p.nx - 2;
-    const int sx = slab(p.ea[0], i, p.nx, true), sy = slab(p.ea[1], j, p.ny, true),
-              sz = slab(p.ea[2], k, p.nz, true);
-    {   // ex: y term added, z term subtracted
-        float v = LDG(p.in[0], c, FE);
-        if (jin && kin) {
-            const float n = curl4(LDG(hz, c + Y, FE), LDG(hz, c, FE), LDG(hy, c + 1, FE), LDG(hy, c, FE));
-            const float f = curl4(LDG(hz, c + 2 * Y, FE), LDG(hz, c - Y, FE), LDG(hy, c + 2, FE), LDG(hy, c - 1, FE));
-            const float cv = LDG(p.ce[0], c, FE);
-            v = fadd(v, fmul(fmul(p.dl, cv), fsub(fmul(27.0f, n), f)));
-            if (sy >= 0) {
-                const uint32_t q = psi_index(p, 1, sy, i, j, k, p.ea[1].P);
-                float ps = FDTD_IN(q, PE3) ? p.psi_e[3][q] : 0.f;
-                v = fadd(v, sterm(T1, sy, ps, d4e(LDG(hz, c - Y, FE), LDG(hz, c, FE), LDG(hz, c + Y, FE), LDG(hz, c + 2 * Y, FE)), p.dl, cv));
-                if (FDTD_IN(q, PE3)) p.psi_e[3][q] = ps;
-            }
-            if (sz >= 0) {
-                const uint32_t q = psi_index(p, 2, sz, i, j, k, p.ea[2].P);
-                float ps = FDTD_IN(q, PE4) ? p.psi_e[4][q] : 0.f;
-                v = fsub(v, sterm(T2, sz, ps, d4e(LDG(hy, c - 1, FE), LDG(hy, c, FE), LDG(hy, c + 1, FE), LDG(hy, c + 2, FE)), p.dl, cv));
-                if (FDTD_IN(q, PE4)) p.psi_e[4][q] = ps;
-            }
-        }
-        if (FDTD_IN(c, FE)) p.out[0][c] = v;
-    }
-    {   // ey: x term subtracted, z term added
-        float v = LDG(p.in[1], c, FE);
-        if (iin && kin) {
-            const float n = curl4(LDG(hx, c + 1, FE), LDG(hx, c, FE), LDG(hz, c + X, FE), LDG(hz, c, FE));
-            const float f = curl4(LDG(hx, c + 2, FE), LDG(hx, c - 1, FE), LDG(hz, c + 2 * X, FE), LDG(hz, c - X, FE));
-            const float cv = LDG(p.ce[1], c, FE);
-            v = fadd(v, fmul(fmul(p.dl, cv), fsub(fmul(27.0f, n), f)));
-            if (sx >= 0) {
-                const uint32_t q = psi_index(p, 0, sx, i, j, k, p.ea[0].P);
-                float ps = FDTD_IN(q, PE0) ? p.psi_e[0][q] : 0.f;
-                v = fsub(v, sterm(T0, sx, ps, d4e(LDG(hz, c - X, FE), LDG(hz, c, FE), LDG(hz, c + X, FE), LDG(hz, c + 2 * X, FE)), p.dl, cv));
-                if (FDTD_IN(q, PE0)) p.psi_e[0][q] = ps;
-            }
-            if (sz >= 0) {
-                const uint32_t q = psi_index(p, 2, sz, i, j, k, p.ea[2].P);
-                float ps = FDTD_IN(q, PE5) ? p.psi_e[5][q] : 0.f;
-                v = fadd(v, sterm(T2, sz, ps, d4e(LDG(hx, c - 1, FE), LDG(hx, c, FE), LDG(hx, c + 1, FE), LDG(hx, c + 2, FE)), p.dl, cv));
-                if (FDTD_IN(q, PE5)) p.psi_e[5][q] = ps;
-            }
-        }
-        if (FDTD_IN(c, FE)) p.out[1][c] = v;
-    }
-    {   // ez: x term added, y term subtracted
-        float v = LDG(p.in[2], c, FE);
-        if (iin && jin) {
-            const float n = curl4(LDG(hy, c + X, FE), LDG(hy, c, FE), LDG(hx, c + Y, FE), LDG(hx, c, FE));
-            const float f = curl4(LDG(hy, c + 2 * X, FE), LDG(hy, c - X, FE), LDG(hx, c + 2 * Y, FE), LDG(hx, c - Y, FE));
-            const float cv = LDG(p.ce[2], c, FE);
-            v = fadd(v, fmul(fmul(p.dl, cv), fsub(fmul(27.0f, n), f)));
-            if (sx >= 0) {
-                const uint32_t q = psi_index(p, 0, sx, i, j, k, p.ea[0].P);
-                float ps = FDTD_IN(q, PE1) ? p.psi_e[1][q] : 0.f;
-                v = fadd(v, sterm(T0, sx, ps, d4e(LDG(hy, c - X, FE), LDG(hy, c, FE), LDG(hy, c + X, FE), LDG(hy, c + 2 * X, FE)), p.dl, cv));
-                if (FDTD_IN(q, PE1)) p.psi_e[1][q] = ps;
-            }
-            if (sy >= 0) {
-                const uint32_t q = psi_index(p, 1, sy, i, j, k, p.ea[1].P);
-                float ps = FDTD_IN(q, PE2) ? p.psi_e[2][q] : 0.f;
-                v = fsub(v, sterm(T1, sy, ps, d4e(LDG(hx, c - Y, FE), LDG(hx, c, FE), LDG(hx, c + Y, FE), LDG(hx, c + 2 * Y, FE)), p.dl, cv));
-                if (FDTD_IN(q, PE2)) p.psi_e[2][q] = ps;
-            }
-        }
-        if (FDTD_IN(c, FE)) p.out[2][c] = v;
-    }
+    if (!edge_group(eb, i, j, k)) return;
+    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true>{p});
 }
 
 // soft sources on edge cells, list order (one thread: a list holds a few sources)
@@ -983,31 +863,41 @@ static int map3(EncodeFn enc, CUtensorMap *m, const float *ptr, const Grid &g, i
 static int choose_x_chunk(int nx, int64_t tiles, int slots, int pf, int pb) {
     int best = std::min(nx, 128);
     int64_t best_t = -1;
-    std::vector<int64_t> heap;
+    std::map<int64_t, int64_t> free_at;  // CTAs by the time they are free
     int last = -1;
     const int least = tiles * ((nx + 47) / 48) < 2 * (int64_t)slots ? 8 : 48;
     for (int xc = 256; xc >= least; xc -= 8) {
         const int c = std::min(xc, nx);
         if (c == last) continue;  // chunks past nx are all the whole grid
         last = c;
-        heap.assign((size_t)slots, 0);
+        free_at = {{0, slots}};
         for (int x0 = 0; x0 < nx; x0 += c) {
             const int x1 = std::min(nx, x0 + c);
             int64_t cost = 6;
             for (int i = x0; i < x1; i++) cost += ((pf > 0 && i <= pf + 1) || (pb > 0 && i >= nx - pb - 2)) ? 2 : 1;
-            for (int64_t t = 0; t < tiles; t++) {  // the CTA free first takes the item
-                std::pop_heap(heap.begin(), heap.end(), std::greater<int64_t>());
-                heap.back() += cost;
-                std::push_heap(heap.begin(), heap.end(), std::greater<int64_t>());
+            for (int64_t left = tiles; left > 0;) {  // the CTAs free first take the items
+                const auto first = *free_at.begin();
+                const int64_t n = std::min(first.second, left);
+                if (n == first.second) free_at.erase(free_at.begin());
+                else free_at.begin()->second -= n;
+                free_at[first.first + cost] += n;
+                left -= n;
             }
         }
-        const int64_t t = *std::max_element(heap.begin(), heap.end());
+        const int64_t t = free_at.rbegin()->first;
         if (best_t < 0 || t < best_t) {
             best_t = t;
             best = c;
         }
     }
     return best;
+}
+
+// launched the plain way, or chained (its grid_wait then stands for the launch's own)
+template <typename... P, typename... A>
+static void launch(bool chained, void (*fn)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, const A &...args) {
+    if (chained) launch_chained(fn, grid, dim3((unsigned)block), smem, st, 1, args...);
+    else fn<<<grid, block, smem, st>>>(args...);
 }
 
 struct fdtd_symp_plan {
@@ -1156,6 +1046,10 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
         }
     }
     for (int q = 0; q < 6; q++) p.in[q] = pl->f[in][q];
+    p.vpsi = p.nz % 4 == 0;
+    for (int q = 0; q < 4; q++)
+        for (const float *a : {p.psi_h_in[q], (const float *)p.psi_h_out[q], (const float *)p.psi_e[q]})
+            p.vpsi = p.vpsi && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
     // the pair kernel's region: E_new of rows [j_lo, j_hi) needs H_new of rows
     // j_lo-1 .. j_hi+1, which must hold no y-slab node of any stage (front
     // nodes 1 .. P, back nodes n-P-1 .. n-1): j_lo = P+2, j_hi = n-P-2; the
@@ -1192,26 +1086,6 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
         p.x_chunk = pl->chunk_val;
         p.nxc = (p.nx + p.x_chunk - 1) / p.x_chunk;
     }
-    // the edge shell: rows outside [j_lo, j_hi), then the columns outside
-    // [k_lo, k_hi) of those rows (every x plane)
-    Edge eb{};
-    auto add_box = [&](int64_t j0, int64_t j1, int64_t k0, int64_t k1) {
-        if (j1 <= j0 || k1 <= k0) return;
-        eb.j0[eb.n] = (int)j0; eb.j1[eb.n] = (int)j1; eb.k0[eb.n] = (int)k0; eb.k1[eb.n] = (int)k1;
-        eb.off[eb.n + 1] = eb.off[eb.n] + (uint32_t)((j1 - j0) * (k1 - k0));
-        eb.rcp[eb.n] = (uint32_t)std::min<uint64_t>((((uint64_t)1 << 32) + (uint64_t)(k1 - k0) - 1) / (uint64_t)(k1 - k0),
-                                                    0xFFFFFFFFull);
-        eb.n++;
-    };
-    if (p.nty_in == 0 || p.ntz_in == 0) {
-        p.nty_in = p.ntz_in = 0;
-        add_box(0, ny, 0, nz);
-    } else {
-        add_box(0, p.j_lo, 0, nz);
-        add_box(p.j_hi, ny, 0, nz);
-        add_box(p.j_lo, p.j_hi, 0, p.k_lo);
-        add_box(p.j_lo, p.j_hi, p.k_hi, nz);
-    }
     // sources per tile of this tiling (the kernel stages at most MAX_SRC per tile)
     if (p.nty_in > 0 && p.ntz_in > 0 && pl->src_ijk.size() / 3 > (size_t)MAX_SRC) {
         std::vector<int> count((size_t)p.nty_in * p.ntz_in * p.nxc, 0);
@@ -1222,23 +1096,58 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
             if (++count[it] > MAX_SRC) return FDTD_ERR_CAPACITY;
         }
     }
+    // the edge shell: rows outside [j_lo, j_hi), then the columns outside
+    // [k_lo, k_hi) of those rows (every x plane)
+    Edge eb{};
+    auto add_box = [&](int64_t j0, int64_t j1, int64_t k0, int64_t k1) {
+        if (j1 <= j0 || k1 <= k0) return;
+        eb.j0[eb.n] = (int)j0; eb.j1[eb.n] = (int)j1; eb.k0[eb.n] = (int)k0; eb.k1[eb.n] = (int)k1;
+        const uint64_t ng = (uint64_t)(k1 - k0 + 3) / 4;
+        eb.off[eb.n + 1] = eb.off[eb.n] + (uint32_t)((uint64_t)(j1 - j0) * ng);
+        eb.rcp[eb.n] = (uint32_t)std::min<uint64_t>((((uint64_t)1 << 32) + ng - 1) / ng, 0xFFFFFFFFull);
+        eb.n++;
+    };
+    // Small grids: the edge kernels alone, over the whole grid, two stage launches a pass on
+    // many blocks where the pair kernel has a few CTAs, each a serial run of planes, and then
+    // the shell's two launches.  us a step, with / without the pair kernel: 64^3 85 / 53 and
+    // with an 8-cell CPML 154 / 75, 96^3 97 / 83 and 197 / 118, 100x200x64 147 / 112 and
+    // 243 / 159; without a shell the pair kernel wins from 128^3 on (151 / 193), with one from
+    // 160^3 (515 / 513, 200^3 850 / 924), earlier where psi rows are no 16-byte multiples.
+    const int64_t cells = (int64_t)p.nx * ny * nz;
+    const bool shell = p.j_lo > 0 || p.j_hi < ny || p.k_lo > 0 || p.k_hi < nz;
+    const bool small = pl->auto_chunk && cells <= (!shell ? 3 << 19 : p.vpsi ? 1 << 22 : 1 << 21);
+    if (small || p.nty_in == 0 || p.ntz_in == 0) {
+        p.nty_in = p.ntz_in = 0;
+        add_box(0, ny, 0, nz);
+    } else {
+        add_box(0, p.j_lo, 0, nz);
+        add_box(p.j_hi, ny, 0, nz);
+        add_box(p.j_lo, p.j_hi, 0, p.k_lo);
+        add_box(p.j_lo, p.j_hi, p.k_hi, nz);
+    }
     cudaStream_t st = as_stream(stream);
     const int64_t items = (int64_t)p.nty_in * p.ntz_in * p.nxc;
+    // Chained launches hide the gaps between a pass's kernels, and the edge kernel's blocks
+    // start beside a pair kernel that leaves room (200^3, 8-cell CPML: 869 -> 850 us a step,
+    // 128^3 356 -> 312).  Pair kernels that fill the GPU lose more to their company than the
+    // gaps cost (256^3 1373 -> 1418, 512^3 8255 -> 8640).
+    const bool chained = cells < (1 << 23);
     if (items > 0) {
         const int nb = (int)std::min<int64_t>(items, pl->slots);
         if (two_h)
-            k_symp_pair<true><<<nb, THREADS, SMEM, st>>>(pl->maps[in], p);
+            launch(chained, k_symp_pair<true>, dim3(nb), THREADS, SMEM, st, pl->maps[in], p);
         else
-            k_symp_pair<false><<<nb, THREADS, SMEM, st>>>(pl->maps[in], p);
+            launch(chained, k_symp_pair<false>, dim3(nb), THREADS, SMEM, st, pl->maps[in], p);
     }
-    const int64_t ecells = eb.off[eb.n];  // per x plane
-    if (ecells > 0) {
-        const dim3 nb((unsigned)((ecells + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx);
+    const int64_t egroups = eb.off[eb.n];  // per x plane
+    if (egroups > 0) {
+        const dim3 nb((unsigned)((egroups + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx);
+        const int32_t beside = chained && items > 0;
         if (two_h)
-            k_edge_h<true><<<nb, EDGE_BLOCK, 0, st>>>(p, eb);
+            launch(chained, k_edge_h<true>, nb, EDGE_BLOCK, 0, st, p, eb, beside);
         else
-            k_edge_h<false><<<nb, EDGE_BLOCK, 0, st>>>(p, eb);
-        k_edge_e<<<nb, EDGE_BLOCK, 0, st>>>(p, eb);
+            launch(chained, k_edge_h<false>, nb, EDGE_BLOCK, 0, st, p, eb, beside);
+        launch(chained, k_edge_e, nb, EDGE_BLOCK, 0, st, p, eb);
         bool esrc = false;
         for (size_t a = 0; a + 2 < pl->src_ijk.size(); a += 3)
             for (int b = 0; b < eb.n; b++)
