@@ -12,20 +12,22 @@
 namespace fdtd {
 namespace fused {
 
-// Single-grid band kernels: a warp per (i, j) row (grid (ceil(ny/4), nx),
-// 4 warps a block), lanes over the row's band cells -- no index division.
+// Band kernels: a thread per band cell, a plane's rows (blockIdx.y: i) one after
+// the other, so that no lane is idle.  A warp a row left 6 to 8 of 32 lanes so with
+// a 12-cell layer, and more with a thinner one; us a step without / with: 128^3 with
+// 8 cells 61.8 / 59.5, 256x256x128 159.2 / 157.5, 203x331x157 206.6 / 204.4.  What
+// bounds them is DRAM: 64 bytes at either end of every row (31 us for the H band of
+// 256x256x128, whose 115 MB a copy would move in 17).
 __global__ void __launch_bounds__(128) k_zband_e(const __grid_constant__ Params p) {
-    const int64_t j = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5), i = blockIdx.y;
+    const uint32_t nk = zband_e_row(p), u = blockIdx.x * 128 + threadIdx.x, j = u / nk;
     if (j >= p.ny) return;
-    const int nk = zband_e_row(p);
-    for (int kb = threadIdx.x & 31; kb < nk; kb += 32) zband_e_at(p, p.t, i, j, kb);
+    zband_e_at(p, p.t, blockIdx.y, j, (int)(u - j * nk));
 }
 
 __global__ void __launch_bounds__(128) k_zband_h(const __grid_constant__ Params p) {
-    const int64_t j = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5), i = blockIdx.y;
+    const uint32_t nk = zband_h_row(p), u = blockIdx.x * 128 + threadIdx.x, j = u / nk;
     if (j >= p.ny) return;
-    const int nk = zband_h_row(p);
-    for (int kb = threadIdx.x & 31; kb < nk; kb += 32) zband_h_at(p, i, j, kb);
+    zband_h_at(p, blockIdx.y, j, (int)(u - j * nk));
 }
 
 }  // namespace fused
@@ -479,11 +481,12 @@ int fdtd_yee_plan_run(fdtd_yee_plan *pl, int64_t t0, int64_t nsteps, void *strea
                        (unsigned)pl->cluster, pl->maps[in], p, bd);
         if (p.zfix) {
             for (int q = 0; q < 6; q++) p.in[q] = pl->f[in][q];
-            const dim3 rows((unsigned)((p.ny + 3) / 4), (unsigned)p.nx);
+            // (a plane's band cells number less than 2^32: the arrays would not fit otherwise)
+            auto plane = [&](int nk) { return dim3((unsigned)((p.ny * nk + 127) / 128), (unsigned)p.nx); };
             // launched the plain way: started early, their waiting blocks hold back the
             // kernel before them (256^3 253 -> 261 us a step)
-            k_zband_e<<<rows, 128, 0, st>>>(p);
-            k_zband_h<<<rows, 128, 0, st>>>(p);
+            k_zband_e<<<plane(zband_e_row(p)), 128, 0, st>>>(p);
+            k_zband_h<<<plane(zband_h_row(p)), 128, 0, st>>>(p);
         }
         FDTD_TRY(check_launch());
         if (pl->has_tfsf) FDTD_TRY(tfsf_launch_1d(&pl->tfsf, n + 1 < nsteps ? 2 : 1, t0 + n + 1, st));

@@ -1144,7 +1144,7 @@ __host__ __device__ __forceinline__ int64_t zband_h_start(const Params &p) {
 // alias a later load as far as the compiler knows, so loads placed after
 // stores would not be overlapped.
 // E band cells per (i, j) row: the front slab's nodes, then the back slab's
-__device__ __forceinline__ int zband_e_row(const Params &p) {
+__host__ __device__ __forceinline__ int zband_e_row(const Params &p) {
     return (((p.faces >> 4) & 1) ? p.P[2] : 0) + (((p.faces >> 5) & 1) ? p.P[2] : 0);
 }
 
@@ -1192,7 +1192,7 @@ __device__ __forceinline__ void zband_e_at(const Params &p, int64_t tstep, int64
 }
 
 // H band cells per (i, j) row: k = 1 .. P+1 (front), then bstart .. nz-1 (back)
-__device__ __forceinline__ int zband_h_row(const Params &p) {
+__host__ __device__ __forceinline__ int zband_h_row(const Params &p) {
     const int64_t fend = ((p.faces >> 4) & 1) ? p.P[2] + 1 : 0;
     return (int)(fend + (p.nz - zband_h_start(p)));
 }
