@@ -30,6 +30,40 @@ __global__ void __launch_bounds__(128) k_zband_h(const __grid_constant__ Params 
     zband_h_at(p, blockIdx.y, j, (int)(u - j * nk));
 }
 
+// The same over all grids of a batched plan: off[s] is the first block of grid s,
+// whose planes take as many whole blocks each.  A block copies its grid's parameters
+// into shared memory once.
+struct BandBatch {
+    int32_t nsims, cur;
+    int64_t t;
+    const Params *params;
+    const int64_t *off;
+};
+constexpr int kBandBlock = 256;
+__host__ __device__ __forceinline__ int64_t band_plane_blocks(const Params &p, int nk) {
+    return (p.ny * nk + kBandBlock - 1) / kBandBlock;
+}
+template <bool E>
+__global__ void __launch_bounds__(kBandBlock) k_zband_batch(const __grid_constant__ BandBatch d) {
+    __shared__ __align__(16) unsigned char s_p[sizeof(Params)];
+    int g = -1;  // the last grid that starts at or before this block
+    for (int b = 0; b < d.nsims; b += kBandBlock) {
+        const int s = b + (int)threadIdx.x;
+        g += __syncthreads_count(s < d.nsims && d.off[s] <= (int64_t)blockIdx.x);
+    }
+    static_assert(sizeof(Params) % 8 == 0, "copied as 8-byte words");
+    const uint64_t *src = reinterpret_cast<const uint64_t *>(d.params + 2 * g + d.cur);
+    for (int w = threadIdx.x; w < (int)(sizeof(Params) / 8); w += kBandBlock) reinterpret_cast<uint64_t *>(s_p)[w] = src[w];
+    __syncthreads();
+    const Params &p = *reinterpret_cast<const Params *>(s_p);
+    const uint32_t nk = E ? zband_e_row(p) : zband_h_row(p), nb = (uint32_t)band_plane_blocks(p, nk);
+    const uint32_t local = (uint32_t)(blockIdx.x - d.off[g]), i = local / nb;
+    const uint32_t u = (local - i * nb) * kBandBlock + threadIdx.x, j = u / nk;
+    if (j >= p.ny) return;
+    if (E) zband_e_at(p, d.t, i, j, (int)(u - j * nk));
+    else zband_h_at(p, i, j, (int)(u - j * nk));
+}
+
 }  // namespace fused
 }  // namespace fdtd
 
@@ -60,7 +94,7 @@ static EncodeTiledFn get_encode_fn() {
 struct KernelEntry {
     int ty, ns, threads, smem;  // smem: without the CPML tables
     FusedKernel fn[2][4];       // single grid: without / with the z-slab terms; bit 0: Drude, bit 1: TFSF
-    FusedKernel fn_batch[2];    // batched, without / with Drude (batched plans take no plane wave)
+    FusedKernel fn_batch[2][2]; // batched: without / with the z-slab terms, Drude (no plane wave)
 };
 
 template <int TY, int NS>
@@ -68,7 +102,8 @@ static KernelEntry entry() {
     KernelEntry e{TY, NS, Layout<TY, NS>::THREADS, Layout<TY, NS>::SMEM, {}, {}};
     single_kernels(TY, NS, e.fn[0]);
     single_kernels_z(TY, NS, e.fn[1]);
-    batch_kernels(TY, NS, e.fn_batch);
+    batch_kernels(TY, NS, e.fn_batch[0]);
+    batch_kernels_z(TY, NS, e.fn_batch[1]);
     return e;
 }
 
@@ -191,11 +226,11 @@ static int capacity_chunk(int64_t nx, int64_t tiles, int nsm) {
 }
 
 // batch_chunk > 0: a grid of a batched plan, which pools every grid's items over
-// one launch (with that chunk unless the caller gives one) and whose kernel
-// applies the z-slab terms itself
+// one launch (with that chunk unless the caller gives one); batch_bands: the
+// batched plan's band kernels finish the z slab
 static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_yee_state *s, const fdtd_cpml *c,
                            const fdtd_sources *src, const fdtd_tile *tile, int32_t *status_dev, int32_t cur,
-                           void *stream, int batch_chunk) {
+                           void *stream, int batch_chunk, bool batch_bands) {
     if (!out || !s || !status_dev) return FDTD_ERR_ARG;
     *out = nullptr;
     Grid g;
@@ -294,7 +329,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         p.th1d = t.h1d;
     }
     // the z slab (when a z face has CPML): inside the fused kernel or by the band kernels
-    p.zfix = (!batch_chunk && p.P[2] > 0 && ((p.faces >> 4) & 3) && use_bands(g)) ? 1 : 0;
+    p.zfix = (p.P[2] > 0 && ((p.faces >> 4) & 3) && (batch_chunk ? batch_bands : use_bands(g))) ? 1 : 0;
     // tile rows with y slab cells (rows j0-1 .. j0+ty-1), counted from either end
     if (p.P[1] > 0)
         for (int t = 0; t < p.nty; t++) {
@@ -449,7 +484,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
 int fdtd_yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_yee_state *s, const fdtd_cpml *c,
                          const fdtd_sources *src, const fdtd_tile *tile, int32_t *status_dev, int32_t cur,
                          void *stream) {
-    return yee_plan_create(out, gp, s, c, src, tile, status_dev, cur, stream, 0);
+    return yee_plan_create(out, gp, s, c, src, tile, status_dev, cur, stream, 0, false);
 }
 
 int fdtd_yee_plan_run(fdtd_yee_plan *pl, int64_t t0, int64_t nsteps, void *stream) {
@@ -559,7 +594,8 @@ struct fdtd_batch_plan {
     int64_t nitems;
     TMaps *d_maps;
     Params *d_params;
-    int64_t *d_off;        // work-item offsets of the fused kernel
+    int64_t *d_off;        // work-item offsets of the fused kernel, then the band kernels' block offsets (E, H)
+    int64_t band_e, band_h;  // blocks of the band kernels
     int32_t *d_queue;        // work queue of the fused kernel (2 counters)
 };
 
@@ -570,8 +606,8 @@ static size_t batch_ws_layout(int32_t nsims, size_t *off_params, size_t *off_ite
     *off_params = o;
     o += (size_t)2 * nsims * sizeof(Params);
     o = (o + 63) / 64 * 64;
-    *off_items = o;  // work-item offsets, then the queue
-    o += (size_t)(nsims + 1) * sizeof(int64_t);
+    *off_items = o;  // work-item offsets, band block offsets (E, H), then the queue
+    o += (size_t)3 * (nsims + 1) * sizeof(int64_t);
     o += 64;
     return o;
 }
@@ -595,7 +631,8 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     if (workspace_bytes < need) return FDTD_ERR_CAPACITY;
     std::vector<TMaps> maps((size_t)2 * nsims);
     std::vector<Params> params((size_t)2 * nsims);
-    std::vector<int64_t> off((size_t)nsims + 1, 0);
+    std::vector<int64_t> off((size_t)3 * (nsims + 1), 0);
+    int64_t *off_e = off.data() + (nsims + 1), *off_h = off_e + (nsims + 1);
     const KernelEntry *ke = nullptr;
     int tab_bytes = 0;
     bool any_drude = false;
@@ -625,6 +662,14 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
             }
         }
     }
+    int64_t cells = 0;
+    for (int32_t s = 0; s < nsims; s++) cells += grids[s].nx * grids[s].ny * grids[s].nz;
+    // The z slab on band kernels (three launches a step) or in the kernel, where the tiles of a
+    // z slab, half of all on grids of up to 192 cells, execute twice a plain one's instructions.
+    // us a step in the kernel / on bands: 8 grids of 24..96 cells an axis, 1.6 Mcells in all,
+    // 97 / 84; 24 of 24..64 (2.1 M) 110 / 105; 64 of 32..192 (80 M) 2022 / 1617; but 8 of 24..64
+    // (0.8 M) 45 / 50 and 4 of 64^3 (1.0 M) 45 / 51, where the launches count
+    const bool bands = cells >= 3 << 19;
     // grids with the longest items (x planes per chunk, then tile rows) come first
     std::vector<int32_t> order((size_t)nsims);
     for (int32_t s = 0; s < nsims; s++) order[s] = s;
@@ -638,7 +683,8 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
         const int32_t u = order[s];
         fdtd_yee_plan *pl = nullptr;
         const int st = yee_plan_create(&pl, &grids[u], &states[u], cpmls ? &cpmls[u] : nullptr,
-                                       srcs ? &srcs[u] : nullptr, tile, status_dev, cur, stream, std::max(chunk, 1));
+                                       srcs ? &srcs[u] : nullptr, tile, status_dev, cur, stream, std::max(chunk, 1),
+                                       bands);
         if (st != FDTD_OK) return st;
         ke = pl->k;
         any_drude = any_drude || pl->base.drude;
@@ -659,6 +705,9 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
             maps[2 * s + b] = pl->maps[b];
         }
         off[s + 1] = off[s] + pl->nitems;
+        const Params &p = pl->base;
+        off_e[s + 1] = off_e[s] + (p.zfix ? p.nx * band_plane_blocks(p, zband_e_row(p)) : 0);
+        off_h[s + 1] = off_h[s] + (p.zfix ? p.nx * band_plane_blocks(p, zband_h_row(p)) : 0);
         fdtd_yee_plan_destroy(pl);
     }
     // fill the workspace on the caller's stream (ordered after that stream's
@@ -685,7 +734,9 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     bp->d_params = reinterpret_cast<Params *>(ws + off_p);
     bp->d_off = reinterpret_cast<int64_t *>(ws + off_i);
     bp->d_queue = reinterpret_cast<int32_t *>(ws + off_i + off.size() * sizeof(int64_t));
-    bp->fn = ke->fn_batch[any_drude ? 1 : 0];
+    bp->band_e = off_e[nsims];
+    bp->band_h = off_h[nsims];
+    bp->fn = ke->fn_batch[bands ? 0 : 1][any_drude ? 1 : 0];
     int nsm = 0, occ = 0;
     const int rs = fused_residency(bp->fn, ke->threads, bp->smem, &nsm, &occ);
     if (rs != FDTD_OK) { delete bp; return rs; }
@@ -713,6 +764,12 @@ int fdtd_batch_plan_run(fdtd_batch_plan *bp, int64_t t0, int64_t nsteps, void *s
         bd.queue = bp->d_queue;
         launch_chained(bp->fn, dim3((unsigned)bp->nblocks), dim3((unsigned)bp->k->threads), (size_t)bp->smem, st, 1,
                        dummy_maps, dummy, bd);
+        if (bp->band_h > 0) {
+            BandBatch d{bp->nsims, bp->cur, t0 + n, bp->d_params, bp->d_off + (bp->nsims + 1)};
+            k_zband_batch<true><<<(unsigned)bp->band_e, kBandBlock, 0, st>>>(d);
+            d.off += bp->nsims + 1;
+            k_zband_batch<false><<<(unsigned)bp->band_h, kBandBlock, 0, st>>>(d);
+        }
         FDTD_TRY(check_launch());
         bp->cur = 1 - bp->cur;
     }

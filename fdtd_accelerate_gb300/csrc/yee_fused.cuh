@@ -1287,11 +1287,12 @@ typedef void (*FusedKernel)(const TMaps, const Params, const BatchDesc);
 
 // Instantiations compiled in separate translation units (the build compiles
 // them in parallel): single-grid kernels without (EXT 0..3) and with (EXT 4..7)
-// the z-slab terms, batched kernels (EXT 4, 5).  false when (ty, ns) is not
-// compiled in.
+// the z-slab terms, batched kernels without (EXT 0, 1) and with them (EXT 4, 5).
+// false when (ty, ns) is not compiled in.
 bool single_kernels(int ty, int ns, FusedKernel out[4]);
 bool single_kernels_z(int ty, int ns, FusedKernel out[4]);
 bool batch_kernels(int ty, int ns, FusedKernel out[2]);
+bool batch_kernels_z(int ty, int ns, FusedKernel out[2]);
 
 }  // namespace fused
 }  // namespace fdtd

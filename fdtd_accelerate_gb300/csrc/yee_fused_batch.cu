@@ -1,4 +1,4 @@
-// Batched instantiations of the fused kernel (many grids per launch).
+// Batched instantiations of the fused kernel (many grids per launch), without the z-slab terms.
 #include "yee_fused.cuh"
 
 namespace fdtd {
@@ -7,8 +7,8 @@ namespace fused {
 bool batch_kernels(int ty, int ns, FusedKernel out[2]) {
 #define FDTD_CASE(TY, NS)                                  \
     if (ty == TY && ns == NS) {                            \
-        out[0] = k_yee_fused<TY, NS, true, 4>;          \
-        out[1] = k_yee_fused<TY, NS, true, 5>;          \
+        out[0] = k_yee_fused<TY, NS, true, 0>;             \
+        out[1] = k_yee_fused<TY, NS, true, 1>;             \
         return true;                                       \
     }
     FDTD_FUSED_TILES(FDTD_CASE)
