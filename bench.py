@@ -53,12 +53,11 @@ NPML = 12
 # from MEASURED_PEAKS.json when present.
 FALLBACK_HBM_GBS = 6790.7
 # DRAM traffic of one time step (dram__bytes_read.sum + dram__bytes_write.sum),
-# from an ncu capture of the same workload scaled to 512x512x256 (three steps,
-# the per-launch values agree to 0.2 %), scaled to another size by the units
+# from an ncu capture of the same workload scaled to 512x512x256, scaled to another size by the units
 # each kernel processes: the fused kernel's bytes per grid cell, and the two
 # z-band kernels' bytes per band cell (nx * ny * 2P z-slab E nodes).
-NCU_FUSED_DRAM_BYTES_PER_CELL = 63.48
-NCU_BAND_DRAM_BYTES_PER_BAND_CELL = 193.0
+NCU_FUSED_DRAM_BYTES_PER_CELL = 63.2
+NCU_BAND_DRAM_BYTES_PER_BAND_CELL = 192.9
 # The plain 128^3 step (one fused launch, no CPML): DRAM bytes of one launch
 # after an L2 flush, from an ncu capture of that workload (three launches,
 # within 2 %); part of the 50 MB of field writes is still in L2 when the

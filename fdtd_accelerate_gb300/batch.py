@@ -1,15 +1,16 @@
-"""Many independent Yee grids advanced by one launch per step.
+"""Many independent Yee grids advanced together, one to three launches per step.
 
 The reference runs one simulation per process and time loop (e.g.
 2nd_order-Yee/CUDA/fdtd3d_201_250x250x320cell_15npml_100000tstep.cu:718-742).
 BatchSolver keeps a list of YeeSolver grids of any (uneven) sizes and
 advances all of them with the batched fused kernel: the work items of every
-grid (z tile x y tile x x chunk) form one list that the persistent CTAs walk,
+grid (z tile x y tile x x chunk) form one list that the persistent CTAs walk (from
+1.5 Mcells on, two more launches finish the z CPML slabs of all grids),
 so small grids that would leave most SMs idle on their own fill the GPU
 together.  Each grid's result is bit-identical to its own YeeSolver.step.
 
 A run of n steps can be captured into one CUDA graph (``run_graph``) so the
-n launches go to the GPU as a single submission; the launch shape comes from
+launches go to the GPU as a single submission; the launch shape comes from
 ``autotune`` (timed candidates, cached in a JSON file).
 """
 import ctypes as C
@@ -108,7 +109,7 @@ class BatchSolver:
                 s.cur = 1 - s.cur
 
     def step(self, n=1):
-        """Advance every grid n steps (n launches on the current stream)."""
+        """Advance every grid n steps (launches on the current stream)."""
         plan = self.plan()
         L = N.lib()
         L.fdtd_batch_plan_set_current(plan, self.cur)

@@ -155,7 +155,7 @@ class YeeSolver:
                          "launches_per_step"), list(info)))
 
     def step(self, n=1):
-        """Advance n steps with the fused kernel (one launch per step)."""
+        """Advance n steps with the fused kernel (plan_info: launches per step)."""
         if self.tfsf is not None:
             # the plan holds the source table's address: a longer table needs a new plan
             old = self.tfsf.amp.data_ptr()

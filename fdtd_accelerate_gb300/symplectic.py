@@ -186,9 +186,10 @@ class SymplecticSolver:
     amplitude) with amplitude a callable of continuous time t (FP64), added
     after every E stage at t = tn + sn/5 (PyCUDA/100-base.py:136).
     fused: take the stage-pair path (one pass per H + E stage pair: the pair
-    kernel inside, the edge kernels on the y/z CPML shell) where pair_path()
-    allows; bit-identical to the per-stage kernels and faster than them
-    (8.25 against 12.3 ms per step on the 512^3 workload); fused=False keeps
+    kernel inside, the edge kernels on the y/z CPML shell, small grids by the
+    edge kernels alone) where pair_path() allows; bit-identical to the
+    per-stage kernels and faster than them (8.01 against 12.5 ms per step on
+    the 512^3 workload, 75 against 98 us at 64^3); fused=False keeps
     the one-launch-per-stage path.  x_chunk: x planes per work item of the
     pair kernel (0: chosen per tiling by the plan).
     """
@@ -283,7 +284,11 @@ class SymplecticSolver:
             return self._pair
         self.close()
         if self._buf[1] is None:
-            self._buf[1] = self._rows(6)
+            # a pass writes every cell of it, so only the rows' padding is cleared
+            nx, ny, nz = self.shape
+            whole = torch.empty((6, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)
+            whole[..., nz:].zero_()
+            self._buf[1] = whole[..., :nz]
         hb = self.cpml.second_h_buffer()
         st = N.SympState()
         for b in range(2):

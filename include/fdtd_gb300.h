@@ -323,7 +323,9 @@ int fdtd_symp_pair_plan_current(const fdtd_symp_plan *plan);
 int fdtd_symp_pair_plan_set_current(fdtd_symp_plan *plan, int32_t cur);
 int fdtd_symp_pair_plan_destroy(fdtd_symp_plan *plan);
 
-/* ---- batched fused step: many independent grids, one launch per step --- */
+/* ---- batched fused step: many independent grids a launch --------------- */
+/* One launch per step; from 1.5 Mcells on, and with a z face's CPML, two band
+ * launches over all grids finish the z slabs. */
 /* Every grid keeps its own state, CPML and sources (arrays as for
  * fdtd_yee_plan_create); all grids advance together (same buffer index,
  * same step number).  The per-grid launch parameters and TMA descriptors
