@@ -461,7 +461,7 @@ __device__ __forceinline__ void tfsf_term(const Params &p, int eh, int face, int
 // The terms of one group (m: its masks) on plane i, E (eh = 0) or H (eh = 1).  A family
 // at a time, 4 cells each: one cell at a time, with the family's face and table looked up
 // for each, a plane of a tile with a y face row took 3 times as long (256^3, 12-cell
-// CPML, all faces of a 128^3 box: 404 us a step, now 340; the same step without a wave 247).
+// CPML, all faces of a 128^3 box: 404 us a step, 340 with this form; without a wave 247).
 __device__ __forceinline__ void tfsf_group(const Params &p, int eh, uint32_t m, int i, int j, int k, V4 &vx, V4 &vy,
                                            V4 &vz) {
     const int32_t i1 = p.tp1[0], i2 = p.tp2[0];
