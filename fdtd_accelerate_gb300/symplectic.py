@@ -210,9 +210,10 @@ class SymplecticSolver:
         self._pair_src = None
         if ce is None:
             ce = [np.full(self.shape, S / 24.0)] * 3
-        self.ce = self._as_rows(ce)
+        self.ce = self._as_f32(ce)
         self.ch = float(S / 24.0) if ch is None else (
-            float(ch) if isinstance(ch, (int, float)) else self._as_rows(ch))
+            float(ch) if isinstance(ch, (int, float)) else self._as_f32(ch))
+        self._coef_rows = {}
         self.cpml = SymplecticCpml(self.shape, npml, faces, S, device=dev, **(cpml_params or {}))
         self.src_spec = list(sources)
         self.max_steps = max_steps
@@ -228,14 +229,25 @@ class SymplecticSolver:
         nx, ny, nz = self.shape
         return torch.zeros((n, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)[..., :nz]
 
-    def _as_rows(self, arrays):
-        """Three coefficient arrays in the fields' layout."""
+    def _as_f32(self, arrays):
+        """Three coefficient arrays on the device: a contiguous float32 tensor of
+        the caller's is used in place, so that edits of it reach the next call."""
+        return [torch.as_tensor(c, dtype=torch.float32, device=self.device).contiguous() for c in arrays]
+
+    def _coefs(self, name):
+        """ce or ch in the fields' layout: the arrays themselves, or their present
+        values on the rows' 16-byte pitch (copied at each call: the caller may have
+        edited the arrays)."""
+        arrays = getattr(self, name)
         if self.shape[2] % 4 == 0:
-            return [torch.as_tensor(c, dtype=torch.float32, device=self.device).contiguous() for c in arrays]
-        out = list(self._rows(3).unbind(0))
-        for dst, c in zip(out, arrays):
-            dst.copy_(torch.as_tensor(c, dtype=torch.float32, device=self.device))
-        return out
+            return arrays
+        if name not in self._coef_rows:
+            self._coef_rows[name] = self._rows(3)
+        nx, ny, nz = self.shape
+        with torch.no_grad():
+            for dst, c in zip(self._coef_rows[name], arrays):
+                dst.copy_(c.reshape(-1)[:nx * ny * nz].view(self.shape))
+        return list(self._coef_rows[name])
 
     def _build_sources(self, nsteps):
         tabs = []
@@ -279,7 +291,7 @@ class SymplecticSolver:
         k1 = (nz - pz - 2) // 16 * 16 if pz and f & 32 else nz
         return max(0, j1 - j0) * max(0, k1 - k0) / (ny * nz)
 
-    def _pair_plan(self):
+    def _pair_plan(self, ce):
         if self._pair is not None and self._pair_src is self._src:
             return self._pair
         self.close()
@@ -299,7 +311,7 @@ class SymplecticSolver:
             e = self.cpml.psi_e[q]
             st.psi_e[q] = e.data_ptr() if e is not None else None
         for q in range(3):
-            st.ce[q] = self.ce[q].data_ptr()
+            st.ce[q] = ce[q].data_ptr()
         if not hasattr(self, "_status"):
             self._status = torch.zeros(1, dtype=torch.int32, device=self.device)
         if not hasattr(self, "_queue"):
@@ -349,7 +361,8 @@ class SymplecticSolver:
             return self.step_stages(n)
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)
-        plan = self._pair_plan()
+        ce = self._coefs("ce")
+        plan = self._pair_plan(ce)
         L = N.lib()
         L.fdtd_symp_pair_plan_set_current(plan, self._cur)
         cp = self.cpml
@@ -397,11 +410,11 @@ class SymplecticSolver:
     def _make_stage_args(self):
         g = grid_of(self.f[0])
         fptr = (C.c_void_p * 6)(*(t.data_ptr() for t in self.f))
-        ceptr = (C.c_void_p * 3)(*(t.data_ptr() for t in self.ce))
+        ceptr = (C.c_void_p * 3)(*(t.data_ptr() for t in self._coefs("ce")))
         if isinstance(self.ch, float):
             chptr, chv = None, self.ch
         else:
-            chptr, chv = (C.c_void_p * 3)(*(t.data_ptr() for t in self.ch)), 0.0
+            chptr, chv = (C.c_void_p * 3)(*(t.data_ptr() for t in self._coefs("ch"))), 0.0
         return g, fptr, ceptr, chptr, chv
 
     def _fused_stage(self, e_or_h, coef, cptr, chv, stream):
@@ -417,7 +430,7 @@ class SymplecticSolver:
         """The same steps through the reference-shaped calls: update_h /
         update_e per stage, then the per-axis CPML corrections."""
         nx, ny, nz = self.shape
-        f, ce, ch = self.f, self.ce, self.ch
+        f, ce = self.f, self._coefs("ce")
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)
         with torch.cuda.device(self.device):
@@ -436,7 +449,7 @@ class SymplecticSolver:
 
     def _h_stage(self, cl, stream):
         nx, ny, nz = self.shape
-        f, ch = self.f, self.ch
+        f, ch = self.f, self.ch if isinstance(self.ch, float) else self._coefs("ch")
         if isinstance(ch, float):
             update_h(nx, ny, nz, cl, *f, ch)
         else:

@@ -1,0 +1,47 @@
+"""What a caller of SymplecticSolver holds on rows that are no multiple of 4
+floats is what it holds on aligned ones."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("ex", "ey", "ez", "hx", "hy", "hz")
+
+
+def solver(shape, ce, **kw):
+    from fdtd_accelerate_gb300.symplectic import SymplecticSolver
+    rng = np.random.default_rng(3)
+    s = SymplecticSolver(shape, ce=ce, sources=[("ez", tuple(n // 2 for n in shape), lambda t: 0.1 * t)],
+                         max_steps=64, **kw)
+    s.set_fields(**{k: (0.1 * rng.standard_normal(shape)).astype(np.float32) for k in NAMES})
+    return s
+
+
+def coefs(shape, seed=4):
+    rng = np.random.default_rng(seed)
+    return [torch.from_numpy((0.743 / 24 / rng.uniform(1.0, 4.0, shape)).astype(np.float32)).cuda() for _ in range(3)]
+
+
+def assert_same(a, b):
+    torch.cuda.synchronize()
+    for k in NAMES:
+        assert torch.equal(a.fields[k], b.fields[k]), k
+
+
+@pytest.mark.parametrize("how", ["step", "step_stages", "step_unfused"])
+@pytest.mark.parametrize("nz", [44, 45])
+def test_edited_coefficients_reach_the_next_call(nz, how):
+    shape = (20, 40, nz)
+    ce = coefs(shape)
+    s = solver(shape, ce, ch=[0.75 * c for c in coefs(shape, 5)] if how != "step" else None)
+    getattr(s, how)(32)
+    for c in ce:
+        c.mul_(0.5)
+    before = {k: v.clone() for k, v in s.fields.items()}
+    getattr(s, how)(32)
+    r = solver(shape, [c.clone() for c in ce], ch=s.ch)
+    r.set_fields(**before)
+    r.tstep = 33
+    getattr(r, how)(32)
+    assert_same(s, r)
