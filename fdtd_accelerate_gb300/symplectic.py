@@ -201,8 +201,11 @@ class SymplecticSolver:
         dev = self.device
         self.S = S
         # state buffers: buf[cur] holds the fields; the stage-pair path writes
-        # buf[1 - cur] from buf[cur] (the second buffer is allocated on first use)
-        self._buf = [self._rows(6), None]
+        # buf[1 - cur] from buf[cur] (the second buffer is allocated on first use).
+        # Where rows are no multiple of 4 floats it runs on copies with 16-byte
+        # rows (_pitched) and the fields stay in buf[0].
+        self._buf = [torch.zeros((6,) + self.shape, dtype=torch.float32, device=dev), None]
+        self._pitched = None
         self._cur = 0
         self.fused = fused
         self.x_chunk = int(x_chunk)
@@ -213,7 +216,6 @@ class SymplecticSolver:
         self.ce = self._as_f32(ce)
         self.ch = float(S / 24.0) if ch is None else (
             float(ch) if isinstance(ch, (int, float)) else self._as_f32(ch))
-        self._coef_rows = {}
         self.cpml = SymplecticCpml(self.shape, npml, faces, S, device=dev, **(cpml_params or {}))
         self.src_spec = list(sources)
         self.max_steps = max_steps
@@ -222,32 +224,25 @@ class SymplecticSolver:
         self._stage_args = None
         self._build_sources(max(max_steps, 1))
 
-    def _rows(self, n):
-        """n zeroed arrays of the grid's shape whose rows start on 16-byte
-        boundaries (the pitch is nz rounded up to 4 floats), as the TMA copies
-        of the stage-pair path need them."""
-        nx, ny, nz = self.shape
-        return torch.zeros((n, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)[..., :nz]
-
     def _as_f32(self, arrays):
         """Three coefficient arrays on the device: a contiguous float32 tensor of
         the caller's is used in place, so that edits of it reach the next call."""
         return [torch.as_tensor(c, dtype=torch.float32, device=self.device).contiguous() for c in arrays]
 
-    def _coefs(self, name):
-        """ce or ch in the fields' layout: the arrays themselves, or their present
-        values on the rows' 16-byte pitch (copied at each call: the caller may have
-        edited the arrays)."""
-        arrays = getattr(self, name)
-        if self.shape[2] % 4 == 0:
-            return arrays
-        if name not in self._coef_rows:
-            self._coef_rows[name] = self._rows(3)
+    def _pair_arrays(self):
+        """The two state buffers and the ce arrays that the stage-pair path runs
+        on: the solver's own, or copies on rows of 16 bytes (as the TMA copies
+        need them; the pitch is nz rounded up to 4 floats)."""
         nx, ny, nz = self.shape
-        with torch.no_grad():
-            for dst, c in zip(self._coef_rows[name], arrays):
-                dst.copy_(c.reshape(-1)[:nx * ny * nz].view(self.shape))
-        return list(self._coef_rows[name])
+        if nz % 4 == 0:
+            if self._buf[1] is None:
+                self._buf[1] = torch.empty_like(self._buf[0])  # a pass writes every cell of it
+            return self._buf, self.ce
+        if self._pitched is None:
+            # the rows' padding is neither read nor written
+            self._pitched = [torch.empty((n, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)[..., :nz]
+                             for n in (6, 6, 3)]
+        return self._pitched[:2], self._pitched[2]
 
     def _build_sources(self, nsteps):
         tabs = []
@@ -263,7 +258,7 @@ class SymplecticSolver:
     @property
     def f(self):
         """ex, ey, ez, hx, hy, hz of the current state buffer."""
-        return list(self._buf[self._cur])
+        return list(self._buf[0 if self.shape[2] % 4 else self._cur])
 
     @property
     def fields(self):
@@ -291,21 +286,15 @@ class SymplecticSolver:
         k1 = (nz - pz - 2) // 16 * 16 if pz and f & 32 else nz
         return max(0, j1 - j0) * max(0, k1 - k0) / (ny * nz)
 
-    def _pair_plan(self, ce):
+    def _pair_plan(self, buf, ce):
         if self._pair is not None and self._pair_src is self._src:
             return self._pair
         self.close()
-        if self._buf[1] is None:
-            # a pass writes every cell of it, so only the rows' padding is cleared
-            nx, ny, nz = self.shape
-            whole = torch.empty((6, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)
-            whole[..., nz:].zero_()
-            self._buf[1] = whole[..., :nz]
         hb = self.cpml.second_h_buffer()
         st = N.SympState()
         for b in range(2):
             for q in range(6):
-                st.f[b][q] = self._buf[b][q].data_ptr()
+                st.f[b][q] = buf[b][q].data_ptr()
                 st.psi_h[b][q] = hb[b][q].data_ptr() if hb[b][q] is not None else None
         for q in range(6):
             e = self.cpml.psi_e[q]
@@ -319,7 +308,7 @@ class SymplecticSolver:
         h = C.c_void_p()
         src = self._src.struct()
         with torch.cuda.device(self.device):
-            N.call("fdtd_symp_pair_plan_create", C.byref(h), C.byref(grid_of(self._buf[0][0])), C.byref(st),
+            N.call("fdtd_symp_pair_plan_create", C.byref(h), C.byref(grid_of(buf[0][0])), C.byref(st),
                    C.byref(src), int(self.x_chunk), int(self._cur), C.c_void_p(self._status.data_ptr()),
                    C.c_void_p(self._queue.data_ptr()), stream_of(self._buf[0][0]))
         self._pair, self._pair_src = h, self._src
@@ -361,8 +350,13 @@ class SymplecticSolver:
             return self.step_stages(n)
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)
-        ce = self._coefs("ce")
-        plan = self._pair_plan(ce)
+        buf, ce = self._pair_arrays()
+        plan = self._pair_plan(buf, ce)
+        if self.shape[2] % 4:  # the present values: the caller may have edited any of them
+            with torch.no_grad():
+                buf[self._cur].copy_(self._buf[0])
+                for dst, c in zip(ce, self.ce):
+                    dst.copy_(c.reshape(-1)[:dst.numel()].view(self.shape))
         L = N.lib()
         L.fdtd_symp_pair_plan_set_current(plan, self._cur)
         cp = self.cpml
@@ -379,6 +373,9 @@ class SymplecticSolver:
                            float(CL[sn]), two, float(DL[sn]), ch, 4 * tn + sn if self.src_spec else -1, stream)
                     self._cur = 1 - self._cur
                     cp.set_hcur(self._cur)
+            if self.shape[2] % 4:
+                with torch.no_grad():
+                    self._buf[0].copy_(buf[self._cur])
             self._stage_args = None
             self._fused_stage(0, CL[4], None, ch, stream)
         self.tstep += n
@@ -389,7 +386,7 @@ class SymplecticSolver:
         stage.  Fields of 2^31 or more elements (the stage kernel's offsets are
         32-bit) take the per-call path of step_unfused."""
         f = self.f
-        if f[0].shape[0] * f[0].stride(0) >= 2 ** 31:
+        if f[0].numel() >= 2 ** 31:
             return self.step_unfused(n)
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)
@@ -410,11 +407,11 @@ class SymplecticSolver:
     def _make_stage_args(self):
         g = grid_of(self.f[0])
         fptr = (C.c_void_p * 6)(*(t.data_ptr() for t in self.f))
-        ceptr = (C.c_void_p * 3)(*(t.data_ptr() for t in self._coefs("ce")))
+        ceptr = (C.c_void_p * 3)(*(t.data_ptr() for t in self.ce))
         if isinstance(self.ch, float):
             chptr, chv = None, self.ch
         else:
-            chptr, chv = (C.c_void_p * 3)(*(t.data_ptr() for t in self._coefs("ch"))), 0.0
+            chptr, chv = (C.c_void_p * 3)(*(t.data_ptr() for t in self.ch)), 0.0
         return g, fptr, ceptr, chptr, chv
 
     def _fused_stage(self, e_or_h, coef, cptr, chv, stream):
@@ -430,7 +427,7 @@ class SymplecticSolver:
         """The same steps through the reference-shaped calls: update_h /
         update_e per stage, then the per-axis CPML corrections."""
         nx, ny, nz = self.shape
-        f, ce = self.f, self._coefs("ce")
+        f, ce = self.f, self.ce
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)
         with torch.cuda.device(self.device):
@@ -449,7 +446,7 @@ class SymplecticSolver:
 
     def _h_stage(self, cl, stream):
         nx, ny, nz = self.shape
-        f, ch = self.f, self.ch if isinstance(self.ch, float) else self._coefs("ch")
+        f, ch = self.f, self.ch
         if isinstance(ch, float):
             update_h(nx, ny, nz, cl, *f, ch)
         else:

@@ -45,3 +45,26 @@ def test_edited_coefficients_reach_the_next_call(nz, how):
     r.tstep = 33
     getattr(r, how)(32)
     assert_same(s, r)
+
+
+@pytest.mark.parametrize("nz", [44, 45])
+def test_fields_are_dense(nz):
+    """The fields of any grid are contiguous arrays, which the per-call functions
+    take together with arrays of the caller's."""
+    from fdtd_accelerate_gb300 import symplectic as S
+    shape = (20, 40, nz)
+    ce = coefs(shape)
+    s = solver(shape, ce)
+    held = s.fields
+    s.step(32)
+    for k in NAMES:
+        assert s.fields[k].is_contiguous() and s.fields[k].data_ptr() == held[k].data_ptr()
+        s.fields[k].view(-1)[0] += 1.0
+    e = [torch.zeros(shape, device="cuda") for _ in range(3)]
+    h = s.f[3:]
+    S.update_e(*shape, S.DL[0], *e, *h, *ce)
+    r = [torch.zeros(shape, device="cuda") for _ in range(3)]
+    S.update_e(*shape, S.DL[0], *r, *[x.clone() for x in h], *ce)
+    torch.cuda.synchronize()
+    for a, b in zip(e, r):
+        assert torch.equal(a, b)
