@@ -276,6 +276,16 @@ class SymplecticSolver:
         return (self.fused and isinstance(self.ch, float) and min(self.shape) >= 4
                 and nx * ny * padded_nz(nz) < 2 ** 31 and (nz % 4 == 0 or self._inside() >= 0.65))
 
+    def _runs_pairs(self, n):
+        """Whether step(n) takes the stage pairs: where pair_path() allows and, on
+        copies of the state, nothing that the stage kernels take is refused."""
+        if not self.pair_path():
+            return False
+        if self.shape[2] % 4 == 0:
+            return True
+        # the pair kernel stages 64 sources a tile at most: no layout of so few exceeds that
+        return len(self.src_spec) <= 64
+
     def _inside(self):
         """Share of the grid that the pair kernel advances: rows P+2 and more
         from a y face, columns from a z face likewise, in steps of 16."""
@@ -346,7 +356,7 @@ class SymplecticSolver:
         step_stages()."""
         if n <= 0:
             return
-        if not self.pair_path():
+        if not self._runs_pairs(n):
             return self.step_stages(n)
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)

@@ -9,11 +9,11 @@ pytestmark = pytest.mark.gpu
 NAMES = ("ex", "ey", "ez", "hx", "hy", "hz")
 
 
-def solver(shape, ce, **kw):
+def solver(shape, ce, sources=None, max_steps=300, **kw):
     from fdtd_accelerate_gb300.symplectic import SymplecticSolver
     rng = np.random.default_rng(3)
-    s = SymplecticSolver(shape, ce=ce, sources=[("ez", tuple(n // 2 for n in shape), lambda t: 0.1 * t)],
-                         max_steps=64, **kw)
+    s = SymplecticSolver(shape, ce=ce, max_steps=max_steps,
+                         sources=sources or [("ez", tuple(n // 2 for n in shape), lambda t: 1e-3 * t)], **kw)
     s.set_fields(**{k: (0.1 * rng.standard_normal(shape)).astype(np.float32) for k in NAMES})
     return s
 
@@ -35,15 +35,15 @@ def test_edited_coefficients_reach_the_next_call(nz, how):
     shape = (20, 40, nz)
     ce = coefs(shape)
     s = solver(shape, ce, ch=[0.75 * c for c in coefs(shape, 5)] if how != "step" else None)
-    getattr(s, how)(32)
+    getattr(s, how)(128)
     for c in ce:
         c.mul_(0.5)
     before = {k: v.clone() for k, v in s.fields.items()}
-    getattr(s, how)(32)
+    getattr(s, how)(128)
     r = solver(shape, [c.clone() for c in ce], ch=s.ch)
     r.set_fields(**before)
-    r.tstep = 33
-    getattr(r, how)(32)
+    r.tstep = 129
+    getattr(r, how)(128)
     assert_same(s, r)
 
 
@@ -56,7 +56,7 @@ def test_fields_are_dense(nz):
     ce = coefs(shape)
     s = solver(shape, ce)
     held = s.fields
-    s.step(32)
+    s.step(128)
     for k in NAMES:
         assert s.fields[k].is_contiguous() and s.fields[k].data_ptr() == held[k].data_ptr()
         s.fields[k].view(-1)[0] += 1.0
@@ -68,3 +68,15 @@ def test_fields_are_dense(nz):
     torch.cuda.synchronize()
     for a, b in zip(e, r):
         assert torch.equal(a, b)
+
+
+def test_many_sources_in_one_tile():
+    """More sources than the pair kernel stages for a tile: the stage kernels take
+    any number of them."""
+    shape = (20, 40, 45)
+    src = [(c, (i, j, 6), lambda t, q=q: 1e-3 * q * t)
+           for q, (c, i, j) in enumerate((c, i, j) for c in ("ex", "ez") for i in range(2, 18) for j in (3, 5, 7))]
+    a, b = (solver(shape, coefs(shape), sources=src, fused=fused) for fused in (True, False))
+    for s in (a, b):
+        s.step(128)
+    assert_same(a, b)
