@@ -284,7 +284,14 @@ class SymplecticSolver:
         if self.shape[2] % 4 == 0:
             return True
         # the pair kernel stages 64 sources a tile at most: no layout of so few exceeds that
-        return len(self.src_spec) <= 64
+        if len(self.src_spec) > 64:
+            return False
+        # a plan waits for its stream when it is made, which a capture forbids
+        with torch.cuda.device(self.device):
+            return self._plan_ready() or not torch.cuda.is_current_stream_capturing()
+
+    def _plan_ready(self):
+        return self._pair is not None and self._pair_src is self._src
 
     def _inside(self):
         """Share of the grid that the pair kernel advances: rows P+2 and more
@@ -297,7 +304,7 @@ class SymplecticSolver:
         return max(0, j1 - j0) * max(0, k1 - k0) / (ny * nz)
 
     def _pair_plan(self, buf, ce):
-        if self._pair is not None and self._pair_src is self._src:
+        if self._plan_ready():
             return self._pair
         self.close()
         hb = self.cpml.second_h_buffer()

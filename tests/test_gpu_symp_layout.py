@@ -80,3 +80,21 @@ def test_many_sources_in_one_tile():
     for s in (a, b):
         s.step(128)
     assert_same(a, b)
+
+
+@pytest.mark.parametrize("first", [True, False])
+def test_step_under_capture(first):
+    """step() of odd rows in a CUDA graph, as the solver's first call (the stage
+    kernels) and after one that made the pair plan."""
+    shape = (20, 40, 45)
+    a, b = (solver(shape, coefs(shape)) for _ in range(2))
+    for s in (a, b):
+        if not first:
+            s.step(128)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        a.step(128)
+    assert a._plan_ready() != first
+    graph.replay()
+    b.step(128)
+    assert_same(a, b)
