@@ -203,7 +203,7 @@ class SymplecticSolver:
         # state buffers: buf[cur] holds the fields; the stage-pair path writes
         # buf[1 - cur] from buf[cur] (the second buffer is allocated on first use).
         # Where rows are no multiple of 4 floats it runs on copies with 16-byte
-        # rows (_pitched) and the fields stay in buf[0].
+        # rows (_pitched; False: no memory for them) and the fields stay in buf[0].
         self._buf = [torch.zeros((6,) + self.shape, dtype=torch.float32, device=dev), None]
         self._pitched = None
         self._cur = 0
@@ -239,9 +239,14 @@ class SymplecticSolver:
                 self._buf[1] = torch.empty_like(self._buf[0])  # a pass writes every cell of it
             return self._buf, self.ce
         if self._pitched is None:
-            # the rows' padding is neither read nor written
-            self._pitched = [torch.empty((n, nx, ny, padded_nz(nz)), dtype=torch.float32, device=self.device)[..., :nz]
-                             for n in (6, 6, 3)]
+            try:
+                self.cpml.second_h_buffer()
+                # the rows' padding is neither read nor written
+                self._pitched = [torch.empty((n, nx, ny, padded_nz(nz)), dtype=torch.float32,
+                                             device=self.device)[..., :nz] for n in (6, 6, 3)]
+            except torch.cuda.OutOfMemoryError:
+                self._pitched = False
+                return None, None
         return self._pitched[:2], self._pitched[2]
 
     def _build_sources(self, nsteps):
@@ -288,7 +293,9 @@ class SymplecticSolver:
             return False
         # a plan waits for its stream when it is made, which a capture forbids
         with torch.cuda.device(self.device):
-            return self._plan_ready() or not torch.cuda.is_current_stream_capturing()
+            if not self._plan_ready() and torch.cuda.is_current_stream_capturing():
+                return False
+        return self._pitched is not False
 
     def _plan_ready(self):
         return self._pair is not None and self._pair_src is self._src
@@ -368,6 +375,8 @@ class SymplecticSolver:
         if self.src_spec and self.tstep + n > self._src_steps:
             self._build_sources(self.tstep + n)
         buf, ce = self._pair_arrays()
+        if buf is None:  # no memory for the copies: the stage kernels work in place
+            return self.step_stages(n)
         plan = self._pair_plan(buf, ce)
         if self.shape[2] % 4:  # the present values: the caller may have edited any of them
             with torch.no_grad():

@@ -98,3 +98,21 @@ def test_step_under_capture(first):
     graph.replay()
     b.step(128)
     assert_same(a, b)
+
+
+def test_no_memory_for_the_copies():
+    """A grid whose state fits the device and whose second state does not."""
+    shape = (64, 100, 101)
+    a, b = (solver(shape, coefs(shape), npml=(4, 0, 0), fused=fused) for fused in (True, False))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (8 << 20)) / total)
+    try:
+        a.step(128)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    b.step(128)
+    assert_same(a, b)
+    for q in range(2):
+        assert torch.equal(a.cpml.psi_e[q], b.cpml.psi_e[q]) and torch.equal(a.cpml.psi_h[q], b.cpml.psi_h[q])
