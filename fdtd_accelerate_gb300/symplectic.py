@@ -270,24 +270,45 @@ class SymplecticSolver:
         return dict(zip(("ex", "ey", "ez", "hx", "hy", "hz"), self.f))
 
     def pair_path(self):
-        """True when step() runs the fused stage pairs: uniform ch, fewer than
-        2^31 elements (with the rows' padding), every extent at least 4, and
-        on rows that are no multiple of 4 floats at least 65 % of the grid
-        clear of the y/z CPML shell (below that the stage kernels are faster:
-        80x80x81 with 8 cells, 45 % clear, 568 us for 4 steps against 778;
-        150x171x163, 69 %, 607 us a step against 563; 300x300x301 with 10,
-        82 %, 2908 against 2180; 200x200x201 without CPML 805 against 496)."""
+        """True when step() can run the fused stage pairs: uniform ch, fewer than
+        2^31 elements (with the rows' padding), every extent at least 4, and on
+        rows that are no multiple of 4 floats, where runs of few steps or on a
+        small grid keep the stage kernels (_runs_pairs), at least 65 % of the
+        grid clear of the y/z CPML shell."""
         nx, ny, nz = self.shape
         return (self.fused and isinstance(self.ch, float) and min(self.shape) >= 4
                 and nx * ny * padded_nz(nz) < 2 ** 31 and (nz % 4 == 0 or self._inside() >= 0.65))
 
     def _runs_pairs(self, n):
         """Whether step(n) takes the stage pairs: where pair_path() allows and, on
-        copies of the state, nothing that the stage kernels take is refused."""
+        copies of the state, they pay for these and nothing that the stage kernels
+        take is refused.
+
+        The copies, their buffers and the plan cost a solver's first call 0.3 to
+        1.5 ms and every call two passes over the state.  Measured with them, ms for
+        n steps, stage kernels / pairs, first call of a fresh solver: no y/z shell,
+        64x64x65 n = 16 1.62 / 1.42, 80x80x81 n = 128 13.3 / 12.0, 200x200x201
+        n = 8 6.40 / 4.64, 256x256x257 n = 5 7.76 / 6.26; with a shell 256x256x257
+        and 10 cells n = 5 9.19 / 9.00, n = 16 29.2 / 24.8, 200x250x251 and 15 cells
+        n = 16 22.8 / 22.1.  Between them the stage kernels are as fast or faster, a
+        long run as well: 128 steps of 110x110x111 18.7 / 20.6, 100x120x121 with 4
+        cells 24.7 / 29.5, 160x160x161 with 10 69.9 / 74.6."""
         if not self.pair_path():
             return False
-        if self.shape[2] % 4 == 0:
+        nx, ny, nz = self.shape
+        if nz % 4 == 0:
             return True
+        cells, shell = nx * ny * nz, self._inside() < 1.0
+        if cells >= 1 << 24:
+            least = 5
+        elif cells >= 1 << (23 if shell else 22):
+            least = 16
+        elif cells <= 1 << 19 and not shell:
+            least = 128
+        else:
+            return False
+        if n < least:
+            return False
         # the pair kernel stages 64 sources a tile at most: no layout of so few exceeds that
         if len(self.src_spec) > 64:
             return False

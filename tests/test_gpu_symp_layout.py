@@ -102,7 +102,7 @@ def test_step_under_capture(first):
 
 def test_no_memory_for_the_copies():
     """A grid whose state fits the device and whose second state does not."""
-    shape = (64, 100, 101)
+    shape = (64, 80, 81)
     a, b = (solver(shape, coefs(shape), npml=(4, 0, 0), fused=fused) for fused in (True, False))
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
@@ -116,3 +116,19 @@ def test_no_memory_for_the_copies():
     assert_same(a, b)
     for q in range(2):
         assert torch.equal(a.cpml.psi_e[q], b.cpml.psi_e[q]) and torch.equal(a.cpml.psi_h[q], b.cpml.psi_h[q])
+
+
+@pytest.mark.parametrize("shape,npml,n,pairs", [
+    ((20, 40, 45), 0, 1, False), ((20, 40, 45), 0, 127, False), ((20, 40, 45), 0, 128, True),
+    ((90, 90, 91), 0, 128, False), ((64, 100, 121), 3, 128, False), ((160, 160, 165), 0, 15, False),
+    ((160, 160, 165), 0, 16, True), ((160, 160, 165), 6, 16, False), ((200, 204, 207), 6, 16, True),
+    ((256, 256, 257), 6, 4, False), ((256, 256, 257), 6, 5, True)])
+def test_short_runs_keep_the_stage_kernels(shape, npml, n, pairs):
+    """Runs too short, or grids too small, to make up for the copies of the state
+    neither make a plan nor allocate a second state."""
+    a, b = (solver(shape, coefs(shape), npml=npml, fused=fused) for fused in (True, False))
+    assert a.pair_path()
+    for s in (a, b):
+        s.step(n)
+    assert a._plan_ready() == pairs and (a._pitched is not None) == pairs
+    assert_same(a, b)
