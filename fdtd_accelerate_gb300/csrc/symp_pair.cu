@@ -274,9 +274,7 @@ k_symp_pair(const __grid_constant__ Maps mk, const __grid_constant__ Params p) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         s_abort = 0;
     }
-    // nothing above touches global memory; the edge kernel may start beside this one, whose
-    // CTAs (never more than are resident) have all seen the launches before it end
-    grid_wait();
+    grid_wait();  // nothing above touches global memory
     grid_release();
     // the group of this thread: H row hr (j0-1+hr), group g (columns
     // k0-4+4g .. k0-1+4g).  Tile groups first (row hr = 1 + tid/8, groups
@@ -781,14 +779,10 @@ struct EdgeStage {
 
 template <bool HH>
 __global__ void __launch_bounds__(EDGE_BLOCK)
-k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb, int32_t beside) {
-    // beside: started by the pair kernel's release, so the launches before that one have
-    // ended, and this one reads nothing that the pair kernel writes.  Its own end stands for
-    // both kernels': its last block waits for the pair kernel.
-    if (!beside) grid_wait();
+k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
+    grid_wait();
     grid_release();
     int i, j, k;
-    if (beside && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && threadIdx.x == 0) grid_wait();
     if (!edge_group(eb, i, j, k)) return;
     sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false>{p});
 }
@@ -912,7 +906,19 @@ struct fdtd_symp_plan {
     bool auto_chunk;               // x_chunk chosen per tiling (the caller passed 0)
     int64_t chunk_key[4] = {-1, -1, -1, -1};  // tiling the cached choice was made for
     int chunk_val = 0;
+    // where the shell's H kernel runs beside the pair kernel: its stream, and the events
+    // of the fork from the caller's stream and of the join
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    ~fdtd_symp_plan() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);  // returns at once; its work is done first
+    }
 };
+
+// grids whose pair kernel leaves room on the GPU for kernels beside it
+static bool leaves_room(const Grid &g) { return g.nx * g.ny * g.nz < (1 << 23); }
 
 extern "C" {
 
@@ -996,6 +1002,13 @@ int fdtd_symp_pair_plan_create(fdtd_symp_plan **out, const fdtd_grid *gp, const 
     if (e != cudaSuccess) { set_cuda_error(e); delete pl; return FDTD_ERR_CUDA; }
     if (occ < 1) { delete pl; return FDTD_ERR_UNSUPPORTED; }
     pl->slots = nsm * occ;
+    // (up to 2^21 cells a plan that chooses its chunk runs no pair kernel, or no shell)
+    if (leaves_room(g) && (!pl->auto_chunk || g.nx * g.ny * g.nz > (1 << 21))) {
+        e = cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&pl->fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&pl->join, cudaEventDisableTiming);
+        if (e != cudaSuccess) { set_cuda_error(e); delete pl; return FDTD_ERR_CUDA; }
+    }
     *out = pl;
     return FDTD_OK;
 }
@@ -1127,11 +1140,19 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
     }
     cudaStream_t st = as_stream(stream);
     const int64_t items = (int64_t)p.nty_in * p.ntz_in * p.nxc;
-    // Chained launches hide the gaps between a pass's kernels, and the edge kernel's blocks
-    // start beside a pair kernel that leaves room (200^3, 8-cell CPML: 869 -> 850 us a step,
-    // 128^3 356 -> 312).  Pair kernels that fill the GPU lose more to their company than the
-    // gaps cost (256^3 1373 -> 1418, 512^3 8255 -> 8640).
-    const bool chained = cells < (1 << 23);
+    const int64_t egroups = eb.off[eb.n];  // per x plane
+    // Where the pair kernel leaves room, the shell's H kernel runs beside it, on the plan's
+    // own stream (neither reads what the other writes; k_edge_e reads both), and the passes
+    // of a pair or edge kernel alone are chained, which hides the gaps between launches.
+    // us a step with an 8-cell CPML, one after the other / beside: 164^3 626 / 517, 200^3
+    // 910 / 782 (launched the plain way 842).  Pair kernels that fill the GPU lose to their
+    // company (256^3 1373 -> 1418, 512^3 8255 -> 8640).
+    const bool beside = pl->side && items > 0 && egroups > 0, chained = leaves_room(pl->g) && !beside;
+    if (beside) {
+        cudaError_t e = cudaEventRecord(pl->fork, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(pl->side, pl->fork, 0);
+        if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
+    }
     if (items > 0) {
         const int nb = (int)std::min<int64_t>(items, pl->slots);
         if (two_h)
@@ -1139,14 +1160,18 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
         else
             launch(chained, k_symp_pair<false>, dim3(nb), THREADS, SMEM, st, pl->maps[in], p);
     }
-    const int64_t egroups = eb.off[eb.n];  // per x plane
     if (egroups > 0) {
         const dim3 nb((unsigned)((egroups + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx);
-        const int32_t beside = chained && items > 0;
+        const cudaStream_t hs = beside ? pl->side : st;
         if (two_h)
-            launch(chained, k_edge_h<true>, nb, EDGE_BLOCK, 0, st, p, eb, beside);
+            launch(chained, k_edge_h<true>, nb, EDGE_BLOCK, 0, hs, p, eb);
         else
-            launch(chained, k_edge_h<false>, nb, EDGE_BLOCK, 0, st, p, eb, beside);
+            launch(chained, k_edge_h<false>, nb, EDGE_BLOCK, 0, hs, p, eb);
+        if (beside) {
+            cudaError_t e = cudaEventRecord(pl->join, hs);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(st, pl->join, 0);
+            if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
+        }
         launch(chained, k_edge_e, nb, EDGE_BLOCK, 0, st, p, eb);
         bool esrc = false;
         for (size_t a = 0; a + 2 < pl->src_ijk.size(); a += 3)

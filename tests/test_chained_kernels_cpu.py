@@ -1,0 +1,66 @@
+"""Rules that the chained kernels (started while the launch before them drains)
+keep, read off their sources: a missing wait or a load through the read-only path
+changes no result that a test on one GPU would be sure to see."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fdtd_accelerate_gb300", "csrc")
+
+
+def source(path):
+    with open(path) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def block(text, at):
+    """The brace block that opens at or after position at."""
+    a = text.index("{", at)
+    depth = 0
+    for i in range(a, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[a:i + 1]
+    raise ValueError("unbalanced braces")
+
+
+def kernels():
+    """name -> body of every kernel definition."""
+    out = {}
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = source(path)
+        for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\s*\(", text):
+            out[m.group(1)] = block(text, m.end())
+    return out
+
+
+KERNELS = kernels()
+CHAINED = sorted(k for k, body in KERNELS.items() if "grid_wait" in body or "grid_release" in body)
+
+
+def test_chained_kernels_are_found():
+    assert CHAINED == ["k_edge_e", "k_edge_h", "k_symp_pair", "k_yee_fused"]
+
+
+@pytest.mark.parametrize("name", CHAINED)
+def test_every_thread_waits(name):
+    """grid_wait() under no condition but the kernel's template arguments."""
+    body = KERNELS[name]
+    waits = [m.start() for m in re.finditer(r"\bgrid_wait\(\)", body)]
+    assert waits
+    for at in waits:
+        start = max(body.rfind(c, 0, at) for c in ";{}")
+        assert not body[start + 1:at].strip(), "conditional: " + body[start + 1:at]
+        depth, heads = 0, []
+        for i in range(at - 1, 0, -1):
+            if body[i] == "}":
+                depth += 1
+            elif body[i] == "{":
+                if depth == 0:
+                    heads.append(body[max(body.rfind(c, 0, i) for c in ";{}") + 1:i].strip())
+                else:
+                    depth -= 1
+        assert set(heads) <= {"if (!BATCH)", "else"}, heads
+    assert not re.search(r"\breturn;", body[:waits[0]])
