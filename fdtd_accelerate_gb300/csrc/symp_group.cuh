@@ -58,21 +58,10 @@ struct Group {
         : nx(nx_), ny(ny_), nz(nz_), X(sx), Y(sy), i(i_), j(j_), k(k_),
           c((uint32_t)i_ * sx + (uint32_t)j_ * sy + (uint32_t)k_), in(k_ + 4 <= nz_ ? 0xFu : (1u << (nz_ - k_)) - 1),
           n((int64_t)nx_ * sx) {}
-    // the group at offset at of a field this kernel only reads
-    __device__ __forceinline__ F4 ldg(const float *f, uint32_t at) const {
-        F4 r{};
-        if (in == 0xFu) {
-            if (FDTD_IN(at, n) && FDTD_IN(at + 3, n)) {
-                const float4 t = __ldg(reinterpret_cast<const float4 *>(f + at));
-                r = F4{{t.x, t.y, t.z, t.w}};
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (((in >> e) & 1) && FDTD_IN(at + e, n)) r.v[e] = __ldg(f + at + e);
-        }
-        return r;
-    }
+    // the group at offset at of a field.  (A plain load, as all of a chained kernel's but
+    // the table entries: the launch before may write the field while this one is resident,
+    // and the read-only path is for memory that nothing writes in that time.)
+    __device__ __forceinline__ F4 ldf(const float *f, uint32_t at) const { return ld(f, at, in, true, n); }
     // elements at .. at+3 of a psi array or of the updated field, those of mask m
     __device__ static __forceinline__ F4 ld(const float *f, uint32_t at, uint32_t m, bool vec, int64_t ext) {
         F4 r{};
@@ -101,34 +90,34 @@ struct Group {
     // stencil along x or y (stride s); the rows must exist
     template <bool E>
     __device__ __forceinline__ Window rows(const float *f, uint32_t s) const {
-        return E ? Window{ldg(f, c - s), ldg(f, c), ldg(f, c + s), ldg(f, c + 2 * s)}
-                 : Window{ldg(f, c - 2 * s), ldg(f, c - s), ldg(f, c), ldg(f, c + s)};
+        return E ? Window{ldf(f, c - s), ldf(f, c), ldf(f, c + s), ldf(f, c + 2 * s)}
+                 : Window{ldf(f, c - 2 * s), ldf(f, c - s), ldf(f, c), ldf(f, c + s)};
     }
     // stencil along z; past either end of the row the values are zeros that no updated cell uses
     template <bool E>
     __device__ __forceinline__ Window along_z(const float *f) const {
-        const F4 o = ldg(f, c);
+        const F4 o = ldf(f, c);
         if (E) {
-            const float l = k > 0 && FDTD_IN(c - 1, n) ? __ldg(f + c - 1) : 0.f;
+            const float l = k > 0 && FDTD_IN(c - 1, n) ? f[c - 1] : 0.f;
             float r0 = 0.f, r1 = 0.f;
             if (k + 5 < nz) {
                 if (FDTD_IN(c + 5, n)) {
-                    const float2 t = __ldg(reinterpret_cast<const float2 *>(f + c + 4));
+                    const float2 t = *reinterpret_cast<const float2 *>(f + c + 4);
                     r0 = t.x;
                     r1 = t.y;
                 }
             } else if (k + 4 < nz && FDTD_IN(c + 4, n)) {
-                r0 = __ldg(f + c + 4);
+                r0 = f[c + 4];
             }
             return Window{{{l, o.v[0], o.v[1], o.v[2]}}, o, {{o.v[1], o.v[2], o.v[3], r0}}, {{o.v[2], o.v[3], r0, r1}}};
         }
         float l0 = 0.f, l1 = 0.f;
         if (k > 0 && FDTD_IN(c - 2, n)) {
-            const float2 t = __ldg(reinterpret_cast<const float2 *>(f + c - 2));
+            const float2 t = *reinterpret_cast<const float2 *>(f + c - 2);
             l0 = t.x;
             l1 = t.y;
         }
-        const float r = k + 4 < nz && FDTD_IN(c + 4, n) ? __ldg(f + c + 4) : 0.f;
+        const float r = k + 4 < nz && FDTD_IN(c + 4, n) ? f[c + 4] : 0.f;
         return Window{{{l0, l1, o.v[0], o.v[1]}}, {{l1, o.v[0], o.v[1], o.v[2]}}, o, {{o.v[1], o.v[2], o.v[3], r}}};
     }
 };

@@ -204,8 +204,6 @@ __device__ __forceinline__ int64_t fext(const Params &p) { return (int64_t)p.nx 
 __device__ __forceinline__ int64_t pext(const Params &p, int ax, int P) {
     return ax == 0 ? 2LL * P * p.ny * p.nz : (ax == 1 ? 2LL * p.nx * P * p.nz : 2LL * p.nx * p.ny * P);
 }
-// a read-only global load through the non-coherent path, checked in the debug build
-#define LDG(a, i, n) (FDTD_IN(i, n) ? __ldg((a) + (i)) : 0.f)
 
 // four consecutive floats of shared memory (16-byte aligned)
 struct V4 {
@@ -462,8 +460,8 @@ k_symp_pair(const __grid_constant__ Maps mk, const __grid_constant__ Params p) {
                 if (sxh >= 0) {
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
-                        py[c] = (uy >> c) & 1 ? LDG(p.psi_h_in[0], offx + c, pext(p, 0, p.ha[0].P)) : 0.f;
-                        pz[c] = (uz >> c) & 1 ? LDG(p.psi_h_in[1], offx + c, pext(p, 0, p.ha[0].P)) : 0.f;
+                        py[c] = ((uy >> c) & 1) && FDTD_IN(offx + c, pext(p, 0, p.ha[0].P)) ? p.psi_h_in[0][offx + c] : 0.f;
+                        pz[c] = ((uz >> c) & 1) && FDTD_IN(offx + c, pext(p, 0, p.ha[0].P)) ? p.psi_h_in[1][offx + c] : 0.f;
                     }
                 }
                 if (sxh < 0) {
@@ -770,7 +768,7 @@ struct EdgeStage {
     }
     __device__ __forceinline__ float coef(int st) const { return E ? p.dl : st ? p.cl_b : p.cl_a; }
     __device__ __forceinline__ sg::F4 cv(int q, const sg::Group &g) const {
-        return E ? g.ldg(p.ce[q], g.c) : sg::F4{{p.ch, p.ch, p.ch, p.ch}};
+        return E ? g.ldf(p.ce[q], g.c) : sg::F4{{p.ch, p.ch, p.ch, p.ch}};
     }
     __device__ __forceinline__ float main(int st, float v, float cv, float d27) const {
         return E ? fadd(v, fmul(fmul(p.dl, cv), d27)) : fsub(v, fmul(st ? p.clch_b : p.clch_a, d27));

@@ -449,13 +449,13 @@ __device__ __forceinline__ uint32_t tfsf_masks(const Params &p, int eh, int64_t 
 
 // v += 0.5 (c * F1d[idx]) on the cells m of the group: one face, slot 0 or 1 of it
 __device__ __forceinline__ void tfsf_term(const Params &p, int eh, int face, int slot, int ax, uint32_t m, V4 &v) {
-    const float *f1d = eh == 0 ? p.th1d : p.te1d;  // read-only inside the fused kernel
+    const float *f1d = eh == 0 ? p.th1d : p.te1d;  // (plain loads: the launch before this one writes it)
     const float c = p.tcoef[eh][face][slot];
     const int ix = p.tix[eh][face][slot];
     const int at = ix >= 0 ? ix : ax + p.tvo, step = ix < 0 && p.taxis == 2 ? 1 : 0;
 #pragma unroll
     for (int e = 0; e < 4; e++)
-        if ((m >> e) & 1) v.v[e] = fadd(v.v[e], fmul(0.5f, fmul(c, __ldg(f1d + at + e * step))));
+        if ((m >> e) & 1) v.v[e] = fadd(v.v[e], fmul(0.5f, fmul(c, f1d[at + e * step])));
 }
 
 // The terms of one group (m: its masks) on plane i, E (eh = 0) or H (eh = 1).  A family

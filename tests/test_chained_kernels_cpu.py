@@ -64,3 +64,13 @@ def test_every_thread_waits(name):
                     depth -= 1
         assert set(heads) <= {"if (!BATCH)", "else"}, heads
     assert not re.search(r"\breturn;", body[:waits[0]])
+
+
+@pytest.mark.parametrize("name", ["symp_pair.cu", "symp_group.cuh", "yee_fused.cuh", "yee_fused.cu"])
+def test_read_only_loads_of_tables_alone(name):
+    """The launch before a chained kernel may write its fields, psi and 1-D arrays
+    while the kernel is resident: only the CPML tables go through __ldg."""
+    text = source(os.path.join(CSRC, name))
+    assert not re.search(r"#define[^\n]*__ldg|ld\.global\.nc", text)
+    for arg in re.findall(r"__ldg\(([^;]*)", text):
+        assert re.match(r"T\.(b|a|km1) \+ s", arg), arg
