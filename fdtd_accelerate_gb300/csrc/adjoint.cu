@@ -437,8 +437,15 @@ __global__ void __launch_bounds__(kB) k_adj_h(Args A) {
 struct F4 {
     float v[4];
 };
+// of an array that the kernel only reads
 __device__ __forceinline__ F4 ld4(const float *p) {
     const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+    return F4{{t.x, t.y, t.z, t.w}};
+}
+// of one that it also writes: the read-only path is for memory that nothing writes while
+// the kernel runs
+__device__ __forceinline__ F4 lw4(const float *p) {
+    const float4 t = *reinterpret_cast<const float4 *>(p);
     return F4{{t.x, t.y, t.z, t.w}};
 }
 __device__ __forceinline__ F4 ld4(const float *p, bool on) { return on ? ld4(p) : F4{}; }
@@ -498,7 +505,7 @@ __global__ void __launch_bounds__(kB) k_adj_e4(Args A, uint32_t ng, int vec) {
     const F4 hz0 = ld4(lhz + c, ig && jg), hzj = ld4(lhz + c + Y, jl && ig), hzi = ld4(lhz + c + X, il && jg);
     F4 hyi = ld4(lhy + c + X, il && jl), hxj = ld4(lhx + c + Y, il && jl);
     const float hxk4 = jg && !last ? __ldg(lhx + c + 4) : 0.f, hyk4 = ig && !last ? __ldg(lhy + c + 4) : 0.f;
-    F4 l0 = ld4(A.lf[0] + c), l1 = ld4(A.lf[1] + c), l2 = ld4(A.lf[2] + c);
+    F4 l0 = lw4(A.lf[0] + c), l1 = lw4(A.lf[1] + c), l2 = lw4(A.lf[2] + c);
     if (first) hx0.v[0] = hy0.v[0] = hyi.v[0] = hxj.v[0] = 0.f;  // (k > 0 masks; k+1 neighbours are unaffected)
     F4 d0, d1, d2;
 #pragma unroll
@@ -599,7 +606,7 @@ __global__ void __launch_bounds__(kB) k_adj_e4(Args A, uint32_t ng, int vec) {
         }
     }
     auto accumulate = [&](float *gp, const F4 &l, const F4 &G, int top) {
-        F4 a = ld4(gp + c);
+        F4 a = lw4(gp + c);
 #pragma unroll
         for (int e = 0; e < 4; e++) a.v[e] = fadd(a.v[e], fmul(l.v[e], G.v[e]));
         st4(gp + c, a, glo, min(ghi, top));
@@ -635,7 +642,7 @@ __global__ void __launch_bounds__(kB) k_adj_h4(Args A, uint32_t ng, int vec) {
     F4 n0 = nu4(0, 0, jl), n1 = nu4(1, 0, il), n1i = nu4(1, -X, ig && jg), n0j = nu4(0, -Y, ig && jg);
     const F4 n2 = nu4(2, 0, il && jl), n2j = nu4(2, -Y, jg && il), n2i = nu4(2, -X, ig && jl);
     const float n1k = nu1(1, il && !first), n0k = nu1(0, jl && !first);
-    F4 h0 = ld4(A.lf[3] + c), h1 = ld4(A.lf[4] + c), h2 = ld4(A.lf[5] + c);
+    F4 h0 = lw4(A.lf[3] + c), h1 = lw4(A.lf[4] + c), h2 = lw4(A.lf[5] + c);
     if (last) n0.v[3] = n1.v[3] = n1i.v[3] = n0j.v[3] = 0.f;  // (k < nz-1 masks)
     F4 d0, d1, d2;
 #pragma unroll

@@ -74,3 +74,13 @@ def test_read_only_loads_of_tables_alone(name):
     assert not re.search(r"#define[^\n]*__ldg|ld\.global\.nc", text)
     for arg in re.findall(r"__ldg\(([^;]*)", text):
         assert re.match(r"T\.(b|a|km1) \+ s", arg), arg
+
+
+@pytest.mark.parametrize("name", ["k_adj_e4", "k_adj_h4"])
+def test_written_arrays_are_not_read_as_read_only(name):
+    """No array that the adjoint cell kernels store to is loaded through ld4 / ldp /
+    __ldg in the same kernel."""
+    body = KERNELS[name]
+    stored = set(re.findall(r"\bst4\(([\w.\[\]]+)", body))
+    assert len(stored) >= 3
+    assert not stored & set(re.findall(r"\b(?:ld4|ldp|__ldg)\(([\w.\[\]]+)", body))
