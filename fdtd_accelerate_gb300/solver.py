@@ -78,7 +78,10 @@ class YeeSolver:
 
     # ------------------------------------------------------------------ views
     def _views(self, b):
-        return list(self._state[b].narrow(3, 0, self.shape[2]).unbind(0))
+        # one view operation for each: the views of an unbind() refuse writes that autograd records
+        nx, ny, _ = self.shape
+        n, strides = nx * ny * self.nzp, (ny * self.nzp, self.nzp, 1)
+        return [self._state.as_strided(self.shape, strides, (6 * b + q) * n) for q in range(6)]
 
     @property
     def fields(self):
