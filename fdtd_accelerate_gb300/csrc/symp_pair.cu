@@ -794,19 +794,48 @@ k_edge_e(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true>{p});
 }
 
-// soft sources on edge cells, list order (one thread: a list holds a few sources)
-__global__ void k_edge_src(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || p.t < 0 || p.t >= p.namp) return;
-    for (int s = 0; s < p.nsrc; s++) {
-        const int si = p.src_ijk[3 * s], sj = p.src_ijk[3 * s + 1], sk = p.src_ijk[3 * s + 2];
-        bool in = false;
+// Soft sources on edge cells, as a walk of the list in order would add them: a thread a
+// source, the list staged in shared memory a block at a time.  The first source of a cell
+// and component adds all of them, the others nothing.  (Small grids are all shell: 64x96x96
+// with 1080 sources, us a step, one thread walking the list 1904, this form 178; with one
+// source 87.)
+constexpr int SRC_BLOCK = 256, SRC_STAGE = 1024;
+__global__ void __launch_bounds__(SRC_BLOCK) k_edge_src(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
+    __shared__ int64_t s_key[SRC_STAGE];  // 4 * cell offset + component, -1: past the list
+    __shared__ float s_v[SRC_STAGE];
+    const int tid = threadIdx.x, s = blockIdx.x * SRC_BLOCK + tid;
+    auto key_of = [&](int q) {
+        return 4 * ((int64_t)p.src_ijk[3 * q] * p.sx + (int64_t)p.src_ijk[3 * q + 1] * p.sy + p.src_ijk[3 * q + 2]) +
+               p.src_comp[q];
+    };
+    int64_t key = -2;  // none
+    if (s < p.nsrc) {
+        const int sj = p.src_ijk[3 * s + 1], sk = p.src_ijk[3 * s + 2];
         for (int b = 0; b < eb.n; b++)
-            in |= sj >= eb.j0[b] && sj < eb.j1[b] && sk >= eb.k0[b] && sk < eb.k1[b];
-        if (!in) continue;
-        float *f = p.out[p.src_comp[s]];
-        const int64_t c = (int64_t)si * p.sx + (int64_t)sj * p.sy + sk;
-        if (FDTD_IN(c, fext(p))) f[c] = fadd(f[c], p.src_amp[(int64_t)s * p.namp + p.t]);
+            if (sj >= eb.j0[b] && sj < eb.j1[b] && sk >= eb.k0[b] && sk < eb.k1[b]) key = key_of(s);
+        if (key >= 0 && !FDTD_IN(key >> 2, fext(p))) key = -2;
     }
+    bool first = key >= 0;
+    float *f = p.out[key & 3] + (key >> 2);
+    float v = first ? *f : 0.f;
+    for (int r0 = 0; r0 < p.nsrc; r0 += SRC_STAGE) {
+        __syncthreads();
+#pragma unroll
+        for (int u = tid; u < SRC_STAGE; u += SRC_BLOCK) {
+            const bool in = r0 + u < p.nsrc;
+            s_key[u] = in ? key_of(r0 + u) : -1;
+            s_v[u] = in ? p.src_amp[(int64_t)(r0 + u) * p.namp + p.t] : 0.f;
+        }
+        __syncthreads();
+        const int n = (min(SRC_STAGE, p.nsrc - r0) + 15) / 16 * 16;
+#pragma unroll 16
+        for (int r = 0; r < n; r++)
+            if (s_key[r] == key) {
+                if (r0 + r < s) first = false;
+                else v = fadd(v, s_v[r]);
+            }
+    }
+    if (first) *f = v;
 }
 
 }  // namespace sp
@@ -1176,7 +1205,7 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
             for (int b = 0; b < eb.n; b++)
                 esrc |= pl->src_ijk[a + 1] >= eb.j0[b] && pl->src_ijk[a + 1] < eb.j1[b] &&
                         pl->src_ijk[a + 2] >= eb.k0[b] && pl->src_ijk[a + 2] < eb.k1[b];
-        if (esrc && src_t >= 0 && src_t < p.namp) k_edge_src<<<1, 32, 0, st>>>(p, eb);
+        if (esrc && src_t >= 0 && src_t < p.namp) k_edge_src<<<(p.nsrc + SRC_BLOCK - 1) / SRC_BLOCK, SRC_BLOCK, 0, st>>>(p, eb);
     }
     FDTD_TRY(check_launch());
     pl->cur = ob;
