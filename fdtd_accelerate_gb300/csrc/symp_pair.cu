@@ -874,19 +874,16 @@ static int map3(EncodeFn enc, CUtensorMap *m, const float *ptr, const Grid &g, i
 }
 
 // x planes per work item when the caller leaves the choice to the plan: of
-// the chunks 48 .. 256 (steps of 8; from 8 on where chunks of 48 make fewer
-// items than two rounds of CTAs: with 48 planes at least, 150x171x163 filled
-// half of them), the one whose greedy schedule of a pass's items over the
-// resident CTAs ends first.  The queue hands items out
+// the chunks least .. 256 (steps of 8), the one whose greedy schedule of a
+// pass's items over the resident CTAs ends first.  The queue hands items out
 // x chunk by x chunk; an item costs its planes (x-slab planes, which carry
 // the CPML terms, twice) plus the 6 iterations that fill the pipeline.  The
 // largest chunk wins ties (fewer fills).
-static int choose_x_chunk(int nx, int64_t tiles, int slots, int pf, int pb) {
+static int choose_x_chunk(int nx, int64_t tiles, int slots, int pf, int pb, int least) {
     int best = std::min(nx, 128);
     int64_t best_t = -1;
     std::map<int64_t, int64_t> free_at;  // CTAs by the time they are free
     int last = -1;
-    const int least = tiles * ((nx + 47) / 48) < 2 * (int64_t)slots ? 8 : 48;
     for (int xc = 256; xc >= least; xc -= 8) {
         const int c = std::min(xc, nx);
         if (c == last) continue;  // chunks past nx are all the whole grid
@@ -932,7 +929,7 @@ struct fdtd_symp_plan {
     int cur;
     bool auto_chunk;               // x_chunk chosen per tiling (the caller passed 0)
     int64_t chunk_key[4] = {-1, -1, -1, -1};  // tiling the cached choice was made for
-    int chunk_val = 0;
+    int chunk_val = 0, count_chunk = 0;
     // where the shell's H kernel runs beside the pair kernel: its stream, and the events
     // of the fork from the caller's stream and of the join
     cudaStream_t side = nullptr;
@@ -1120,22 +1117,32 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
     if (pl->auto_chunk && p.nty_in > 0 && p.ntz_in > 0) {
         const int64_t key[4] = {p.nty_in, p.ntz_in, pf(0), pb(0)};
         if (!std::equal(key, key + 4, pl->chunk_key)) {
-            pl->chunk_val = choose_x_chunk(p.nx, (int64_t)p.nty_in * p.ntz_in, pl->slots, pf(0), pb(0));
+            // 48 planes and more, or 8 and more where chunks of 48 make fewer items than two
+            // rounds of CTAs (150x171x163 then filled half of them).  The chunk of 48 and more
+            // stays the one in which sources are counted: it fixes which layouts are refused.
+            const int64_t tiles = (int64_t)p.nty_in * p.ntz_in;
+            pl->count_chunk = pl->chunk_val = choose_x_chunk(p.nx, tiles, pl->slots, pf(0), pb(0), 48);
+            if (tiles * ((p.nx + 47) / 48) < 2 * (int64_t)pl->slots)
+                pl->chunk_val = choose_x_chunk(p.nx, tiles, pl->slots, pf(0), pb(0), 8);
             std::copy(key, key + 4, pl->chunk_key);
         }
         p.x_chunk = pl->chunk_val;
         p.nxc = (p.nx + p.x_chunk - 1) / p.x_chunk;
     }
     // sources per tile of this tiling (the kernel stages at most MAX_SRC per tile)
-    if (p.nty_in > 0 && p.ntz_in > 0 && pl->src_ijk.size() / 3 > (size_t)MAX_SRC) {
-        std::vector<int> count((size_t)p.nty_in * p.ntz_in * p.nxc, 0);
+    auto sources_fit = [&](int chunk) {
+        std::vector<int> count((size_t)p.nty_in * p.ntz_in * ((p.nx + chunk - 1) / chunk), 0);
         for (size_t a = 0; a + 2 < pl->src_ijk.size(); a += 3) {
             const int si = pl->src_ijk[a], sj = pl->src_ijk[a + 1], sk = pl->src_ijk[a + 2];
             if (sj < p.j_lo || sj >= p.j_hi || sk < p.k_lo || sk >= p.k_hi) continue;
-            const size_t it = ((size_t)(si / p.x_chunk) * p.nty_in + (sj - p.j_lo) / TY) * p.ntz_in + (sk - p.kt0) / TZ;
-            if (++count[it] > MAX_SRC) return FDTD_ERR_CAPACITY;
+            const size_t it = ((size_t)(si / chunk) * p.nty_in + (sj - p.j_lo) / TY) * p.ntz_in + (sk - p.kt0) / TZ;
+            if (++count[it] > MAX_SRC) return false;
         }
-    }
+        return true;
+    };
+    if (p.nty_in > 0 && p.ntz_in > 0 && pl->src_ijk.size() / 3 > (size_t)MAX_SRC &&
+        !(sources_fit(p.x_chunk) && (!pl->auto_chunk || pl->count_chunk == p.x_chunk || sources_fit(pl->count_chunk))))
+        return FDTD_ERR_CAPACITY;
     // the edge shell: rows outside [j_lo, j_hi), then the columns outside
     // [k_lo, k_hi) of those rows (every x plane)
     Edge eb{};

@@ -43,3 +43,17 @@ def test_long_lists(shape, npml, each):
     one = solver(shape, coefs(shape), npml=npml, max_steps=10)
     one.step(1)
     assert step_us(a) < 3 * step_us(one)
+
+
+@pytest.mark.parametrize("planes,fits", [(32, True), (36, False)])
+def test_layouts_counted_in_chunks_of_48_planes(planes, fits):
+    """Which layouts are refused does not follow the shorter x chunks of small grids:
+    two rows of `planes` sources in the tile of rows 8 .. 23."""
+    shape = (64, 64, 64)
+    src = [("ez", (i, j, 20), lambda t: 1e-3 * t) for i in range(10, 10 + planes) for j in (10, 20)]
+    s = solver(shape, coefs(shape), sources=src, npml=6, max_steps=4)
+    if fits:
+        s.step(1)
+    else:
+        with pytest.raises(ValueError, match="capacity"):
+            s.step(1)
