@@ -1082,6 +1082,11 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
             dst[w][ax] = A;
         }
     }
+    // the two H stages share slab indices and psi: with another layer the second's tables
+    // would be read where they have no entries
+    for (int ax = 0; ax < 3; ax++)
+        if (p.ha[ax].P != p.hb[ax].P || p.ha[ax].front != p.hb[ax].front || p.ha[ax].back != p.hb[ax].back)
+            return FDTD_ERR_ARG;
     for (int q = 0; q < 6; q++) p.in[q] = pl->f[in][q];
     p.vpsi = p.nz % 4 == 0;
     for (int q = 0; q < 4; q++)

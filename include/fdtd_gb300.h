@@ -312,7 +312,8 @@ int fdtd_symp_pair_plan_create(fdtd_symp_plan **plan, const fdtd_grid *g, const 
 /* One pass: the H stage cl_a (with two_h = 1, then the H stage cl_b), the E
  * stage dl, then the sources at amplitude index src_t, reading buffer cur and
  * writing the other.  Each stage's CPML tables come from its fdtd_cpml (the
- * H tables of h_a / h_b, the E tables of e; NULL: no CPML); ch is uniform.
+ * H tables of h_a / h_b, the E tables of e; NULL: no CPML; with two_h the layers
+ * of h_a and h_b must be alike, else FDTD_ERR_ARG); ch is uniform.
  * Bit-identical to fdtd_symplectic_stage_f32 for each stage in turn and
  * fdtd_add_sources_f32.  Replaces one (update_h, update_e) pair of the
  * stage loop of 4th_order-Symplectic/PyCUDA/100-base.py:124-141. */

@@ -132,3 +132,25 @@ def test_short_runs_keep_the_stage_kernels(shape, npml, n, pairs):
         s.step(n)
     assert a._plan_ready() == pairs and (a._pitched is not None) == pairs
     assert_same(a, b)
+
+
+def test_two_h_stages_of_unlike_layers_are_refused():
+    """A pass of two H stages whose layers differ: an error code, and the state as it was."""
+    import ctypes as C
+    from fdtd_accelerate_gb300 import _native as N
+    from fdtd_accelerate_gb300.symplectic import CL, DL
+    s = solver((20, 40, 44), coefs((20, 40, 44)), npml=4)
+    s.step(1)
+    before = {k: v.clone() for k, v in s.fields.items()}
+    a, e, none, thin, half = s.cpml._structs[CL[0]], s.cpml._structs[DL[0]], N.Cpml(), N.Cpml(), N.Cpml()
+    for other, npml, faces in ((thin, 3, 0x3F), (half, 4, 0x2F)):
+        C.memmove(C.byref(other), C.byref(a), C.sizeof(a))
+        other.npml[2], other.faces = npml, faces
+    ref = lambda c: C.byref(c) if c is not None else None
+    for ha, hb in ((a, None), (None, a), (a, none), (a, thin), (thin, a), (a, half)):
+        st = N.lib().fdtd_symp_pair_run(s._pair, ref(ha), ref(hb), ref(e), CL[4], CL[0], 1, DL[0], float(s.ch), -1, None)
+        assert st == N.FDTD_ERR_ARG
+    assert N.lib().fdtd_symp_pair_plan_current(s._pair) == s._cur
+    torch.cuda.synchronize()
+    for k in NAMES:
+        assert torch.equal(s.fields[k], before[k]), k
