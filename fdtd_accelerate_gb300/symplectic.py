@@ -227,7 +227,13 @@ class SymplecticSolver:
     def _as_f32(self, arrays):
         """Three coefficient arrays on the device: a contiguous float32 tensor of
         the caller's is used in place, so that edits of it reach the next call."""
-        return [torch.as_tensor(c, dtype=torch.float32, device=self.device).contiguous() for c in arrays]
+        out = [torch.as_tensor(c, dtype=torch.float32, device=self.device).contiguous() for c in arrays]
+        nx, ny, nz = self.shape
+        for c in out:  # (the kernels take the address: any shape of enough elements does)
+            if c.numel() < nx * ny * nz:
+                raise ValueError("a coefficient array of shape %s has fewer elements than the %s grid"
+                                 % (tuple(c.shape), self.shape))
+        return out
 
     def _pair_arrays(self):
         """The two state buffers and the ce arrays that the stage-pair path runs

@@ -19,3 +19,14 @@ def test_symplectic_fields_and_coefficients(nz):
     w = torch.full((6, 7, nz), 0.5, requires_grad=True)
     s = SymplecticSolver((6, 7, nz), ce=[w] * 3, ch=[w] * 3, device="cpu")
     assert s.fields["ex"].is_contiguous() and s.ce[0].data_ptr() == w.data_ptr() and s.ch[2].data_ptr() == w.data_ptr()
+
+
+@pytest.mark.parametrize("nz", [8, 9])
+def test_symplectic_coefficients_of_too_few_elements(nz):
+    from fdtd_accelerate_gb300.symplectic import SymplecticSolver
+    full = torch.zeros(6 * 7 * nz)
+    for bad in (torch.zeros(nz), torch.zeros(6, 7, nz - 1), 0.5):
+        for kw in ({"ce": [full, full, bad]}, {"ch": [bad, full, full]}):
+            with pytest.raises(ValueError, match="fewer elements"):
+                SymplecticSolver((6, 7, nz), device="cpu", **kw)
+    SymplecticSolver((6, 7, nz), ce=[full] * 3, ch=[full.view(6, 7, nz)] * 3, device="cpu")
