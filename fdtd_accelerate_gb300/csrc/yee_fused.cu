@@ -159,18 +159,20 @@ static int encode_map(EncodeTiledFn enc, CUtensorMap *m, const float *ptr, const
 constexpr int kTileY = 8, kStages = 3;
 constexpr int kCluster = 8;
 
-// Whether a single grid's z slab is left to the band kernels.  In the fused
-// kernel a z-edge tile takes twice the time of a plain one a plane (its row
-// warps run the z code for a quarter of their lanes), and its neighbours then
-// share no halo reads with it; the band kernels cost two launches and a second
-// pass over the row ends.  Measured, fused / bands, us a step with CPML on all
-// faces: 64^3 15 / 23, 80^3 33 / 35, 128^3 65 / 62, 256x256x128 186 / 160,
-// 256^3 315 / 247, 400x300x200 633 / 412, 512^3 1739 / 1545, 1024x1024x512
-// 6078 / 5843.  Grids of few (i, j) rows keep the bands' three
-// launches, which plan_info reports and the tests of it expect.
-static bool use_bands(const Grid &g) {
-    const int64_t rows = g.nx * g.ny;
-    return rows < 2048 || rows * g.nz >= ((int64_t)1 << 21);
+// Whether a single grid's z slab (slab nodes a row) is left to the band kernels.
+// In the fused kernel a z-edge tile takes twice the time of a plain one a plane
+// (its row warps run the z code for a quarter of their lanes), and its neighbours
+// then share no halo reads with it; the band kernels cost two launches and a second
+// pass over the row ends.  Measured, fused / bands, us a step with an 8-cell CPML on
+// all faces: 48^3 16 / 21, 64^3 16 / 21, 80^3 34 / 33, 100x100x64 28 / 29, 100^3
+// 51 / 46, 52x162x171 65 / 54, 125x125x130 89 / 73, with a Drude box 104 / 77; with 12
+// cells 256x256x128 186 / 160, 512^3 1739 / 1545.  Rows that are mostly slab lose
+// earlier: 200x200x20 with a Drude box 112 / 70, 1000x60x20 157 / 101 (the kernels before
+// these 104 and 132).  Grids of few (i, j) rows keep the bands' three launches, which
+// plan_info reports and the tests of it expect.
+static bool use_bands(const Grid &g, int slab) {
+    const int64_t rows = g.nx * g.ny, cells = rows * g.nz;
+    return rows < 2048 || cells >= (2 * slab > g.nz ? 3 << 18 : 13 << 16);
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -329,7 +331,7 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         p.th1d = t.h1d;
     }
     // the z slab (when a z face has CPML): inside the fused kernel or by the band kernels
-    p.zfix = (p.P[2] > 0 && ((p.faces >> 4) & 3) && (batch_chunk ? batch_bands : use_bands(g))) ? 1 : 0;
+    p.zfix = (p.P[2] > 0 && ((p.faces >> 4) & 3) && (batch_chunk ? batch_bands : use_bands(g, zband_e_row(p)))) ? 1 : 0;
     // tile rows with y slab cells (rows j0-1 .. j0+ty-1), counted from either end
     if (p.P[1] > 0)
         for (int t = 0; t < p.nty; t++) {

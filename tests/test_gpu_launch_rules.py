@@ -1,0 +1,49 @@
+"""Launch rules of the fused step on the forms that an earlier rule slowed down: the
+route taken, and the step through it equal to the array calls bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("ex", "ey", "ez", "hx", "hy", "hz")
+
+
+def solver(shape, npml, drude=False, tfsf=False, tile=None):
+    import fdtd_accelerate_gb300 as F
+    rng = np.random.default_rng(8)
+    extra = {}
+    if drude:
+        extra["drude"] = F.DrudeAde(shape, [n // 4 for n in shape], [n // 2 for n in shape])
+        extra["drude"].set_coeff(0.2, 0.05)
+    if tfsf:
+        extra["tfsf"] = F.Tfsf(shape, [npml + 5] * 3, [n - npml - 6 for n in shape], wavelength=12.0, steps=16)
+    s = F.YeeSolver(shape, npml=npml, tile=tile, sources=[("ez", tuple(n // 2 for n in shape), np.sin(0.3 * np.arange(12.0)))],
+                    **extra)
+    s.set_fields(**{k: (0.1 * rng.standard_normal(shape)).astype(np.float32) for k in NAMES})
+    return s
+
+
+def check(a, b, n=3):
+    a.step(n)
+    b.step_unfused(n)
+    torch.cuda.synchronize()
+    a.check_status()
+    for k in NAMES:
+        assert torch.equal(a.fields[k], b.fields[k]), k
+    for q in range(6):
+        if a.psi_e()[q] is not None:
+            assert torch.equal(a.psi_e()[q], b.psi_e()[q]) and torch.equal(a.cpml.psi_h[q], b.cpml.psi_h[q]), q
+
+
+@pytest.mark.parametrize("shape,npml,drude,band", [
+    ((1000, 60, 20), 8, False, 1),     # rows that are mostly slab
+    ((197, 200, 20), 8, True, 1),      # the line of such rows: 786432 cells
+    ((196, 200, 20), 8, True, 0),
+    ((52, 162, 171), 8, True, 1),
+    ((95, 95, 95), 6, False, 1),       # the line of the others: 851968 cells
+    ((94, 95, 95), 6, False, 0)])
+def test_z_slab_route(shape, npml, drude, band):
+    a, b = (solver(shape, npml, drude) for _ in range(2))
+    assert a.plan_info()["z_band"] == band
+    check(a, b)
