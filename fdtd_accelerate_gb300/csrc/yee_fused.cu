@@ -352,7 +352,16 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
     const int max_ctas = tile ? (int)tile->ctas_per_sm : 0;
     if (max_ctas > 0) occ = std::min(occ, max_ctas);
     const int cap_chunk = xch ? xch : capacity_chunk(g.nx, (int64_t)p.ntz * p.nty, nsm);
-    if (!xch) xch = batch_chunk ? batch_chunk : single_chunk(g.nx, (int64_t)p.ntz * p.nty, (int64_t)nsm * occ);
+    if (!xch) {
+        xch = batch_chunk ? batch_chunk : single_chunk(g.nx, (int64_t)p.ntz * p.nty, (int64_t)nsm * occ);
+        // With a wave and CPML a tile's planes take up to three times as long where they hold
+        // faces and slabs, and a launch of one round lasts as long as its slowest item: no
+        // longer chunks than give 3 items an SM.  us a step, one round / this, a box 5 cells
+        // off the layer: 180^3 with 4 cells 249 / 170, 150^3 with 8 211 / 152, 300x120x120
+        // 198 / 154, with a Drude box 211 / 182 (the kernels before these: 223, 191, 184, 217);
+        // 256^3 takes several rounds and keeps its chunk.
+        if (p.tfsf && pml) xch = std::min(xch, cap_chunk);
+    }
     pl->x_chunk = p.x_chunk = (int)std::min<int64_t>(xch, g.nx);
     p.nxc = (int)((g.nx + pl->x_chunk - 1) / pl->x_chunk);
     pl->nitems = (int64_t)p.ntz * p.nty * p.nxc;

@@ -47,3 +47,14 @@ def test_z_slab_route(shape, npml, drude, band):
     a, b = (solver(shape, npml, drude) for _ in range(2))
     assert a.plan_info()["z_band"] == band
     check(a, b)
+
+
+@pytest.mark.parametrize("shape,npml,drude,tile,most", [
+    ((180, 180, 180), 4, False, None, 16), ((300, 120, 120), 8, True, None, 16), ((125, 125, 130), 8, False, None, 8),
+    ((125, 125, 130), 8, False, (8, 40), 40)])
+def test_x_chunk_with_a_wave(shape, npml, drude, tile, most):
+    """Grids with a wave and CPML whose launch would be one round of long items take
+    chunks that give 3 items an SM; a chunk of the caller's stays."""
+    a, b = (solver(shape, npml, drude, True, tile) for _ in range(2))
+    assert a.plan_info()["x_chunk"] == most
+    check(a, b)
