@@ -447,23 +447,27 @@ __device__ __forceinline__ uint32_t tfsf_masks(const Params &p, int eh, int64_t 
     return m;
 }
 
-// v += 0.5 (c * F1d[idx]) on the cells m of the group: one face, slot 0 or 1 of it
-__device__ __forceinline__ void tfsf_term(const Params &p, int eh, int face, int slot, int ax, uint32_t m, V4 &v) {
-    const float *f1d = eh == 0 ? p.th1d : p.te1d;  // (plain loads: the launch before this one writes it)
+// v += 0.5 (c * F1d[idx]) on the cells m of the group: one face, slot 0 or 1 of it.
+// The 1-D arrays go through the read-only path (plain loads: 200^3 194 -> 214 us a step).
+// Nothing writes them while this kernel is resident, as the 1-D step before it calls no
+// grid_release(); and no load can move above the wait, after which zero is known.
+__device__ __forceinline__ void tfsf_term(const Params &p, int zero, int eh, int face, int slot, int ax, uint32_t m,
+                                          V4 &v) {
+    const float *f1d = eh == 0 ? p.th1d : p.te1d;
     const float c = p.tcoef[eh][face][slot];
     const int ix = p.tix[eh][face][slot];
-    const int at = ix >= 0 ? ix : ax + p.tvo, step = ix < 0 && p.taxis == 2 ? 1 : 0;
+    const int at = (ix >= 0 ? ix : ax + p.tvo) + zero, step = ix < 0 && p.taxis == 2 ? 1 : 0;
 #pragma unroll
     for (int e = 0; e < 4; e++)
-        if ((m >> e) & 1) v.v[e] = fadd(v.v[e], fmul(0.5f, fmul(c, f1d[at + e * step])));
+        if ((m >> e) & 1) v.v[e] = fadd(v.v[e], fmul(0.5f, fmul(c, __ldg(f1d + at + e * step))));
 }
 
 // The terms of one group (m: its masks) on plane i, E (eh = 0) or H (eh = 1).  A family
 // at a time, 4 cells each: one cell at a time, with the family's face and table looked up
 // for each, a plane of a tile with a y face row took 3 times as long (256^3, 12-cell
 // CPML, all faces of a 128^3 box: 404 us a step, 340 with this form; without a wave 247).
-__device__ __forceinline__ void tfsf_group(const Params &p, int eh, uint32_t m, int i, int j, int k, V4 &vx, V4 &vy,
-                                           V4 &vz) {
+__device__ __forceinline__ void tfsf_group(const Params &p, int zero, int eh, uint32_t m, int i, int j, int k, V4 &vx,
+                                           V4 &vy, V4 &vz) {
     const int32_t i1 = p.tp1[0], i2 = p.tp2[0];
     const bool xb = i == i2, xface = (i == (eh ? i1 : i1 - 1) && (p.tfaces & 1)) || (xb && ((p.tfaces >> 1) & 1));
     if (!tin(i, i1, eh ? i2 - 1 : i2)) m &= ~0x0000ffu;  // y, z faces of the x component
@@ -474,15 +478,15 @@ __device__ __forceinline__ void tfsf_group(const Params &p, int eh, uint32_t m, 
     const int fx = xb ? 1 : 0, fy = j == p.tp2[1] ? 3 : 2;
     const uint32_t back = k <= p.tp2[2] && p.tp2[2] < k + 4 ? 1u << (p.tp2[2] - k) : 0u;
     auto zfaces = [&](uint32_t z, int slot, V4 &v) {
-        if (z & ~back) tfsf_term(p, eh, 4, slot, ax, z & ~back, v);
-        if (z & back) tfsf_term(p, eh, 5, slot, ax, z & back, v);
+        if (z & ~back) tfsf_term(p, zero, eh, 4, slot, ax, z & ~back, v);
+        if (z & back) tfsf_term(p, zero, eh, 5, slot, ax, z & back, v);
     };
-    if (m & 15u) tfsf_term(p, eh, fy, 1, ax, m & 15u, vx);
+    if (m & 15u) tfsf_term(p, zero, eh, fy, 1, ax, m & 15u, vx);
     if ((m >> 4) & 15u) zfaces((m >> 4) & 15u, 0, vx);
-    if ((m >> 8) & 15u) tfsf_term(p, eh, fx, 0, ax, (m >> 8) & 15u, vy);
+    if ((m >> 8) & 15u) tfsf_term(p, zero, eh, fx, 0, ax, (m >> 8) & 15u, vy);
     if ((m >> 12) & 15u) zfaces((m >> 12) & 15u, 1, vy);
-    if ((m >> 16) & 15u) tfsf_term(p, eh, fx, 1, ax, (m >> 16) & 15u, vz);
-    if (m >> 20) tfsf_term(p, eh, fy, 0, ax, m >> 20, vz);
+    if ((m >> 16) & 15u) tfsf_term(p, zero, eh, fx, 1, ax, (m >> 16) & 15u, vz);
+    if (m >> 20) tfsf_term(p, zero, eh, fy, 0, ax, m >> 20, vz);
 }
 
 // EXT: bit 0: the Drude box is compiled in, bit 1: the TFSF faces, bit 2: the
@@ -562,6 +566,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    [[maybe_unused]] int zero = 0;  // of a value that the compiler knows only after the wait (tfsf_term)
     if (!BATCH) {
         if (producer)
             for (int c = 0; c < 3; c++) {
@@ -570,6 +575,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                 prefetch_tmap(&mk.ce[c]);
             }
         grid_wait();
+        if (TFSF) asm volatile("" : "+r"(zero) : : "memory");
         stage_tables();
     } else {
         grid_wait();
@@ -933,7 +939,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     }
                 }
                 // TFSF: E += 0.5 (c * H1d), after the CPML terms, before the sources
-                if (gen && TFSF && tplane && te) tfsf_group(p, 0, te, i, jj, kk, ex, ey, ez);
+                if (gen && TFSF && tplane && te) tfsf_group(p, zero, 0, te, i, jj, kk, ex, ey, ez);
                 if (gen && i >= smin && i <= smax) {  // soft sources, list order
                     const uint32_t ij_here = ((uint32_t)i << 16) | (uint32_t)jj;
                     const int ns = nls >= 0 ? nls : p.nsrc;
@@ -1035,7 +1041,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
                     stz4(p.psi_h[5], qz, m1, zh, pz1, pext_y(p, 5));
                 }
                 // TFSF: H += 0.5 (c * E1d), after the CPML terms
-                if (gen && TFSF && tplane && th) tfsf_group(p, 1, th, i, jj, kk, ox, oy, oz);
+                if (gen && TFSF && tplane && th) tfsf_group(p, zero, 1, th, i, jj, kk, ox, oy, oz);
                 const int64_t gi = (int64_t)i * p.sx + (int64_t)jj * p.sy + kk;
                 stg4(p.out[0], gi, inm, true, ex, fext_y(p));
                 stg4(p.out[1], gi, inm, true, ey, fext_y(p));

@@ -68,12 +68,22 @@ def test_every_thread_waits(name):
 
 @pytest.mark.parametrize("name", ["symp_pair.cu", "symp_group.cuh", "yee_fused.cuh", "yee_fused.cu"])
 def test_read_only_loads_of_tables_alone(name):
-    """The launch before a chained kernel may write its fields, psi and 1-D arrays
-    while the kernel is resident: only the CPML tables go through __ldg."""
+    """The launch before a chained kernel may write its fields and psi while the kernel
+    is resident: only the CPML tables (and a wave's 1-D arrays) go through __ldg."""
     text = source(os.path.join(CSRC, name))
     assert not re.search(r"#define[^\n]*__ldg|ld\.global\.nc", text)
     for arg in re.findall(r"__ldg\(([^;]*)", text):
-        assert re.match(r"T\.(b|a|km1) \+ s", arg), arg
+        assert re.match(r"T\.(b|a|km1) \+ s", arg) or (name == "yee_fused.cuh" and arg.startswith("f1d + at")), arg
+
+
+def test_one_dimensional_arrays_of_a_wave():
+    """The fused kernel reads them through __ldg: the kernels that write them start
+    nothing before their own end, and the offset is known after the wait only."""
+    writers = [k for k, body in KERNELS.items() if "1d" in k or "1D" in body or "e1d[" in body or "h1d[" in body]
+    assert writers and not set(writers) & set(CHAINED)
+    text = source(os.path.join(CSRC, "yee_fused.cuh"))
+    assert re.search(r"const int at = \(ix >= 0 \? ix : ax \+ p\.tvo\) \+ zero,", text)
+    assert re.search(r"grid_wait\(\);\s*if \(TFSF\) asm volatile\(\"\" : \"\+r\"\(zero\) : : \"memory\"\);", text)
 
 
 @pytest.mark.parametrize("name", ["k_adj_e4", "k_adj_h4"])
