@@ -359,8 +359,9 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         // longer chunks than give 3 items an SM.  us a step, one round / this, a box 5 cells
         // off the layer: 180^3 with 4 cells 249 / 170, 150^3 with 8 211 / 152, 300x120x120
         // 198 / 154, with a Drude box 211 / 182 (the kernels before these: 223, 191, 184, 217);
-        // 256^3 takes several rounds and keeps its chunk.
-        if (p.tfsf && pml) xch = std::min(xch, cap_chunk);
+        // 256^3 takes several rounds and keeps its chunk.  Not on other launch shapes: one CTA an
+        // SM (100x100x64 with 4 cells 63 / 87) and tiles of 4 rows (80^3, 6 stages, 72 / 84) lose.
+        if (p.tfsf && pml && ty == kTileY && ns == kStages && max_ctas <= 0) xch = std::min(xch, cap_chunk);
     }
     pl->x_chunk = p.x_chunk = (int)std::min<int64_t>(xch, g.nx);
     p.nxc = (int)((g.nx + pl->x_chunk - 1) / pl->x_chunk);
@@ -646,7 +647,7 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     int64_t *off_e = off.data() + (nsims + 1), *off_h = off_e + (nsims + 1);
     const KernelEntry *ke = nullptr;
     int tab_bytes = 0;
-    bool any_drude = false;
+    bool any_drude = false, any_zin = false;  // z terms in the kernel
     const int ty = tile && tile->tile_y ? tile->tile_y : kTileY;
     int chunk = tile ? tile->x_chunk : 0;
     if (ty > 0 && !chunk) {
@@ -679,8 +680,10 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     // z slab, half of all on grids of up to 192 cells, execute twice a plain one's instructions.
     // us a step in the kernel / on bands: 8 grids of 24..96 cells an axis, 1.6 Mcells in all,
     // 97 / 84; 24 of 24..64 (2.1 M) 110 / 105; 64 of 32..192 (80 M) 2022 / 1617; but 8 of 24..64
-    // (0.8 M) 45 / 50 and 4 of 64^3 (1.0 M) 45 / 51, where the launches count
-    const bool bands = cells >= 3 << 19;
+    // (0.8 M) 45 / 50 and 4 of 64^3 (1.0 M) 45 / 51, where the launches count.  Tiles of 4 rows,
+    // a third of whose warps are halo, are faster on bands at any size: 64 of 14..24 (0.4 M) 93 / 71,
+    // with Drude boxes 115 / 92 (the kernels before these 92 and 99)
+    const bool bands = cells >= 3 << 19 || ty == 4;
     // grids with the longest items (x planes per chunk, then tile rows) come first
     std::vector<int32_t> order((size_t)nsims);
     for (int32_t s = 0; s < nsims; s++) order[s] = s;
@@ -699,6 +702,7 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
         if (st != FDTD_OK) return st;
         ke = pl->k;
         any_drude = any_drude || pl->base.drude;
+        any_zin = any_zin || (pl->base.P[2] > 0 && ((pl->base.faces >> 4) & 3) && !pl->base.zfix);
         tab_bytes = std::max(tab_bytes, 6 * 2 * (pl->base.P[0] + pl->base.P[1] + pl->base.P[2]) * 4);
         for (int b = 0; b < 2; b++) {
             Params p = pl->base;
@@ -747,7 +751,7 @@ int fdtd_batch_plan_create(fdtd_batch_plan **out, int32_t nsims, const fdtd_grid
     bp->d_queue = reinterpret_cast<int32_t *>(ws + off_i + off.size() * sizeof(int64_t));
     bp->band_e = off_e[nsims];
     bp->band_h = off_h[nsims];
-    bp->fn = ke->fn_batch[bands ? 0 : 1][any_drude ? 1 : 0];
+    bp->fn = ke->fn_batch[any_zin ? 1 : 0][any_drude ? 1 : 0];
     int nsm = 0, occ = 0;
     const int rs = fused_residency(bp->fn, ke->threads, bp->smem, &nsm, &occ);
     if (rs != FDTD_OK) { delete bp; return rs; }
@@ -803,6 +807,10 @@ int fdtd_batch_plan_info(const fdtd_batch_plan *bp, int32_t *info, int32_t n) {
     info[3] = bp->nblocks;
     info[4] = bp->k->threads;
     info[5] = bp->smem;
+    if (n >= 8) {
+        info[6] = bp->band_h > 0;
+        info[7] = bp->band_h > 0 ? 3 : 1;
+    }
     return FDTD_OK;
 }
 

@@ -325,8 +325,8 @@ int fdtd_symp_pair_plan_set_current(fdtd_symp_plan *plan, int32_t cur);
 int fdtd_symp_pair_plan_destroy(fdtd_symp_plan *plan);
 
 /* ---- batched fused step: many independent grids a launch --------------- */
-/* One launch per step; from 1.5 Mcells on, and with a z face's CPML, two band
- * launches over all grids finish the z slabs. */
+/* One launch per step; from 1.5 Mcells on, or with tiles of 4 rows, and with a
+ * z face's CPML, two band launches over all grids finish the z slabs. */
 /* Every grid keeps its own state, CPML and sources (arrays as for
  * fdtd_yee_plan_create); all grids advance together (same buffer index,
  * same step number).  The per-grid launch parameters and TMA descriptors
@@ -347,7 +347,8 @@ int fdtd_batch_plan_create(fdtd_batch_plan **plan, int32_t nsims, const fdtd_gri
 int fdtd_batch_plan_run(fdtd_batch_plan *plan, int64_t t0, int64_t nsteps, void *stream);
 int fdtd_batch_plan_current(const fdtd_batch_plan *plan);
 int fdtd_batch_plan_set_current(fdtd_batch_plan *plan, int32_t cur);
-/* info[0..5] = tile_y, stages, work items, CTAs launched, threads/CTA, shared bytes/CTA */
+/* info[0..5] = tile_y, stages, work items, CTAs launched, threads/CTA, shared bytes/CTA;
+ * with n >= 8 also info[6], info[7] as fdtd_yee_plan_info */
 int fdtd_batch_plan_info(const fdtd_batch_plan *plan, int32_t *info, int32_t n);
 int fdtd_batch_plan_destroy(fdtd_batch_plan *plan);
 

@@ -58,3 +58,26 @@ def test_x_chunk_with_a_wave(shape, npml, drude, tile, most):
     a, b = (solver(shape, npml, drude, True, tile) for _ in range(2))
     assert a.plan_info()["x_chunk"] == most
     check(a, b)
+
+
+@pytest.mark.parametrize("npml,drude,tile,launches", [(0, True, None, 1), (5, True, (4,), 3), (5, False, (4, 20, 0, 6), 3),
+                                                      (5, True, None, 1)])
+def test_batch_routes(npml, drude, tile, launches):
+    """Small batches: band launches for tiles of 4 rows, none without a z layer."""
+    import ctypes as C
+    import fdtd_accelerate_gb300 as F
+    from fdtd_accelerate_gb300 import _native as N
+    shapes = [(24 + q, 30, 22 + 3 * q) for q in range(8)]
+    a, b = ([solver(sh, npml, drude and q % 2 == 0) for q, sh in enumerate(shapes)] for _ in range(2))
+    batch = F.BatchSolver(a, tile=tile)
+    info = (C.c_int32 * 8)()
+    N.call("fdtd_batch_plan_info", batch.plan(), info, 8)
+    batch.step(1)
+    batch.step(2)
+    torch.cuda.synchronize()
+    batch.check_status()
+    for s, r in zip(a, b):
+        r.step_unfused(3)
+        for k in NAMES:
+            assert torch.equal(s.fields[k], r.fields[k]), k
+    assert info[7] == launches
