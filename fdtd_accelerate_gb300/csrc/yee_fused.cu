@@ -168,11 +168,17 @@ constexpr int kCluster = 8;
 // 51 / 46, 52x162x171 65 / 54, 125x125x130 89 / 73, with a Drude box 104 / 77; with 12
 // cells 256x256x128 186 / 160, 512^3 1739 / 1545.  Rows that are mostly slab lose
 // earlier: 200x200x20 with a Drude box 112 / 70, 1000x60x20 157 / 101 (the kernels before
-// these 104 and 132).  Grids of few (i, j) rows keep the bands' three launches, which
-// plan_info reports and the tests of it expect.
-static bool use_bands(const Grid &g, int slab) {
+// these 104 and 132).  So do launch shapes of the caller's with a Drude box or a wave,
+// fused / bands (the kernels before): 80^3, 4 cells, both, tiles of 4 rows 92 / 67 (69),
+// 60x200x40 92 / 64 (72); a wave and a chunk of 8 planes, 48^3 53 / 46 (49).  Grids of few
+// (i, j) rows keep the bands' three launches, which plan_info reports and the tests of it
+// expect.
+static bool use_bands(const Grid &g, int slab, const fdtd_tile *tile, bool drude, bool tfsf) {
     const int64_t rows = g.nx * g.ny, cells = rows * g.nz;
-    return rows < 2048 || cells >= (2 * slab > g.nz ? 3 << 18 : 13 << 16);
+    const bool own = tile && tile->tile_y != 16 &&  // (tiles of 16 rows: 60x70x90, a Drude box, 26 / 27)
+                     (tile->tile_y || tile->x_chunk || tile->ctas_per_sm > 0 || tile->stages);
+    if (own && tfsf && tile->x_chunk) return true;
+    return rows < 2048 || cells >= (own && (drude || tfsf) ? 5 << 16 : 2 * slab > g.nz ? 3 << 18 : 13 << 16);
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -331,7 +337,9 @@ static int yee_plan_create(fdtd_yee_plan **out, const fdtd_grid *gp, const fdtd_
         p.th1d = t.h1d;
     }
     // the z slab (when a z face has CPML): inside the fused kernel or by the band kernels
-    p.zfix = (p.P[2] > 0 && ((p.faces >> 4) & 3) && (batch_chunk ? batch_bands : use_bands(g, zband_e_row(p)))) ? 1 : 0;
+    p.zfix = 0;
+    if (p.P[2] > 0 && ((p.faces >> 4) & 3))
+        p.zfix = batch_chunk ? batch_bands : use_bands(g, zband_e_row(p), tile, p.drude, p.tfsf);
     // tile rows with y slab cells (rows j0-1 .. j0+ty-1), counted from either end
     if (p.P[1] > 0)
         for (int t = 0; t < p.nty; t++) {

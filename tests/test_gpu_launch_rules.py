@@ -49,6 +49,15 @@ def test_z_slab_route(shape, npml, drude, band):
     check(a, b)
 
 
+@pytest.mark.parametrize("shape,drude,tfsf,tile,band", [
+    ((80, 80, 80), True, True, (4,), 1), ((80, 80, 80), True, False, (4, 0, 0, 4), 1), ((80, 80, 80), True, True, None, 0),
+    ((80, 80, 80), False, False, (4,), 0), ((64, 64, 64), True, True, (4, 0, 0, 6), 0), ((48, 48, 48), False, True, (8, 8), 1)])
+def test_z_slab_route_of_the_callers_launch_shapes(shape, drude, tfsf, tile, band):
+    a, b = (solver(shape, 4, drude, tfsf, tile) for _ in range(2))
+    assert a.plan_info()["z_band"] == band
+    check(a, b)
+
+
 @pytest.mark.parametrize("shape,npml,drude,tile,most", [
     ((180, 180, 180), 4, False, None, 16), ((300, 120, 120), 8, True, None, 16), ((125, 125, 130), 8, False, None, 8),
     ((125, 125, 130), 8, False, (8, 40), 40)])
