@@ -683,7 +683,7 @@ def run_tfsf512(args):
 
 
 def run_batched64(args):
-    """64 ragged grids in one launch per step (autotuned, graph-captured) against
+    """64 ragged grids advanced together (autotuned, graph-captured) against
     the same 64 grids solved one after another with the single-grid path."""
     import torch
     import fdtd_accelerate_gb300 as F
@@ -724,14 +724,14 @@ def run_batched64(args):
     ms_seq = a.elapsed_time(b) / n
     cells = batch.cells
     info = batch.plan_info()
-    # one step = the batched fused launch plus the two batched z-band launches
-    # when any grid has a z face with CPML; bytes summed over the grids
+    # one step = the batched fused launch plus, on batches of this size, two z-band
+    # launches over all grids with CPML on a z face; bytes summed over the grids
     band = any(sv.cpml.active and sv.cpml.npml[2] > 0 for sv in batch.solvers)
     per_step = 3 if band else 1
     alg = sum(algorithmic_bytes_per_step(sv.shape, sv.cpml.npml[0]) for sv in batch.solvers)
     peak, peak_src = measured_peak()
     achieved = alg / (ms_batch / 1e3) / 1e9
-    line = _base_line("Mcell-updates/s (64 ragged Yee+CPML grids, one launch per step, FP32)",
+    line = _base_line("Mcell-updates/s (64 ragged Yee+CPML grids advanced together, FP32)",
                       cells / (ms_batch / 1e3) / 1e6, UNIT, args, ms_batch, "f32",
                       "64 grids, axes from {32..192 step 16}, 8-cell CPML, 10 spheres eps_r U[1,8] each, Ez "
                       "centre source; %d steps captured in one CUDA graph; %d cells in all" % (n, cells),

@@ -5,7 +5,8 @@ The reference runs one simulation per process and time loop (e.g.
 BatchSolver keeps a list of YeeSolver grids of any (uneven) sizes and
 advances all of them with the batched fused kernel: the work items of every
 grid (z tile x y tile x x chunk) form one list that the persistent CTAs walk (from
-1.5 Mcells on, two more launches finish the z CPML slabs of all grids),
+1.5 Mcells on, and with tiles of 4 rows, two more launches finish the z CPML slabs of
+all grids),
 so small grids that would leave most SMs idle on their own fill the GPU
 together.  Each grid's result is bit-identical to its own YeeSolver.step.
 

@@ -11,7 +11,9 @@
 // thread -> edge kernels) 64^3 98 -> 75.  Rows of psi that are no 16-byte
 // multiple are read and written one cell at a time, 4 lines an instruction, and
 // gain nothing (300x301x303: 2210 and 2213).  As the in-place stage kernel
-// (k_symp_stage) the group form was slower, 1714 -> 1865 at 256^3.
+// (k_symp_stage) the group form was slower, 1714 -> 1865 at 256^3.  All of it with
+// the fields through the read-only path; with plain loads (ldf) 64^3 76 -> 76, 128^3
+// with 8 cells 267 -> 274, 512^3 8140 -> 8170.
 //
 // H nodes take a backward stencil (offsets -2 .. 1), E nodes a forward one
 // (-1 .. 2); with that, both have the same form.  G: the field that is read.

@@ -15,12 +15,13 @@
 //    (only their owner touches them).
 //  * Split: the pair kernel owns rows [j_lo, j_hi) and columns [k_lo, k_hi),
 //    every x plane, with j_lo = P+2 and j_hi = ny-P-2 (and the same along z,
-//    k_lo rounded up to 4): E_new there needs H_new of rows j_lo-1 .. j_hi+1,
-//    where no y or z CPML node lies.  So the pair kernel carries the x-slab
-//    terms only.  The rest of the grid (the y and z slabs plus two cells) is
-//    the edge shell, advanced by kernels of 4 cells a thread (k_edge_*), out
-//    of place; their E stage runs after the pair kernel has written the inside
-//    H_new.  Small grids are all shell.
+//    k_lo rounded up and k_hi down to 16): E_new there needs H_new of rows
+//    j_lo-1 .. j_hi+1, where no y or z CPML node lies.  So the pair kernel
+//    carries the x-slab terms only.  The rest of the grid (the y slabs plus two
+//    rows, the z slabs plus two columns in steps of 16) is the edge shell,
+//    advanced by kernels of 4 cells a thread (k_edge_*), out of place; their E
+//    stage runs after the pair kernel has written the inside H_new.  Small
+//    grids are all shell.
 //  * Pair kernel, 2.5-D blocking: a CTA owns TZ = 32 (z) x TY = 16 (y) cells
 //    for a chunk of x planes and marches along x.  E_new(i) needs H_new on
 //    planes i-1 .. i+2 and on the rows/columns -1 .. +2 around the tile, so
@@ -709,8 +710,9 @@ k_symp_pair(const __grid_constant__ Maps mk, const __grid_constant__ Params p) {
 }
 
 // ---------------------------------------------------------------------------
-// Edge shell: the cells outside the pair kernel's tiles (the y and z CPML
-// slabs and a tile of margin), 4 z cells a thread (symp_group.cuh), out of place:
+// Edge shell: the cells outside the pair kernel's region (P+2 rows at a y face, P+2
+// columns and up to 15 more at a z face; the whole of a small grid), 4 z cells a
+// thread (symp_group.cuh), out of place:
 //   k_edge_h         H_out = H_in - clch_a curl4(E_in) with its CPML terms
 //                    (psi_h_in -> psi_h_out); in a two-H pass the second
 //                    stage follows in registers (same E_in, psi carried);

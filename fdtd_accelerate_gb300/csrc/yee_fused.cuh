@@ -1125,7 +1125,7 @@ k_yee_fused(const __grid_constant__ TMaps mk, const __grid_constant__ Params pk,
 
 
 // ---------------------------------------------------------------------------
-// z band kernels (single-grid plans).  The fused kernel treats z-slab tiles
+// z band kernels (single-grid and batched plans).  The fused kernel treats z-slab tiles
 // like interior tiles; these two kernels then finish the band in the same
 // operation order as the in-kernel path (and the reference's cpml_e/cpml_h):
 //   E: on E z-slab nodes, psi_e(z) update and E correction, then the sources
