@@ -12,8 +12,8 @@
 // multiple are read and written one cell at a time, 4 lines an instruction, and
 // gain nothing (300x301x303: 2210 and 2213).  As the in-place stage kernel
 // (k_symp_stage) the group form was slower, 1714 -> 1865 at 256^3.  All of it with
-// the fields through the read-only path; with plain loads (ldf) 64^3 76 -> 76, 128^3
-// with 8 cells 267 -> 274, 512^3 8140 -> 8170.
+// the fields through the read-only path; with plain loads (chained launches) 64^3 76 -> 76,
+// 128^3 with 8 cells 267 -> 274, 512^3 8140 -> 8170.
 //
 // H nodes take a backward stencil (offsets -2 .. 1), E nodes a forward one
 // (-1 .. 2); with that, both have the same form.  G: the field that is read.
@@ -38,6 +38,11 @@ struct Tab {
     const float *b, *a, *km1;
 };
 
+template <bool RO, typename T>
+__device__ __forceinline__ T ld1(const T *p) {
+    return RO ? __ldg(p) : *p;
+}
+
 // slab index of node x of n along an axis with P cells a face, -1 outside
 template <bool E>
 __device__ __forceinline__ int slab(int P, bool front, bool back, int x, int n) {
@@ -60,10 +65,25 @@ struct Group {
         : nx(nx_), ny(ny_), nz(nz_), X(sx), Y(sy), i(i_), j(j_), k(k_),
           c((uint32_t)i_ * sx + (uint32_t)j_ * sy + (uint32_t)k_), in(k_ + 4 <= nz_ ? 0xFu : (1u << (nz_ - k_)) - 1),
           n((int64_t)nx_ * sx) {}
-    // the group at offset at of a field.  (A plain load, as all of a chained kernel's but
-    // the table entries: the launch before may write the field while this one is resident,
-    // and the read-only path is for memory that nothing writes in that time.)
-    __device__ __forceinline__ F4 ldf(const float *f, uint32_t at) const { return ld(f, at, in, true, n); }
+    // the group at offset at of a field, RO: through the read-only path.  A chained kernel
+    // takes plain loads: the launch before may write the field while this one is resident,
+    // and the read-only path is for memory that nothing writes in that time.
+    template <bool RO>
+    __device__ __forceinline__ F4 ldf(const float *f, uint32_t at) const {
+        if (!RO) return ld(f, at, in, true, n);
+        F4 r{};
+        if (in == 0xFu) {
+            if (FDTD_IN(at, n) && FDTD_IN(at + 3, n)) {
+                const float4 t = ld1<RO>(reinterpret_cast<const float4 *>(f + at));
+                r = F4{{t.x, t.y, t.z, t.w}};
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (((in >> e) & 1) && FDTD_IN(at + e, n)) r.v[e] = ld1<RO>(f + at + e);
+        }
+        return r;
+    }
     // elements at .. at+3 of a psi array or of the updated field, those of mask m
     __device__ static __forceinline__ F4 ld(const float *f, uint32_t at, uint32_t m, bool vec, int64_t ext) {
         F4 r{};
@@ -90,36 +110,36 @@ struct Group {
         }
     }
     // stencil along x or y (stride s); the rows must exist
-    template <bool E>
+    template <bool E, bool RO>
     __device__ __forceinline__ Window rows(const float *f, uint32_t s) const {
-        return E ? Window{ldf(f, c - s), ldf(f, c), ldf(f, c + s), ldf(f, c + 2 * s)}
-                 : Window{ldf(f, c - 2 * s), ldf(f, c - s), ldf(f, c), ldf(f, c + s)};
+        return E ? Window{ldf<RO>(f, c - s), ldf<RO>(f, c), ldf<RO>(f, c + s), ldf<RO>(f, c + 2 * s)}
+                 : Window{ldf<RO>(f, c - 2 * s), ldf<RO>(f, c - s), ldf<RO>(f, c), ldf<RO>(f, c + s)};
     }
     // stencil along z; past either end of the row the values are zeros that no updated cell uses
-    template <bool E>
+    template <bool E, bool RO>
     __device__ __forceinline__ Window along_z(const float *f) const {
-        const F4 o = ldf(f, c);
+        const F4 o = ldf<RO>(f, c);
         if (E) {
-            const float l = k > 0 && FDTD_IN(c - 1, n) ? f[c - 1] : 0.f;
+            const float l = k > 0 && FDTD_IN(c - 1, n) ? ld1<RO>(f + c - 1) : 0.f;
             float r0 = 0.f, r1 = 0.f;
             if (k + 5 < nz) {
                 if (FDTD_IN(c + 5, n)) {
-                    const float2 t = *reinterpret_cast<const float2 *>(f + c + 4);
+                    const float2 t = ld1<RO>(reinterpret_cast<const float2 *>(f + c + 4));
                     r0 = t.x;
                     r1 = t.y;
                 }
             } else if (k + 4 < nz && FDTD_IN(c + 4, n)) {
-                r0 = f[c + 4];
+                r0 = ld1<RO>(f + c + 4);
             }
             return Window{{{l, o.v[0], o.v[1], o.v[2]}}, o, {{o.v[1], o.v[2], o.v[3], r0}}, {{o.v[2], o.v[3], r0, r1}}};
         }
         float l0 = 0.f, l1 = 0.f;
         if (k > 0 && FDTD_IN(c - 2, n)) {
-            const float2 t = *reinterpret_cast<const float2 *>(f + c - 2);
+            const float2 t = ld1<RO>(reinterpret_cast<const float2 *>(f + c - 2));
             l0 = t.x;
             l1 = t.y;
         }
-        const float r = k + 4 < nz && FDTD_IN(c + 4, n) ? f[c + 4] : 0.f;
+        const float r = k + 4 < nz && FDTD_IN(c + 4, n) ? ld1<RO>(f + c + 4) : 0.f;
         return Window{{{l0, l1, o.v[0], o.v[1]}}, {{l1, o.v[0], o.v[1], o.v[2]}}, o, {{o.v[1], o.v[2], o.v[3], r}}};
     }
 };
@@ -135,6 +155,7 @@ __device__ __forceinline__ float diff4(const Window &w, int e) {
 //   P(ax), front(ax), back(ax), tab(st, ax), coef(st)
 //   cv(q, grp)              coefficient of the cells
 //   main(st, v, cv, d27)    the stage's main term
+//   RO                      fields that are only read go through the read-only path
 template <bool E, int NST, class Ctx>
 __device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
     auto inside = [](int v, int n) { return E ? v > 0 && v < n - 2 : v > 1 && v < n - 1; };
@@ -229,19 +250,19 @@ __device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
         Group::st(x.fout(q), g.c, g.in, true, Group::ld(x.fin(q), g.c, g.in, true, g.n), g.n);
     };
     if (jin && km) {
-        const Window p = g.rows<E>(x.g(2), g.Y), w = g.along_z<E>(x.g(1));
+        const Window p = g.template rows<E, Ctx::RO>(x.g(2), g.Y), w = g.template along_z<E, Ctx::RO>(x.g(1));
         comp(0, km, p, w, 1, 3, p, E, 2, 4, w);
     } else {
         copy(0);
     }
     if (iin && km) {
-        const Window p = g.along_z<E>(x.g(0)), w = g.rows<E>(x.g(2), g.X);
+        const Window p = g.template along_z<E, Ctx::RO>(x.g(0)), w = g.template rows<E, Ctx::RO>(x.g(2), g.X);
         comp(1, km, p, w, 0, 0, w, !E, 2, 5, p);
     } else {
         copy(1);
     }
     if (iin && jin) {
-        const Window p = g.rows<E>(x.g(1), g.X), w = g.rows<E>(x.g(0), g.Y);
+        const Window p = g.template rows<E, Ctx::RO>(x.g(1), g.X), w = g.template rows<E, Ctx::RO>(x.g(0), g.Y);
         comp(2, g.in, p, w, 0, 1, p, E, 1, 2, w);
     } else {
         copy(2);

@@ -751,8 +751,9 @@ __device__ __forceinline__ bool edge_group(const Edge &eb, int &i, int &j, int &
 }
 
 // the edge kernels' stages (sg::stage): E or the H stages a, b of a pass
-template <bool E>
+template <bool E, bool READ_ONLY>
 struct EdgeStage {
+    static constexpr bool RO = READ_ONLY;
     const Params &p;
     __device__ __forceinline__ const Axis &axis(int st, int ax) const { return E ? p.ea[ax] : st ? p.hb[ax] : p.ha[ax]; }
     __device__ __forceinline__ const float *fin(int q) const { return p.in[(E ? 0 : 3) + q]; }
@@ -770,30 +771,32 @@ struct EdgeStage {
     }
     __device__ __forceinline__ float coef(int st) const { return E ? p.dl : st ? p.cl_b : p.cl_a; }
     __device__ __forceinline__ sg::F4 cv(int q, const sg::Group &g) const {
-        return E ? g.ldf(p.ce[q], g.c) : sg::F4{{p.ch, p.ch, p.ch, p.ch}};
+        return E ? g.template ldf<RO>(p.ce[q], g.c) : sg::F4{{p.ch, p.ch, p.ch, p.ch}};
     }
     __device__ __forceinline__ float main(int st, float v, float cv, float d27) const {
         return E ? fadd(v, fmul(fmul(p.dl, cv), d27)) : fsub(v, fmul(st ? p.clch_b : p.clch_a, d27));
     }
 };
 
-template <bool HH>
+// RO: the launch is not chained (see Group::ldf)
+template <bool HH, bool RO>
 __global__ void __launch_bounds__(EDGE_BLOCK)
 k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     grid_wait();
     grid_release();
     int i, j, k;
     if (!edge_group(eb, i, j, k)) return;
-    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false>{p});
+    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false, RO>{p});
 }
 
+template <bool RO>
 __global__ void __launch_bounds__(EDGE_BLOCK)
 k_edge_e(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     grid_wait();
     grid_release();
     int i, j, k;
     if (!edge_group(eb, i, j, k)) return;
-    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true>{p});
+    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true, RO>{p});
 }
 
 // Soft sources on edge cells, as a walk of the list in order would add them: a thread a
@@ -1204,16 +1207,17 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
     if (egroups > 0) {
         const dim3 nb((unsigned)((egroups + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx);
         const cudaStream_t hs = beside ? pl->side : st;
-        if (two_h)
-            launch(chained, k_edge_h<true>, nb, EDGE_BLOCK, 0, hs, p, eb);
+        if (chained)
+            launch(true, two_h ? k_edge_h<true, false> : k_edge_h<false, false>, nb, EDGE_BLOCK, 0, hs, p, eb);
         else
-            launch(chained, k_edge_h<false>, nb, EDGE_BLOCK, 0, hs, p, eb);
+            launch(false, two_h ? k_edge_h<true, true> : k_edge_h<false, true>, nb, EDGE_BLOCK, 0, hs, p, eb);
         if (beside) {
             cudaError_t e = cudaEventRecord(pl->join, hs);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(st, pl->join, 0);
             if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
         }
-        launch(chained, k_edge_e, nb, EDGE_BLOCK, 0, st, p, eb);
+        if (chained) launch(true, k_edge_e<false>, nb, EDGE_BLOCK, 0, st, p, eb);
+        else launch(false, k_edge_e<true>, nb, EDGE_BLOCK, 0, st, p, eb);
         bool esrc = false;
         for (size_t a = 0; a + 2 < pl->src_ijk.size(); a += 3)
             for (int b = 0; b < eb.n; b++)

@@ -72,8 +72,19 @@ def test_read_only_loads_of_tables_alone(name):
     is resident: only the CPML tables (and a wave's 1-D arrays) go through __ldg."""
     text = source(os.path.join(CSRC, name))
     assert not re.search(r"#define[^\n]*__ldg|ld\.global\.nc", text)
+    text = text.replace("return RO ? __ldg(p) : *p;", "")  # the edge kernels' loads, below
     for arg in re.findall(r"__ldg\(([^;]*)", text):
         assert re.match(r"T\.(b|a|km1) \+ s", arg) or (name == "yee_fused.cuh" and arg.startswith("f1d + at")), arg
+
+
+def test_edge_kernels_of_chained_launches():
+    """The edge kernels' read-only forms are launched the plain way."""
+    text = source(os.path.join(CSRC, "symp_pair.cu"))
+    forms = re.findall(r"launch\((\w+), ([^;]*k_edge_[he][^;]*);", text)
+    assert len(forms) == 4
+    for chained, kernel in forms:
+        ro = set(re.findall(r"k_edge_h<\w+, (\w+)>|k_edge_e<(\w+)>", kernel))
+        assert {a or b for a, b in ro} == {{"true": "false", "false": "true"}[chained]}, kernel
 
 
 def test_one_dimensional_arrays_of_a_wave():
