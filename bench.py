@@ -59,10 +59,10 @@ FALLBACK_HBM_GBS = 6790.7
 NCU_FUSED_DRAM_BYTES_PER_CELL = 63.2
 NCU_BAND_DRAM_BYTES_PER_BAND_CELL = 192.9
 # The plain 128^3 step (one fused launch, no CPML): DRAM bytes of one launch
-# after an L2 flush, from an ncu capture of that workload (three launches,
-# within 2 %); part of the 50 MB of field writes is still in L2 when the
-# launch ends, so the write count is low.
-NCU_PLAIN128_DRAM_BYTES = 92.9e6
+# after an L2 flush, from an ncu capture of that workload (three launches, 81.0
+# read and 8.1 .. 11.2 MB written); most of the 50 MB of field writes is still in
+# L2 when the launch ends, so the write count is low.
+NCU_PLAIN128_DRAM_BYTES = 90.2e6
 
 
 def step_traffic_bytes(shape, npml):
