@@ -530,7 +530,7 @@ def run_symp512(args):
     alg_pair = symplectic_pair_bytes_per_step(shape, npml)
     alg_fused = algorithmic_bytes_per_step(shape, npml)
     peak, psrc = measured_peak()
-    pair = s.pair_path()
+    pair = s._runs_pairs(args.steps)
     # the roofline of the path that ran: the stage-pair byte count (four passes
     # of 60 B/cell) or the stage-by-stage one (372 B/cell)
     alg_run = alg_pair if pair else alg

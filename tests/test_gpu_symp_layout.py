@@ -154,3 +154,19 @@ def test_two_h_stages_of_unlike_layers_are_refused():
     torch.cuda.synchronize()
     for k in NAMES:
         assert torch.equal(s.fields[k], before[k]), k
+
+
+def test_pairs_and_stages_by_turns():
+    """Long and short calls of one solver on odd rows, with an x layer (psi of both
+    paths) and edits of the fields between the calls."""
+    shape, npml = (20, 40, 45), (5, 0, 0)
+    a, b = (solver(shape, coefs(shape), npml=npml, fused=fused, max_steps=400) for fused in (True, False))
+    for n in (3, 128, 1, 129, 2):
+        for s in (a, b):
+            s.step(n)
+            s.fields["ey"].mul_(0.5)
+    assert a._plan_ready()
+    assert_same(a, b)
+    for q in range(2):
+        assert torch.equal(a.cpml.psi_e[q], b.cpml.psi_e[q]) and torch.equal(a.cpml.psi_h[q], b.cpml.psi_h[q])
+    a.check_status()
