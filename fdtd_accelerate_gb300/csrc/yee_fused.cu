@@ -170,15 +170,19 @@ constexpr int kCluster = 8;
 // earlier: 200x200x20 with a Drude box 112 / 70, 1000x60x20 157 / 101 (the kernels before
 // these 104 and 132).  So do launch shapes of the caller's with a Drude box or a wave,
 // fused / bands (the kernels before): 80^3, 4 cells, both, tiles of 4 rows 92 / 67 (69),
-// 60x200x40 92 / 64 (72); a wave and a chunk of 8 planes, 48^3 53 / 46 (49).  Grids of few
-// (i, j) rows keep the bands' three launches, which plan_info reports and the tests of it
-// expect.
+// 60x200x40 92 / 64 (72); a wave and a chunk of 8 planes, 48^3 53 / 46 (49); and so do
+// long chunks on their own, whose items march many planes at a plane's latency: 64^3 with
+// 8 cells, chunks of 31 109 / 77 (86), 57x100x124 84 / 46 (60).  Grids of few (i, j) rows
+// keep the bands' three launches, which plan_info reports and the tests of it expect, and
+// so does one chunk on grids below 393 kcells keep its one launch.
 static bool use_bands(const Grid &g, int slab, const fdtd_tile *tile, bool drude, bool tfsf) {
     const int64_t rows = g.nx * g.ny, cells = rows * g.nz;
     const bool own = tile && tile->tile_y != 16 &&  // (tiles of 16 rows: 60x70x90, a Drude box, 26 / 27)
                      (tile->tile_y || tile->x_chunk || tile->ctas_per_sm > 0 || tile->stages);
-    if (own && tfsf && tile->x_chunk) return true;
-    return rows < 2048 || cells >= (own && (drude || tfsf) ? 5 << 16 : 2 * slab > g.nz ? 3 << 18 : 13 << 16);
+    if (own && tile->x_chunk && (tfsf || tile->x_chunk >= 8))
+        return tfsf || drude || rows < 2048 || tile->x_chunk < g.nx || cells >= 3 << 17;
+    const int line = own && (drude || tfsf) ? 5 << 16 : own && !tile->x_chunk ? 3 << 17 : 2 * slab > g.nz ? 3 << 18 : 13 << 16;
+    return rows < 2048 || cells >= line;
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

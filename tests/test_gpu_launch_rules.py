@@ -51,7 +51,9 @@ def test_z_slab_route(shape, npml, drude, band):
 
 @pytest.mark.parametrize("shape,drude,tfsf,tile,band", [
     ((80, 80, 80), True, True, (4,), 1), ((80, 80, 80), True, False, (4, 0, 0, 4), 1), ((80, 80, 80), True, True, None, 0),
-    ((80, 80, 80), False, False, (4,), 0), ((64, 64, 64), True, True, (4, 0, 0, 6), 0), ((48, 48, 48), False, True, (8, 8), 1)])
+    ((70, 72, 72), False, False, (4,), 0), ((80, 80, 80), False, False, (4,), 1), ((64, 64, 64), True, True, (4, 0, 0, 6), 0),
+    ((48, 48, 48), False, True, (8, 8), 1), ((64, 64, 64), False, False, (8, 31), 1), ((57, 100, 124), False, False, (8, 64), 1),
+    ((48, 48, 48), False, False, (8, 48), 0), ((48, 48, 48), True, False, (8, 48), 1), ((64, 64, 64), False, False, (8, 7), 0)])
 def test_z_slab_route_of_the_callers_launch_shapes(shape, drude, tfsf, tile, band):
     a, b = (solver(shape, 4, drude, tfsf, tile) for _ in range(2))
     assert a.plan_info()["z_band"] == band
