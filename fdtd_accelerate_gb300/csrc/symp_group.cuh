@@ -11,9 +11,9 @@
 // thread -> edge kernels) 64^3 98 -> 75.  Rows of psi that are no 16-byte
 // multiple are read and written one cell at a time, 4 lines an instruction, and
 // gain nothing (300x301x303: 2210 and 2213).  As the in-place stage kernel
-// (k_symp_stage) the group form was slower, 1714 -> 1865 at 256^3.  All of it with
-// the fields through the read-only path; with plain loads (chained launches) 64^3 76 -> 76,
-// 128^3 with 8 cells 267 -> 274, 512^3 8140 -> 8170.
+// (k_symp_stage) the group form was slower, 1714 -> 1865 at 256^3.  With each
+// component's results gathered before its stores (Out) 512^3 8158 -> 8096 and 200^3 with 8 cells
+// 823 -> 768; 128^3, through plain loads, 266 where the read-only path took 267.
 //
 // H nodes take a backward stencil (offsets -2 .. 1), E nodes a forward one
 // (-1 .. 2); with that, both have the same form.  G: the field that is read.
@@ -156,6 +156,7 @@ __device__ __forceinline__ float diff4(const Window &w, int e) {
 //   cv(q, grp)              coefficient of the cells
 //   main(st, v, cv, d27)    the stage's main term
 //   RO                      fields that are only read go through the read-only path
+//   LAST                    all stores after all loads
 template <bool E, int NST, class Ctx>
 __device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
     auto inside = [](int v, int n) { return E ? v > 0 && v < n - 2 : v > 1 && v < n - 1; };
@@ -221,14 +222,16 @@ __device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
     };
     // component q from windows p and w (curl of p minus curl of w); CPML terms of the axes ax1
     // (window w1, psi array a1, added when add1) and then ax2
+    struct Out {
+        F4 v, s1, s2;
+        uint32_t m1, m2;
+    };
     auto comp = [&](int q, uint32_t upd, const Window &p, const Window &w, int ax1, int a1, const Window &w1, bool add1,
                     int ax2, int a2, const Window &w2) {
-        F4 v = Group::ld(x.fin(q), g.c, g.in, true, g.n);
+        Out o{Group::ld(x.fin(q), g.c, g.in, true, g.n), F4{}, F4{}, pmask(ax1, upd), pmask(ax2, upd)};
         const F4 cv = x.cv(q, g);
-        const uint32_t m1 = pmask(ax1, upd), m2 = pmask(ax2, upd);
-        F4 s1{}, s2{};
-        if (m1) s1 = pload(ax1, a1, m1);
-        if (m2) s2 = pload(ax2, a2, m2);
+        if (o.m1) o.s1 = pload(ax1, a1, o.m1);
+        if (o.m2) o.s2 = pload(ax2, a2, o.m2);
         F4 d27;
 #pragma unroll
         for (int e = 0; e < 4; e++)
@@ -238,35 +241,48 @@ __device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
         for (int st = 0; st < NST; st++) {
 #pragma unroll
             for (int e = 0; e < 4; e++)
-                if ((upd >> e) & 1) v.v[e] = x.main(st, v.v[e], cv.v[e], d27.v[e]);
-            term(st, ax1, m1, v, s1, w1, cv, add1);
-            term(st, ax2, m2, v, s2, w2, cv, !add1);
+                if ((upd >> e) & 1) o.v.v[e] = x.main(st, o.v.v[e], cv.v[e], d27.v[e]);
+            term(st, ax1, o.m1, o.v, o.s1, w1, cv, add1);
+            term(st, ax2, o.m2, o.v, o.s2, w2, cv, !add1);
         }
-        if (m1) pstore(ax1, a1, m1, s1);
-        if (m2) pstore(ax2, a2, m2, s2);
-        Group::st(x.fout(q), g.c, g.in, true, v, g.n);
+        return o;
     };
-    auto copy = [&](int q) {
-        Group::st(x.fout(q), g.c, g.in, true, Group::ld(x.fin(q), g.c, g.in, true, g.n), g.n);
+    auto copy = [&](int q) { return Out{Group::ld(x.fin(q), g.c, g.in, true, g.n), F4{}, F4{}, 0u, 0u}; };
+    auto store = [&](int q, const Out &o, int ax1, int a1, int ax2, int a2) {
+        if (o.m1) pstore(ax1, a1, o.m1, o.s1);
+        if (o.m2) pstore(ax2, a2, o.m2, o.s2);
+        Group::st(x.fout(q), g.c, g.in, true, o.v, g.n);
     };
+    // LAST: all stores after all loads.  A store could alias a later load as far as the
+    // compiler knows, so that with plain loads the components follow each other: 33x14x156
+    // with 6 cells 75 -> 69 us a step.  It takes 104 registers instead of 78, and larger grids
+    // lose more by that: 96^3 with 8 cells 123 -> 150, 128^3 266 -> 367.
+    Out o0, o1, o2;
     if (jin && km) {
         const Window p = g.template rows<E, Ctx::RO>(x.g(2), g.Y), w = g.template along_z<E, Ctx::RO>(x.g(1));
-        comp(0, km, p, w, 1, 3, p, E, 2, 4, w);
+        o0 = comp(0, km, p, w, 1, 3, p, E, 2, 4, w);
     } else {
-        copy(0);
+        o0 = copy(0);
     }
+    if (!Ctx::LAST) store(0, o0, 1, 3, 2, 4);
     if (iin && km) {
         const Window p = g.template along_z<E, Ctx::RO>(x.g(0)), w = g.template rows<E, Ctx::RO>(x.g(2), g.X);
-        comp(1, km, p, w, 0, 0, w, !E, 2, 5, p);
+        o1 = comp(1, km, p, w, 0, 0, w, !E, 2, 5, p);
     } else {
-        copy(1);
+        o1 = copy(1);
     }
+    if (!Ctx::LAST) store(1, o1, 0, 0, 2, 5);
     if (iin && jin) {
         const Window p = g.template rows<E, Ctx::RO>(x.g(1), g.X), w = g.template rows<E, Ctx::RO>(x.g(0), g.Y);
-        comp(2, g.in, p, w, 0, 1, p, E, 1, 2, w);
+        o2 = comp(2, g.in, p, w, 0, 1, p, E, 1, 2, w);
     } else {
-        copy(2);
+        o2 = copy(2);
     }
+    if (Ctx::LAST) {
+        store(0, o0, 1, 3, 2, 4);
+        store(1, o1, 0, 0, 2, 5);
+    }
+    store(2, o2, 0, 1, 1, 2);
 }
 
 }  // namespace sg

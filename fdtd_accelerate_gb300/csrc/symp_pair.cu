@@ -751,9 +751,12 @@ __device__ __forceinline__ bool edge_group(const Edge &eb, int &i, int &j, int &
 }
 
 // the edge kernels' stages (sg::stage): E or the H stages a, b of a pass
-template <bool E, bool READ_ONLY>
+// FORM of the edge kernels: READ_ONLY for launches that are not chained (see Group::ldf),
+// PLAIN and PLAIN_LAST (see sg::stage) for chained ones
+constexpr int READ_ONLY = 0, PLAIN = 1, PLAIN_LAST = 2;
+template <bool E, int FORM>
 struct EdgeStage {
-    static constexpr bool RO = READ_ONLY;
+    static constexpr bool RO = FORM == READ_ONLY, LAST = FORM == PLAIN_LAST;
     const Params &p;
     __device__ __forceinline__ const Axis &axis(int st, int ax) const { return E ? p.ea[ax] : st ? p.hb[ax] : p.ha[ax]; }
     __device__ __forceinline__ const float *fin(int q) const { return p.in[(E ? 0 : 3) + q]; }
@@ -778,25 +781,24 @@ struct EdgeStage {
     }
 };
 
-// RO: the launch is not chained (see Group::ldf)
-template <bool HH, bool RO>
+template <bool HH, int FORM>
 __global__ void __launch_bounds__(EDGE_BLOCK)
 k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     grid_wait();
     grid_release();
     int i, j, k;
     if (!edge_group(eb, i, j, k)) return;
-    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false, RO>{p});
+    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false, FORM>{p});
 }
 
-template <bool RO>
+template <int FORM>
 __global__ void __launch_bounds__(EDGE_BLOCK)
 k_edge_e(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     grid_wait();
     grid_release();
     int i, j, k;
     if (!edge_group(eb, i, j, k)) return;
-    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true, RO>{p});
+    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true, FORM>{p});
 }
 
 // Soft sources on edge cells, as a walk of the list in order would add them: a thread a
@@ -1189,7 +1191,7 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
     // own stream (neither reads what the other writes; k_edge_e reads both), and the passes
     // of a pair or edge kernel alone are chained, which hides the gaps between launches.
     // us a step with an 8-cell CPML, one after the other / beside: 164^3 626 / 517, 200^3
-    // 910 / 782 (launched the plain way 842).  Pair kernels that fill the GPU lose to their
+    // 910 / 768 (launched the plain way 842).  Pair kernels that fill the GPU lose to their
     // company (256^3 1373 -> 1418, 512^3 8255 -> 8640).
     const bool beside = pl->side && items > 0 && egroups > 0, chained = leaves_room(pl->g) && !beside;
     if (beside) {
@@ -1207,17 +1209,22 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
     if (egroups > 0) {
         const dim3 nb((unsigned)((egroups + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx);
         const cudaStream_t hs = beside ? pl->side : st;
-        if (chained)
-            launch(true, two_h ? k_edge_h<true, false> : k_edge_h<false, false>, nb, EDGE_BLOCK, 0, hs, p, eb);
+        const bool tiny = cells <= 1 << 19;  // (64^3 with 8 cells 77 / 76 us a step, 96^3 123 / 150)
+        if (chained && tiny)
+            launch(true, two_h ? k_edge_h<true, PLAIN_LAST> : k_edge_h<false, PLAIN_LAST>, nb, EDGE_BLOCK, 0, hs, p, eb);
+        else if (chained)
+            launch(true, two_h ? k_edge_h<true, PLAIN> : k_edge_h<false, PLAIN>, nb, EDGE_BLOCK, 0, hs, p, eb);
         else
-            launch(false, two_h ? k_edge_h<true, true> : k_edge_h<false, true>, nb, EDGE_BLOCK, 0, hs, p, eb);
+            launch(false, two_h ? k_edge_h<true, READ_ONLY> : k_edge_h<false, READ_ONLY>, nb, EDGE_BLOCK, 0, hs, p, eb);
         if (beside) {
             cudaError_t e = cudaEventRecord(pl->join, hs);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(st, pl->join, 0);
             if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
         }
-        if (chained) launch(true, k_edge_e<false>, nb, EDGE_BLOCK, 0, st, p, eb);
-        else launch(false, k_edge_e<true>, nb, EDGE_BLOCK, 0, st, p, eb);
+        if (chained)
+            launch(true, tiny ? k_edge_e<PLAIN_LAST> : k_edge_e<PLAIN>, nb, EDGE_BLOCK, 0, st, p, eb);
+        else
+            launch(false, k_edge_e<READ_ONLY>, nb, EDGE_BLOCK, 0, st, p, eb);
         bool esrc = false;
         for (size_t a = 0; a + 2 < pl->src_ijk.size(); a += 3)
             for (int b = 0; b < eb.n; b++)

@@ -81,10 +81,11 @@ def test_edge_kernels_of_chained_launches():
     """The edge kernels' read-only forms are launched the plain way."""
     text = source(os.path.join(CSRC, "symp_pair.cu"))
     forms = re.findall(r"launch\((\w+), ([^;]*k_edge_[he][^;]*);", text)
-    assert len(forms) == 4
+    assert len(forms) == 5
     for chained, kernel in forms:
-        ro = set(re.findall(r"k_edge_h<\w+, (\w+)>|k_edge_e<(\w+)>", kernel))
-        assert {a or b for a, b in ro} == {{"true": "false", "false": "true"}[chained]}, kernel
+        names = set(re.findall(r"k_edge_h<\w+, (\w+)>", kernel) + re.findall(r"k_edge_e<(\w+)>", kernel))
+        assert names and names <= {"true": {"PLAIN", "PLAIN_LAST"}, "false": {"READ_ONLY"}}[chained], kernel
+    assert re.search(r"RO = FORM == READ_ONLY,", text)
 
 
 def test_one_dimensional_arrays_of_a_wave():
