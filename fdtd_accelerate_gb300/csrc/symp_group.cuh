@@ -12,8 +12,8 @@
 // multiple are read and written one cell at a time, 4 lines an instruction, and
 // gain nothing (300x301x303: 2210 and 2213).  As the in-place stage kernel
 // (k_symp_stage) the group form was slower, 1714 -> 1865 at 256^3.  With each
-// component's results gathered before its stores (Out) 512^3 8158 -> 8096 and 200^3 with 8 cells
-// 823 -> 768; 128^3, through plain loads, 266 where the read-only path took 267.
+// component's results gathered before its stores (Out) 512^3 8142 -> 8096 and 200^3 with 8 cells
+// 782 -> 768; 128^3, through plain loads, 266 where the read-only path took 267.
 //
 // H nodes take a backward stencil (offsets -2 .. 1), E nodes a forward one
 // (-1 .. 2); with that, both have the same form.  G: the field that is read.
