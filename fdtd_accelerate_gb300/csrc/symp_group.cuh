@@ -156,9 +156,9 @@ __device__ __forceinline__ float diff4(const Window &w, int e) {
 //   cv(q, grp)              coefficient of the cells
 //   main(st, v, cv, d27)    the stage's main term
 //   RO                      fields that are only read go through the read-only path
-//   LAST                    all stores after all loads
+//   SPLIT                   the thread advances component `only`, else all three
 template <bool E, int NST, class Ctx>
-__device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
+__device__ __forceinline__ void stage(const Group &g, const Ctx &x, int only) {
     auto inside = [](int v, int n) { return E ? v > 0 && v < n - 2 : v > 1 && v < n - 1; };
     const bool iin = inside(g.i, g.nx), jin = inside(g.j, g.ny);
     const int sx = slab<E>(x.P(0), x.front(0), x.back(0), g.i, g.nx);
@@ -253,36 +253,35 @@ __device__ __forceinline__ void stage(const Group &g, const Ctx &x) {
         if (o.m2) pstore(ax2, a2, o.m2, o.s2);
         Group::st(x.fout(q), g.c, g.in, true, o.v, g.n);
     };
-    // LAST: all stores after all loads.  A store could alias a later load as far as the
-    // compiler knows, so that with plain loads the components follow each other: 33x14x156
-    // with 6 cells 75 -> 69 us a step.  It takes 104 registers instead of 78, and larger grids
-    // lose more by that: 96^3 with 8 cells 123 -> 150, 128^3 266 -> 367.
-    Out o0, o1, o2;
-    if (jin && km) {
-        const Window p = g.template rows<E, Ctx::RO>(x.g(2), g.Y), w = g.template along_z<E, Ctx::RO>(x.g(1));
-        o0 = comp(0, km, p, w, 1, 3, p, E, 2, 4, w);
-    } else {
-        o0 = copy(0);
+    auto mine = [&](int q) { return !Ctx::SPLIT || only == q; };
+    Out o;
+    if (mine(0)) {
+        if (jin && km) {
+            const Window p = g.template rows<E, Ctx::RO>(x.g(2), g.Y), w = g.template along_z<E, Ctx::RO>(x.g(1));
+            o = comp(0, km, p, w, 1, 3, p, E, 2, 4, w);
+        } else {
+            o = copy(0);
+        }
+        store(0, o, 1, 3, 2, 4);
     }
-    if (!Ctx::LAST) store(0, o0, 1, 3, 2, 4);
-    if (iin && km) {
-        const Window p = g.template along_z<E, Ctx::RO>(x.g(0)), w = g.template rows<E, Ctx::RO>(x.g(2), g.X);
-        o1 = comp(1, km, p, w, 0, 0, w, !E, 2, 5, p);
-    } else {
-        o1 = copy(1);
+    if (mine(1)) {
+        if (iin && km) {
+            const Window p = g.template along_z<E, Ctx::RO>(x.g(0)), w = g.template rows<E, Ctx::RO>(x.g(2), g.X);
+            o = comp(1, km, p, w, 0, 0, w, !E, 2, 5, p);
+        } else {
+            o = copy(1);
+        }
+        store(1, o, 0, 0, 2, 5);
     }
-    if (!Ctx::LAST) store(1, o1, 0, 0, 2, 5);
-    if (iin && jin) {
-        const Window p = g.template rows<E, Ctx::RO>(x.g(1), g.X), w = g.template rows<E, Ctx::RO>(x.g(0), g.Y);
-        o2 = comp(2, g.in, p, w, 0, 1, p, E, 1, 2, w);
-    } else {
-        o2 = copy(2);
+    if (mine(2)) {
+        if (iin && jin) {
+            const Window p = g.template rows<E, Ctx::RO>(x.g(1), g.X), w = g.template rows<E, Ctx::RO>(x.g(0), g.Y);
+            o = comp(2, g.in, p, w, 0, 1, p, E, 1, 2, w);
+        } else {
+            o = copy(2);
+        }
+        store(2, o, 0, 1, 1, 2);
     }
-    if (Ctx::LAST) {
-        store(0, o0, 1, 3, 2, 4);
-        store(1, o1, 0, 0, 2, 5);
-    }
-    store(2, o2, 0, 1, 1, 2);
 }
 
 }  // namespace sg

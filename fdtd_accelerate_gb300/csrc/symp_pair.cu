@@ -751,12 +751,15 @@ __device__ __forceinline__ bool edge_group(const Edge &eb, int &i, int &j, int &
 }
 
 // the edge kernels' stages (sg::stage): E or the H stages a, b of a pass
-// FORM of the edge kernels: READ_ONLY for launches that are not chained (see Group::ldf),
-// PLAIN and PLAIN_LAST (see sg::stage) for chained ones
-constexpr int READ_ONLY = 0, PLAIN = 1, PLAIN_LAST = 2;
+// FORM of the edge kernels: READ_ONLY for launches that are not chained (see Group::ldf); PLAIN
+// for chained ones; SPLIT for chained ones of tiny grids, a thread a component (blockIdx.z):
+// three components in turn are a thread's latency there, 58x22x36 with 6 cells 75 us a step,
+// split 51, in a graph 64 and 41 (one cell a thread, three components: 71 and 48); 48^3 71 / 53,
+// 64^3 79 / 69, without CPML 58 / 58, 72^3 77 / 84.
+constexpr int READ_ONLY = 0, PLAIN = 1, SPLIT_COMP = 2;
 template <bool E, int FORM>
 struct EdgeStage {
-    static constexpr bool RO = FORM == READ_ONLY, LAST = FORM == PLAIN_LAST;
+    static constexpr bool RO = FORM == READ_ONLY, SPLIT = FORM == SPLIT_COMP;
     const Params &p;
     __device__ __forceinline__ const Axis &axis(int st, int ax) const { return E ? p.ea[ax] : st ? p.hb[ax] : p.ha[ax]; }
     __device__ __forceinline__ const float *fin(int q) const { return p.in[(E ? 0 : 3) + q]; }
@@ -788,7 +791,8 @@ k_edge_h(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     grid_release();
     int i, j, k;
     if (!edge_group(eb, i, j, k)) return;
-    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false, FORM>{p});
+    sg::stage<false, HH ? 2 : 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<false, FORM>{p},
+                              (int)blockIdx.z);
 }
 
 template <int FORM>
@@ -798,7 +802,7 @@ k_edge_e(const __grid_constant__ Params p, const __grid_constant__ Edge eb) {
     grid_release();
     int i, j, k;
     if (!edge_group(eb, i, j, k)) return;
-    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true, FORM>{p});
+    sg::stage<true, 1>(sg::Group(p.nx, p.ny, p.nz, p.sx, p.sy, i, j, k), EdgeStage<true, FORM>{p}, (int)blockIdx.z);
 }
 
 // Soft sources on edge cells, as a walk of the list in order would add them: a thread a
@@ -1207,11 +1211,11 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
             launch(chained, k_symp_pair<false>, dim3(nb), THREADS, SMEM, st, pl->maps[in], p);
     }
     if (egroups > 0) {
-        const dim3 nb((unsigned)((egroups + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx);
+        const bool split = chained && cells <= 3 << 16;
+        const dim3 nb((unsigned)((egroups + EDGE_BLOCK - 1) / EDGE_BLOCK), (unsigned)pl->g.nx, split ? 3u : 1u);
         const cudaStream_t hs = beside ? pl->side : st;
-        const bool tiny = cells <= 1 << 19;  // (64^3 with 8 cells 77 / 76 us a step, 96^3 123 / 150)
-        if (chained && tiny)
-            launch(true, two_h ? k_edge_h<true, PLAIN_LAST> : k_edge_h<false, PLAIN_LAST>, nb, EDGE_BLOCK, 0, hs, p, eb);
+        if (split)
+            launch(true, two_h ? k_edge_h<true, SPLIT_COMP> : k_edge_h<false, SPLIT_COMP>, nb, EDGE_BLOCK, 0, hs, p, eb);
         else if (chained)
             launch(true, two_h ? k_edge_h<true, PLAIN> : k_edge_h<false, PLAIN>, nb, EDGE_BLOCK, 0, hs, p, eb);
         else
@@ -1222,7 +1226,7 @@ int fdtd_symp_pair_run(fdtd_symp_plan *pl, const fdtd_cpml *ch_tabs_a, const fdt
             if (e != cudaSuccess) { set_cuda_error(e); return FDTD_ERR_CUDA; }
         }
         if (chained)
-            launch(true, tiny ? k_edge_e<PLAIN_LAST> : k_edge_e<PLAIN>, nb, EDGE_BLOCK, 0, st, p, eb);
+            launch(true, split ? k_edge_e<SPLIT_COMP> : k_edge_e<PLAIN>, nb, EDGE_BLOCK, 0, st, p, eb);
         else
             launch(false, k_edge_e<READ_ONLY>, nb, EDGE_BLOCK, 0, st, p, eb);
         bool esrc = false;

@@ -84,7 +84,7 @@ def test_edge_kernels_of_chained_launches():
     assert len(forms) == 5
     for chained, kernel in forms:
         names = set(re.findall(r"k_edge_h<\w+, (\w+)>", kernel) + re.findall(r"k_edge_e<(\w+)>", kernel))
-        assert names and names <= {"true": {"PLAIN", "PLAIN_LAST"}, "false": {"READ_ONLY"}}[chained], kernel
+        assert names and names <= {"true": {"PLAIN", "SPLIT_COMP"}, "false": {"READ_ONLY"}}[chained], kernel
     assert re.search(r"RO = FORM == READ_ONLY,", text)
 
 
