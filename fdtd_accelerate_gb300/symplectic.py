@@ -188,7 +188,7 @@ class SymplecticSolver:
     fused: take the stage-pair path (one pass per H + E stage pair: the pair
     kernel inside, the edge kernels on the y/z CPML shell, small grids by the
     edge kernels alone) where pair_path() allows; bit-identical to the
-    per-stage kernels and faster than them (8.01 against 12.5 ms per step on
+    per-stage kernels and faster than them (7.90 against 12.5 ms per step on
     the 512^3 workload, 76 against 98 us at 64^3); fused=False keeps
     the one-launch-per-stage path.  x_chunk: x planes per work item of the
     pair kernel (0: chosen per tiling by the plan).
